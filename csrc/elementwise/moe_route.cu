@@ -82,10 +82,16 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ldl, const fl
         probs[(int64_t)t * E + e] = p[i];
         s[i] = p[i] + (bias ? bias[e] : 0.f);
       } else {
-        s[i] = -CUDART_INF_F;
+        s[i] = 0.f;                        // no expert: never chosen
       }
     }
-    // k rounds of arg-max over the warp; ties go to the lower expert index
+    // k rounds of arg-max over the warp; ties go to the lower expert index. `open` holds the entries of this lane
+    // that may still be chosen: k <= E, so some lane always has one, and the choice stays inside [0, E) whatever the
+    // scores are. A score that is not a number counts as the lowest one (a row whose softmax is not finite takes its
+    // first k experts); its weight carries the NaN into the output.
+    unsigned open = 0;
+#pragma unroll
+    for (int i = 0; i < kMaxExpertsPerLane; ++i) open |= (unsigned)(lane + 32 * i < E) << i;
     float sel_w[kMaxTopK];
     int sel_e[kMaxTopK];
     float wsum = 0.f;
@@ -95,8 +101,9 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ldl, const fl
 #pragma unroll
       for (int i = 0; i < kMaxExpertsPerLane; ++i) {
         const int e = lane + 32 * i;
-        if (s[i] > best || (s[i] == best && e < best_e)) {
-          best = s[i];
+        const float key = isnan(s[i]) ? -CUDART_INF_F : s[i];
+        if ((open >> i & 1) != 0 && (key > best || (key == best && e < best_e))) {
+          best = key;
           best_e = e;
         }
       }
@@ -115,7 +122,7 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ldl, const fl
       for (int i = 0; i < kMaxExpertsPerLane; ++i)
         if (lane + 32 * i == best_e) {
           pw = p[i];
-          s[i] = -CUDART_INF_F;
+          open &= ~(1u << i);
         }
       pw = __shfl_sync(0xffffffffu, pw, best_e & 31);
       sel_w[j] = pw;

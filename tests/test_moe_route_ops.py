@@ -88,6 +88,42 @@ def test_route_kernel_matches_reference(E, k, renorm, use_bias):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("E,k", [(8, 2), (8, 8), (33, 3), (64, 6), (256, 8)])
+@pytest.mark.parametrize("use_bias", [False, True])
+def test_route_kernel_stays_in_range_for_rows_that_are_not_finite(E, k, use_bias):
+    """A token whose logits hold NaN or infinities still gets k different experts of the E there are (the tables that
+    follow are indexed with them), weights that carry the NaN, and leaves the other tokens' choices alone."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import moe_route as mr
+    torch.manual_seed(E * 10 + k)
+    T, inf, nan = 300, float("inf"), float("nan")
+    perm = torch.rand(T, E, device="cuda").argsort(dim=-1).float()
+    logits = ((perm - E / 2) / 32).to(torch.bfloat16)
+    bias = torch.randn(E, device="cuda") * 1e-4 if use_bias else None
+    _, clean_idx, clean_w, _ = mr.route(logits, bias, k, True)
+    bad = {3: nan, 64: inf, 65: -inf}                       # one entry: NaN, +inf (softmax NaN), -inf (softmax fine)
+    for row, value in bad.items():
+        logits[row, E // 2] = value
+    logits[100], logits[101], logits[102] = nan, inf, -inf   # whole rows: no score compares
+    not_finite = torch.zeros(T, dtype=torch.bool, device="cuda")
+    not_finite[[3, 64, 100, 101, 102]] = True
+    logits.requires_grad_()
+    probs, idx, w, counts = mr.route(logits, bias, k, True)
+    ops.check_status("moe route")
+    assert idx.min().item() >= 0 and idx.max().item() < E
+    assert (idx.long().sort(dim=1).values.diff(dim=1) > 0).all(), "an expert twice"
+    assert torch.equal(counts.long(), torch.bincount(idx.reshape(-1).long(), minlength=E)) and counts.numel() == E
+    assert torch.equal(torch.isnan(probs).all(dim=1), not_finite) and torch.equal(torch.isnan(w).all(dim=1), not_finite)
+    assert (idx[not_finite].long() == torch.arange(k, device="cuda")).all()
+    same = ~not_finite
+    same[65] = False
+    assert torch.equal(idx[same], clean_idx[same]) and torch.equal(w[same], clean_w[same])
+    assert probs[65, E // 2].item() == 0 and w[65].isfinite().all()
+    (w * torch.randn_like(w)).sum().backward()
+    assert torch.equal(logits.grad.isfinite().all(dim=1), ~not_finite)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("T,E,k,C", [(512, 8, 2, 100), (4096, 64, 6, 300), (100, 4, 1, 1000)])
 def test_slots_kernel_matches_reference(T, E, k, C):
     from picotron_b200.ops import moe_route as mr
