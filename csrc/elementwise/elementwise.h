@@ -106,13 +106,15 @@ int pico_moe_combine_bwd(const void* dy, const void* out, const int32_t* row_of_
 // Dropless layout of E <= 256 experts for R routed rows (idx int32 [R], 16-byte aligned; counts int32 [E]):
 // expert e owns slots [seg_start[e], seg_start[e+1]), multiples of 128, its rows first in row order.
 // slot_of_row int32 [R]; row_of_slot int32 [128 * max_tiles] (-1 in padding slots; not written past
-// seg_start[E]); seg_start int32 [E + 1]; tile_group int32 [max_tiles], -1 past the last segment.
+// seg_start[E]); seg_start int32 [E + 1]; tile_group int32 [max_tiles], -1 past the last segment. Rows of no
+// expert, or more of them than the counts say, get slot -1 and set the status words.
 int pico_moe_layout(const int32_t* idx, const int32_t* counts, int R, int E, int max_tiles, int32_t* slot_of_row,
                     int32_t* row_of_slot, int32_t* seg_start, int32_t* tile_group, cudaStream_t stream);
 // out[s] = x[row_of_slot[s] / k] for s < *used (zeros where row_of_slot[s] < 0); bf16 rows of width d.
 int pico_moe_gather(const void* x, const int32_t* row_of_slot, const int32_t* used, void* out, int slots, int k, int d,
                     cudaStream_t stream);
-// y[t] = sum_j w[t,j] * x[slot_of_row[t,j]] (w NULL: plain sum), fp32 sums in the order of j; bf16 rows of width d.
+// y[t] = sum_j w[t,j] * x[slot_of_row[t,j]] (w NULL: plain sum), fp32 sums in the order of j; bf16 rows of width d; NaN
+// where a slot is negative.
 int pico_moe_scatter_sum(const void* x, const int32_t* slot_of_row, const float* w, void* y, int T, int k, int d,
                          cudaStream_t stream);
 

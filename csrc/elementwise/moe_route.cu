@@ -29,6 +29,7 @@
 #include <math_constants.h>
 
 #include "../common/host.h"
+#include "../common/ptx.cuh"
 #include "elementwise.h"
 
 namespace pico {
@@ -264,31 +265,36 @@ moe_combine_kernel(const __nv_bfloat16* __restrict__ out, const int32_t* __restr
 }
 
 // One CTA per expert. Expert e's segment starts at the sum of the padded counts before it; its rows keep row
-// order. Every thread takes kRowsPerThread consecutive rows of a pass (one 16-byte load per four), so a
+// order. Every thread takes kLayoutRows consecutive rows of a pass (one 16-byte load per four), so a
 // pass costs one block scan for 16384 rows; a scan per 1024 rows (moe_slots_kernel) took 70 us for 49152
 // rows, most of it barriers.
+// Nothing is written or named outside the tables, whatever idx and counts hold: a row of no expert, or one that its
+// expert's count leaves no slot, gets slot -1 and a slot of no row holds -1, and the status words report it.
 constexpr int kLayoutThreads = 1024;
 constexpr int kLayoutRows = 16;
+constexpr int kLayoutBadRow = 3200, kLayoutBadCount = 3201;   // sites in the status words
 __global__ void __launch_bounds__(kLayoutThreads)
 moe_layout_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ counts, int R, int E, int max_tiles,
                   int32_t* __restrict__ slot_of_row, int32_t* __restrict__ row_of_slot,
-                  int32_t* __restrict__ seg_start, int32_t* __restrict__ tile_group) {
+                  int32_t* __restrict__ seg_start, int32_t* __restrict__ tile_group, int* status) {
   const int e = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   __shared__ int warp_tot[kLayoutThreads / 32];
-  __shared__ int s_before[kLayoutThreads / 32];
-  // padded rows of the experts before this one (E <= 256 < blockDim.x)
-  int mine = 0;
-  if ((int)threadIdx.x < e) mine = (counts[threadIdx.x] + 127) & ~127;
+  __shared__ unsigned s_before[kLayoutThreads / 32];
+  // padded rows of the experts before this one (E <= 256 < blockDim.x), no more than the tables hold
+  const unsigned room = 128u * max_tiles;
+  auto padded_rows = [&](int i) { return ((unsigned)min(max(counts[i], 0), R) + 127u) & ~127u; };
+  unsigned before = (int)threadIdx.x < e ? min(padded_rows(threadIdx.x), room) : 0u;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
-  if (lane == 0) s_before[warp] = mine;
+  for (int o = 16; o > 0; o >>= 1) before = min(before + __shfl_xor_sync(0xffffffffu, before, o), room);
+  if (lane == 0) s_before[warp] = before;
   __syncthreads();
-  int seg = 0;
+  before = 0;
 #pragma unroll
-  for (int i = 0; i < 256 / 32; ++i) seg += s_before[i];
-  const int n = counts[e];
-  const int padded = (n + 127) & ~127;
+  for (int i = 0; i < 256 / 32; ++i) before = min(before + s_before[i], room);
+  const int seg = (int)before;
+  const int padded = (int)min(padded_rows(e), room - before);
+  const int n = min(max(counts[e], 0), padded);
   if (threadIdx.x == 0) {
     seg_start[e] = seg;
     if (e == E - 1) seg_start[E] = seg + padded;
@@ -296,20 +302,30 @@ moe_layout_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ c
   for (int i = threadIdx.x; i < padded / 128; i += blockDim.x) tile_group[seg / 128 + i] = e;
   if (e == E - 1)
     for (int i = (seg + padded) / 128 + threadIdx.x; i < max_tiles; i += blockDim.x) tile_group[i] = -1;
-  for (int i = n + threadIdx.x; i < padded; i += blockDim.x) row_of_slot[seg + i] = -1;
   int running = 0;                       // rows of this expert before the current pass
   for (int base = 0; base < R; base += kLayoutThreads * kLayoutRows) {
     const int r0 = base + threadIdx.x * kLayoutRows;
-    uint32_t hit = 0;                    // which of this thread's rows belong to the expert
+    uint32_t hit = 0, none = 0;          // which of this thread's rows belong to the expert, and which to none
+    auto look = [&](int q, int v) {
+      hit |= (uint32_t)(v == e) << q;
+      none |= (uint32_t)((unsigned)v >= (unsigned)E) << q;
+    };
     if (r0 + kLayoutRows <= R) {
 #pragma unroll
-      for (int q = 0; q < kLayoutRows / 4; ++q) {
-        const int4 v = reinterpret_cast<const int4*>(idx + r0)[q];   // idx is 16-byte aligned, r0 a multiple of 16
-        hit |= (uint32_t)(v.x == e) << (4 * q) | (uint32_t)(v.y == e) << (4 * q + 1) |
-               (uint32_t)(v.z == e) << (4 * q + 2) | (uint32_t)(v.w == e) << (4 * q + 3);
+      for (int q = 0; q < kLayoutRows; q += 4) {
+        const int4 v = *reinterpret_cast<const int4*>(idx + r0 + q);   // idx is 16-byte aligned, r0 a multiple of 16
+        look(q, v.x);
+        look(q + 1, v.y);
+        look(q + 2, v.z);
+        look(q + 3, v.w);
       }
     } else {
-      for (int q = 0; q < kLayoutRows && r0 + q < R; ++q) hit |= (uint32_t)(idx[r0 + q] == e) << q;
+      for (int q = 0; q < kLayoutRows && r0 + q < R; ++q) look(q, idx[r0 + q]);
+    }
+    for (; e == 0 && none != 0; none &= none - 1) {    // one CTA answers for the rows of no expert
+      const int r = r0 + __ffs(none) - 1;
+      slot_of_row[r] = -1;
+      report_error(status, PICO_ERR_BOUNDS, kLayoutBadRow, r);
     }
     const int c = __popc(hit);
     int incl = c;
@@ -334,12 +350,14 @@ moe_layout_kernel(const int32_t* __restrict__ idx, const int32_t* __restrict__ c
     while (hit != 0) {
       const int q = __ffs(hit) - 1;
       hit &= hit - 1;
-      slot_of_row[r0 + q] = seg + pos;
-      row_of_slot[seg + pos] = r0 + q;
+      slot_of_row[r0 + q] = pos < n ? seg + pos : -1;
+      if (pos < n) row_of_slot[seg + pos] = r0 + q;
       ++pos;
     }
     running += total;
   }
+  for (int i = min(running, n) + threadIdx.x; i < padded; i += blockDim.x) row_of_slot[seg + i] = -1;
+  if (threadIdx.x == 0 && running != counts[e]) report_error(status, PICO_ERR_BOUNDS, kLayoutBadCount, e);
 }
 
 // One warp per slot; slots at or past *used are left alone.
@@ -371,7 +389,8 @@ moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict
   }
 }
 
-// One warp per token, fp32 sums in the order of k. kHasW: weighted by w[t, j].
+// One warp per token, fp32 sums in the order of k. kHasW: weighted by w[t, j]. A row without a slot (-1, which the
+// layout reports) makes its token's sum NaN.
 template <bool kHasW>
 __global__ void __launch_bounds__(256)
 moe_scatter_sum_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ slot_of_row,
@@ -392,7 +411,9 @@ moe_scatter_sum_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __res
       uint4 raw[kMaxTopK];               // all k rows' loads in flight
 #pragma unroll
       for (int j = 0; j < kMaxTopK; ++j)
-        if (j < k) raw[j] = reinterpret_cast<const uint4*>(x + (int64_t)slot[j] * d)[v];
+        if (j < k)
+          raw[j] = slot[j] >= 0 ? reinterpret_cast<const uint4*>(x + (int64_t)slot[j] * d)[v]
+                                : make_uint4(~0u, ~0u, ~0u, ~0u);     // bf16 NaNs
       float acc[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -539,7 +560,7 @@ extern "C" int pico_moe_layout(const int32_t* idx, const int32_t* counts, int R,
     return -2;
   }
   moe_layout_kernel<<<E, kLayoutThreads, 0, stream>>>(idx, counts, R, E, max_tiles, slot_of_row, row_of_slot, seg_start,
-                                                     tile_group);
+                                                     tile_group, pico_status_buffer());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) pico_host::set_error("moe_layout: %s", cudaGetErrorString(e));
   return (int)e;

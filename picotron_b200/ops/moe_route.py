@@ -221,7 +221,7 @@ class _CombineRowsFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         out, w, row_of_slot, used = ctx.saved_tensors
-        dout, dw = torch.empty_like(out), torch.empty_like(w)      # every row has a slot: all of dw is written
+        dout, dw = torch.empty_like(out), torch.zeros_like(w)      # a row that the layout could not place keeps 0
         ext().moe_combine_bwd(dy.contiguous(), out, row_of_slot, w, dout, dw, w.shape[1], used)
         count_launch()
         return dout, dw, None, None, None

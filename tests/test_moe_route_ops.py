@@ -214,3 +214,83 @@ def test_local_experts_layer_matches_the_tensor_path(T, E, k, latent, monkeypatc
     assert len(got[0]) == len(got[1])
     for a, b in zip(*got):
         assert ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)).item() < 2 ** -6
+
+
+@pytest.mark.gpu
+def test_layout_reports_rows_that_it_cannot_place():
+    """Indices that name no expert and counts that disagree with the indices: everything read later stays inside the
+    tables (slot -1, row -1), the other rows lie where they would, and the status words say so."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import moe_route as mr
+    T, E, k, d = 300, 4, 2, 64
+    g = torch.Generator(device="cuda").manual_seed(5)
+    idx = torch.randint(0, E, (T, k), device="cuda", generator=g, dtype=torch.int32)
+    good = idx.clone()
+    idx[7, 1], idx[8, 0], idx[299, 1] = E, -1, 2 ** 31 - 1
+    placed = ((idx >= 0) & (idx < E)).reshape(-1)
+    counts = torch.bincount(idx.reshape(-1)[placed], minlength=E).int()
+    slot, table, layout = mr.local_layout(idx, counts)
+    with pytest.raises(RuntimeError, match="bounds"):
+        ops.check_status()
+    want, fill = [], [0] * E
+    for e in idx.reshape(-1).tolist():
+        want.append(layout.seg_start[e].item() + fill[e] if 0 <= e < E else -1)
+        if 0 <= e < E:
+            fill[e] += 1
+    assert slot.tolist() == want
+    used = layout.seg_start[-1].item()
+    rows = torch.arange(T * k, device="cuda", dtype=torch.int32)[placed]
+    assert torch.equal(table[slot[placed].long()], rows) and (table[:used] >= 0).sum().item() == rows.numel()
+    # the sums: NaN for the tokens with such a row, the others as always
+    x = torch.randn(T, d, device="cuda", generator=g).to(torch.bfloat16).requires_grad_()
+    w = torch.rand(T, k, device="cuda", generator=g).requires_grad_()
+    out = mr.gather_rows(x, slot, table, layout, k)
+    y = mr.combine_rows(out, w, slot, table, layout)
+    y.backward(torch.ones_like(y))
+    bad = torch.zeros(T, dtype=torch.bool, device="cuda")
+    bad[[7, 8, 299]] = True
+    assert torch.equal(torch.isnan(y).all(dim=1), bad) and torch.equal(torch.isnan(x.grad).all(dim=1), bad)
+    assert torch.allclose(y[~bad].float(), (x * w.sum(1, keepdim=True))[~bad].float(), rtol=2 ** -7)
+    assert (w.grad.reshape(-1)[~placed] == 0).all() and w.grad.isfinite().all()
+    # counts below and above what the indices hold, and far beyond the tables
+    for wrong in ([0, 0, 0, 0], [1, 600, 0, 300], [2 ** 31 - 1] * E, [-5] * E):
+        slot, table, layout = mr.local_layout(good, torch.tensor(wrong, device="cuda", dtype=torch.int32))
+        with pytest.raises(RuntimeError, match="bounds"):
+            ops.check_status()
+        used = layout.seg_start[-1].item()
+        assert 0 <= used <= layout.rows and slot.max().item() < used and slot.min().item() >= -1
+        assert used == 0 or (table[:used].max().item() < T * k and table[:used].min().item() >= -1)
+        assert layout.tile_group.max().item() < E and layout.tile_group.min().item() >= -1
+        assert (layout.seg_start.diff() >= 0).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("E,k", [(8, 2), (64, 6)])
+def test_tokens_that_are_not_finite_stay_among_themselves(E, k):
+    """A diverging token through the whole layer: NaN in its own outputs and input gradient, the others as without it."""
+    from types import SimpleNamespace
+    from picotron_b200 import ops
+    from picotron_b200 import process_group_manager as pgm
+    from picotron_b200.parallel.expert_parallel import MoELayer
+    if pgm.process_group_manager is None:
+        pgm.setup_process_group_manager(1, 1, 1, 1, 1)
+    torch.manual_seed(E)
+    with torch.device("cuda"):
+        layer = MoELayer(SimpleNamespace(hidden_size=512, intermediate_size=256, num_experts=E,
+                                         num_experts_per_tok=k)).to(torch.bfloat16)
+    clean = torch.randn(257, 512, device="cuda", dtype=torch.bfloat16)
+    dirty = clean.clone()
+    dirty[3, 17], dirty[200] = float("nan"), float("inf")
+    dy = torch.randn_like(clean)
+    got = []
+    for x in (clean, dirty):
+        x.requires_grad_()
+        assert layer._local_routed_ok(x)
+        y = layer(x)
+        y.backward(dy)
+        got.append((y.detach(), x.grad))
+    ops.check_status("moe layer")
+    same = torch.ones(257, dtype=torch.bool, device="cuda")
+    same[[3, 200]] = False
+    for a, b in zip(*got):
+        assert torch.isnan(b[~same]).all() and torch.equal(a[same], b[same])
