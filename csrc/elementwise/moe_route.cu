@@ -553,10 +553,10 @@ extern "C" int pico_moe_combine(const void* out, const int32_t* idx, const int32
 extern "C" int pico_moe_layout(const int32_t* idx, const int32_t* counts, int R, int E, int max_tiles,
                                int32_t* slot_of_row, int32_t* row_of_slot, int32_t* seg_start, int32_t* tile_group,
                                cudaStream_t stream) {
-  if (R < 0 || E < 1 || E > 32 * kMaxExpertsPerLane || max_tiles < (R + 127) / 128 + E ||
+  if (R < 0 || E < 1 || E > 32 * kMaxExpertsPerLane || max_tiles < (R + 127) / 128 + (E < R ? E : R) ||
       (reinterpret_cast<uintptr_t>(idx) & 15) != 0) {
-    pico_host::set_error("moe_layout: %d rows, %d experts (max %d), %d tiles (at least rows / 128 + experts), "
-                         "16-byte aligned indices", R, E, 32 * kMaxExpertsPerLane, max_tiles);
+    pico_host::set_error("moe_layout: %d rows, %d experts (max %d), %d tiles (at least rows / 128 + experts that can "
+                         "have rows), 16-byte aligned indices", R, E, 32 * kMaxExpertsPerLane, max_tiles);
     return -2;
   }
   moe_layout_kernel<<<E, kLayoutThreads, 0, stream>>>(idx, counts, R, E, max_tiles, slot_of_row, row_of_slot, seg_start,

@@ -147,6 +147,12 @@ def combine(out: torch.Tensor, idx: torch.Tensor, pos: torch.Tensor, w: torch.Te
 
 
 # ------------------------------------------------------------------------- dropless, all experts local
+def max_tiles(rows: int, num_experts: int) -> int:
+    """128-row tiles that ``rows`` routed rows can fill: each expert that has any may leave its last tile short. (Not
+    every expert counts: one token and 256 experts would take 257 tiles of every activation and not 9.)"""
+    return (rows + 127) // 128 + min(num_experts, rows)
+
+
 def layout_ref(idx: torch.Tensor, num_experts: int):
     """(slot_of_row [R], row_of_slot, seg_start [E+1], tile_group) of the dropless layout: every expert's
     rows in row order, its segment padded to whole 128-row tiles. Host integers; the test oracle."""
@@ -158,7 +164,7 @@ def layout_ref(idx: torch.Tensor, num_experts: int):
     for c in counts:
         seg.append(seg[-1] + (c + 127) // 128 * 128)
     rows = len(flat)
-    tiles = rows // 128 + (1 if rows % 128 else 0) + num_experts
+    tiles = max_tiles(rows, num_experts)
     table, slots_, fill = [-1] * (128 * tiles), [0] * rows, list(seg[:-1])
     for r, e in enumerate(flat):
         slots_[r] = fill[e]
@@ -176,7 +182,7 @@ def local_layout(idx: torch.Tensor, counts: torch.Tensor):
     are sized for the most padding there can be; what is filled ends at ``layout.seg_start[E]``."""
     from .grouped_gemm import TILE, GroupLayout
     R, E = idx.numel(), counts.numel()
-    tiles = (R + TILE - 1) // TILE + E
+    tiles = max_tiles(R, E)
     # one allocation for the four tables
     buf = torch.empty(R + TILE * tiles + tiles + E + 1, device=idx.device, dtype=torch.int32)
     slot_of_row, row_of_slot, tile_group, seg_start = buf.split([R, TILE * tiles, tiles, E + 1])

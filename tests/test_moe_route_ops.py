@@ -166,6 +166,35 @@ def test_reference_layout_orders_and_pads():
     assert all(table[s].item() == r for r, s in enumerate(slot.tolist())) and (table >= 0).sum() == 6
 
 
+@pytest.mark.parametrize("rows,E", [(1, 256), (8, 256), (255, 256), (300, 256), (129, 1), (1000, 7), (4096, 64)])
+def test_layout_buffers_hold_every_routing_and_little_more(rows, E):
+    """Enough tiles for the routing that pads most (single rows in as many experts as there are, the rest in one), and
+    never a tile for an expert that cannot have a row."""
+    from picotron_b200.ops import moe_route as mr
+    n = min(rows, E)
+    counts = [1] * (n - 1) + [rows - (n - 1)]
+    worst = sum((c + 127) // 128 for c in counts)
+    assert worst <= mr.max_tiles(rows, E) <= worst + (rows + 127) // 128
+    idx = torch.tensor([e for e, c in enumerate(counts) for _ in range(c)])
+    slot, table, seg, owner = mr.layout_ref(idx, E)
+    assert table.numel() == 128 * mr.max_tiles(rows, E) == 128 * owner.numel() and seg[-1] == 128 * worst
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,E,k", [(1, 256, 8), (3, 256, 1), (40, 64, 6)])
+def test_layout_kernel_with_more_experts_than_rows(T, E, k):
+    from picotron_b200 import ops
+    from picotron_b200.ops import moe_route as mr
+    idx = torch.stack([torch.randperm(E, device="cuda")[:k] for _ in range(T)]).int()
+    counts = torch.bincount(idx.reshape(-1), minlength=E).int()
+    slot, table, layout = mr.local_layout(idx, counts)
+    ops.check_status("moe layout")
+    rslot, rtable, rseg, rowner = mr.layout_ref(idx, E)
+    used = rseg[-1].item()
+    assert torch.equal(slot, rslot) and torch.equal(table[:used], rtable[:used])
+    assert torch.equal(layout.seg_start, rseg) and torch.equal(layout.tile_group, rowner)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("T,E,k,skew", [(1, 4, 1, 0), (777, 64, 6, 0), (4096, 256, 8, 2), (2731, 8, 6, 3), (8192, 64, 6, 1)])
 def test_layout_kernel_matches_reference(T, E, k, skew):
