@@ -843,6 +843,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   m.def("gemm_parts", &gemm_parts);
   m.def("gemm_parts_of_k", [](int64_t M, int64_t N, int64_t K) { return pico_gemm_parts_of_k((int)M, (int)N, (int)K); });
+  m.def("gemm_plan", [](int64_t sms, int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn, int64_t out_mode, int64_t max_ctas) {
+    std::array<int, 4> plan;
+    check(pico_gemm_plan((int)sms, (int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, (int)max_ctas, plan.data()), "gemm_plan");
+    return plan;
+  });
   m.def("gemm_new", &gemm_new);
   m.def("linear_fwd", &linear_fwd);
   m.def("rmsnorm_new", &rmsnorm_new);

@@ -17,6 +17,11 @@ int pico_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, i
                    int ldd, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
                    cudaStream_t stream);
 
+// What pico_gemm_bf16 runs such a product on, given `sms` SMs (0: those of the current device): plan[0] the CTA pairs
+// at work (0: one-CTA tiles), plan[1] the tile width, and for pairs plan[2] the 256 x 256 output tiles and plan[3] how
+// many of them are not cut along K.
+int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas, int plan[4]);
+
 // D[M,N] (bf16, row stride ldd) = A[M,K] * op(B) summed in `parts` stretches of K, each by its own CTAs into its
 // own fp32 slab, the slabs then added in order (deterministic) and rounded once. For products with few tiles and
 // a long K. slabs: scratch of parts * ceil(M / 128) * 128 * N floats, 16-byte aligned.

@@ -593,31 +593,29 @@ static int dispatch_bn(const void* A, const void* B, void* D, int M, int N, int 
 // one-CTA kernels lose against the pair kernel at large sizes (8192 x 16384 x 2048: pair 1564 TFLOP/s,
 // one CTA 128 x 256 1394). Pair tiles win when there are many of them; narrower ones when a nearly
 // empty last round would cost more than their extra operand traffic.
-struct GemmChoice {
-  bool pair;
-  int bn;
-};
-
-static GemmChoice choose_tile(int M, int N, int K, int a_mn, int b_mn, int out_mode, int max_ctas) {
-  int sms = pico_host::num_sms();
+// The accumulating form may cut the tiles of its last, partial round along K (partial sums can be added to D as
+// they are) when each pair gets at least 3 blocks of them: the one more epilogue that it costs is about 5 blocks.
+GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn, int b_mn, int out_mode, int max_ctas) {
   if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
-  const double kb = (K + BK - 1) / BK;
-  auto tiles = [&](int tm, int tn) { return (double)((M + tm - 1) / tm) * ((N + tn - 1) / tn); };
-  auto rounds = [](double t, double slots) { return (double)(int64_t)((t + slots - 1) / slots); };
-  GemmChoice best{false, 128};
-  double best_cost = rounds(tiles(128, 128), sms) * kb * 256 * 1.3 + 1500;
-  const double wide = rounds(tiles(128, 256), sms) * kb * 512 * 1.12 + 2500;
+  const int64_t kb = (K + BK - 1) / BK;
+  auto tiles = [&](int tm, int tn) { return (int64_t)((M + tm - 1) / tm) * ((N + tn - 1) / tn); };
+  auto rounds = [](int64_t t, int64_t slots) { return (t + slots - 1) / slots; };
+  GemmPlan best{false, 64, 0, 0, 0};
+  if (N <= 64) return best;               // narrow outputs waste less of the tile with a smaller bn
+  best.bn = 128;
+  double best_cost = (double)(rounds(tiles(128, 128), sms) * kb) * 256 * 1.3 + 1500;
+  const double wide = (double)(rounds(tiles(128, 256), sms) * kb) * 512 * 1.12 + 2500;
   if (wide < best_cost) {
     best_cost = wide;
-    best = GemmChoice{false, 256};
+    best.bn = 256;
   }
-  if (sms >= 2 && M > BM && N > 128 && gemm_pair_has(a_mn, b_mn, out_mode)) {
-    const int pairs = sms / 2;
-    const double t = tiles(2 * BM, 256);
-    // the accumulating form cuts its last round into equal shares, at the price of one more epilogue
-    const bool cut = out_mode == OUT_F32_ACC && t * kb / pairs >= 3;
-    const double cost = cut ? t / pairs * kb * 512 + 5000 : rounds(t, pairs) * kb * 512 + 2500;
-    if (cost < best_cost) best = GemmChoice{true, 256};
+  const int64_t t = tiles(2 * BM, 256);
+  if (sms >= 2 && M > BM && N > 128 && gemm_pair_has(a_mn, b_mn, out_mode) && t < INT32_MAX) {
+    const int64_t pairs = sms / 2, rest = t % pairs;
+    const bool cut = out_mode == OUT_F32_ACC && rest * kb / pairs >= 3;
+    const double cost = cut ? (double)(t / pairs * kb + rounds(rest * kb, pairs)) * 512 + 5000
+                            : (double)(rounds(t, pairs) * kb) * 512 + 2500;
+    if (cost < best_cost) best = GemmPlan{true, 256, (int)pairs, (int)t, (int)(cut ? t - rest : t)};
   }
   return best;
 }
@@ -692,22 +690,28 @@ extern "C" int pico_gemm_bf16_ex(const void* A, const void* B, void* D, int M, i
                                  int ldb, int ldd, int a_mn_major, int b_mn_major, int out_mode,
                                  int max_ctas, const PicoGemmComm* comm, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  // Narrow outputs waste less of the tile with a smaller BN.
-  if (N <= 64)
-    return pico::dispatch_bn<64>(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode,
-                                 max_ctas, comm, stream);
-  pico::GemmChoice c{false, 256};
+  pico::GemmPlan plan{false, 256, 0, 0, 0};
   if (comm == nullptr)
-    c = pico::choose_tile(M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas);
+    plan = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas);
+  else if (N <= 64)
+    plan.bn = 64;
   else if (N <= 128 || ((N + 127) / 128) * ((M + 127) / 128) <= pico_host::num_sms())
-    c.bn = 128;   // no more 128 x 128 tiles than SMs: one wave either way
-  if (c.pair)
-    return pico::gemm_pair(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, stream);
-  if (c.bn == 128)
-    return pico::dispatch_bn<128>(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major,
-                                  out_mode, max_ctas, comm, stream);
-  return pico::dispatch_bn<256>(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode,
-                                max_ctas, comm, stream);
+    plan.bn = 128;   // no more 128 x 128 tiles than SMs: one wave either way
+  if (plan.pair)
+    return pico::gemm_pair(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, stream);
+  auto one_cta = plan.bn == 64 ? pico::dispatch_bn<64> : plan.bn == 128 ? pico::dispatch_bn<128> : pico::dispatch_bn<256>;
+  return one_cta(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, comm, stream);
+}
+
+extern "C" int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
+                              int plan[4]) {
+  const pico::GemmPlan p = pico::plan_gemm(sms > 0 ? sms : pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode,
+                                           max_ctas);
+  plan[0] = p.pair ? p.pairs : 0;
+  plan[1] = p.bn;
+  plan[2] = p.tiles;
+  plan[3] = p.whole;
+  return 0;
 }
 
 extern "C" int pico_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,

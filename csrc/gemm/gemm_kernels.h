@@ -8,9 +8,19 @@ enum GemmOutMode : int { GEMM_OUT_BF16 = 0, GEMM_OUT_F32 = 1, GEMM_OUT_F32_ACC =
 
 constexpr int kGemmPairUnsupported = -10;
 
-// CTA-pair kernel with 256 x 256 tiles; operands as pico_gemm_bf16.
+// What a plain product runs on: the CTA-pair kernel (256 x 256 tiles) or the one-CTA kernel with 128 x bn tiles.
+// Pair kernel: `whole` of the `tiles` output tiles are dealt to the pairs as they are, the others (the last, partial
+// round of an accumulating product) are cut along K into equal shares for all pairs.
+struct GemmPlan {
+  bool pair;
+  int bn;
+  int pairs, tiles, whole;
+};
+GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas);
+
+// CTA-pair kernel; operands as pico_gemm_bf16, `plan` as plan_gemm gives it for them.
 bool gemm_pair_has(int a_mn_major, int b_mn_major, int out_mode);
-int gemm_pair(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
-              int a_mn_major, int b_mn_major, int out_mode, int max_ctas, cudaStream_t stream);
+int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
+              int a_mn_major, int b_mn_major, int out_mode, cudaStream_t stream);
 
 }  // namespace pico

@@ -340,8 +340,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 }
 
 template <int BN, int A_MN, int B_MN, int OUT>
-static int launch(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int max_ctas,
-                  cudaStream_t stream) {
+static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
+                  int ldd, cudaStream_t stream) {
   using C = Cfg<BN>;
   using pico_host::Swizzle;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -370,18 +370,9 @@ static int launch(const void* A, const void* B, void* D, int M, int N, int K, in
     }
     attr_dev = dev;
   }
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
-  int ctas = pico_host::num_sms();
-  if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
-  int pairs = ctas / 2;
-  int whole = tiles;
-  // cut the last round along K where partial sums can be added to D and the shares are long enough
-  // (the extra reduce-add of a tile costs about as much as 5 blocks; choose_tile counts it)
-  const int rest = tiles % pairs;
-  const int num_kb = (K + BK - 1) / BK;
-  if (OUT == GEMM_OUT_F32_ACC && rest != 0 && (int64_t)rest * num_kb / pairs >= 3) whole = tiles - rest;
-  if (whole == tiles && tiles < pairs) pairs = tiles;
-  pico_host::launch_ahead(kern, 2 * pairs, kThreads, C::kSmemBytes, stream, ta, tb, td, M, N, K, whole, pico_status_buffer());
+  const int pairs = plan.whole == plan.tiles && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
+  pico_host::launch_ahead(kern, 2 * pairs, kThreads, C::kSmemBytes, stream, ta, tb, td, M, N, K, plan.whole,
+                          pico_status_buffer());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     pico_host::set_error("gemm launch: %s", cudaGetErrorString(e));
@@ -391,11 +382,11 @@ static int launch(const void* A, const void* B, void* D, int M, int N, int K, in
 }
 
 template <int BN>
-static int dispatch(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int a_mn,
-                    int b_mn, int out_mode, int max_ctas, cudaStream_t st) {
+static int dispatch(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
+                    int ldd, int a_mn, int b_mn, int out_mode, cudaStream_t st) {
 #define PICO_CASE(AM, BMJ, OM)                                 \
   if (a_mn == AM && b_mn == BMJ && out_mode == OM)             \
-    return launch<BN, AM, BMJ, OM>(A, B, D, M, N, K, lda, ldb, ldd, max_ctas, st);
+    return launch<BN, AM, BMJ, OM>(plan, A, B, D, M, N, K, lda, ldb, ldd, st);
   PICO_CASE(0, 0, GEMM_OUT_BF16)
   PICO_CASE(0, 1, GEMM_OUT_BF16)
   PICO_CASE(1, 1, GEMM_OUT_BF16)
@@ -411,9 +402,9 @@ bool gemm_pair_has(int a_mn, int b_mn, int out_mode) {
          (out_mode == GEMM_OUT_F32_ACC && a_mn == 1 && b_mn == 1);
 }
 
-int gemm_pair(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int a_mn,
-              int b_mn, int out_mode, int max_ctas, cudaStream_t stream) {
-  return pair::dispatch<256>(A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, max_ctas, stream);
+int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
+              int a_mn, int b_mn, int out_mode, cudaStream_t stream) {
+  return pair::dispatch<256>(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, stream);
 }
 
 }  // namespace pico

@@ -189,3 +189,37 @@ def test_untracked_only_where_nothing_watches_the_call():
     with torch.inference_mode():
         note(torch.ones(2))
     assert seen == [False, True, False, False, False, True]
+
+
+def test_gemm_plan_cuts_what_it_prices_as_cut():
+    """The model that chooses a product's tiles and the launch share one decision about cutting the last round along K:
+    no tile, or every tile of the partial round, each pair's share at least 3 blocks, accumulating products only."""
+    from picotron_b200 import ops
+    if not ops.ext_available():
+        pytest.skip("extension not built")
+    plan = ops.ext().gemm_plan
+    cuts = pairs_seen = 0
+    for sms in (148, 132, 74, 9, 2, 1):
+        for max_ctas in (0, 1, 2, 37):
+            at_work = (min(sms, max_ctas) if max_ctas else sms) // 2
+            for M in (64, 128, 129, 520, 2048, 5120, 16384):
+                for N in (8, 64, 65, 264, 960, 2048, 11008):
+                    for K in (8, 192, 1999, 2048, 16384):
+                        for acc in (False, True):
+                            pairs, bn, tiles, whole = plan(sms, M, N, K, acc, acc, 2 if acc else 0, max_ctas)
+                            assert bn == 64 if N <= 64 else bn in (128, 256)
+                            if pairs == 0:
+                                continue
+                            pairs_seen += 1
+                            assert pairs == at_work and bn == 256 and tiles == -(-M // 256) * -(-N // 256)
+                            rest, blocks = tiles % pairs, -(-K // 64)
+                            cut = acc and rest * blocks // pairs >= 3
+                            assert whole == (tiles - rest if cut else tiles)
+                            cuts += cut
+    assert pairs_seen > 1000 and cuts > 100
+    # 80 tiles of 32 blocks on 74 pairs: the 6 left over give each pair 2 blocks, too few to cut, and a second round for
+    # them costs more (2 x 32 x 512 cycles) than three rounds of 128 x 128 tiles (3 x 32 x 333)
+    assert plan(148, 5120, 960, 2048, True, True, 2, 0)[:2] == [0, 128]
+    assert plan(148, 5120, 960, 8192, True, True, 2, 0) == [74, 256, 80, 74]      # 10 blocks each
+    assert plan(148, 4736, 1024, 8192, True, True, 2, 0)[2:] == [76, 74]
+    assert plan(148, 9472, 512, 8192, True, True, 2, 0)[2:] == [74, 74]           # whole rounds: nothing left to cut
