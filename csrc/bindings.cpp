@@ -1,6 +1,6 @@
 // Python bindings: thin adapters from torch tensors to the C entry points. They run on the
-// current CUDA stream of the tensor's device, never allocate on the hot path except where a
-// result tensor is returned, and raise with the library's own error text.
+// current CUDA stream of the tensor's device, never allocate on the hot path except a result
+// tensor that is returned or a product's scratch, and raise with the library's own error text.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
@@ -47,9 +47,12 @@ void gemm(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, int64_t M, in
               "gemm: bf16 operands required");
   TORCH_CHECK((out_mode == 0) == (D.scalar_type() == at::kBFloat16), "gemm: output dtype/mode mismatch");
   c10::cuda::CUDAGuard guard(A.device());
+  at::Tensor scratch;
+  if (const int64_t n = pico_gemm_scratch((int)M, (int)N, (int)K, a_mn_major, b_mn_major, (int)out_mode, (int)max_ctas))
+    scratch = at::empty({n}, D.options());
   check(pico_gemm_bf16(A.data_ptr(), B.data_ptr(), D.data_ptr(), (int)M, (int)N, (int)K, (int)lda,
                        (int)ldb, (int)ldd, a_mn_major, b_mn_major, (int)out_mode, (int)max_ctas,
-                       stream_of(A)),
+                       scratch.defined() ? scratch.data_ptr<float>() : nullptr, stream_of(A)),
         "gemm");
 }
 
@@ -845,7 +848,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_parts_of_k", [](int64_t M, int64_t N, int64_t K) { return pico_gemm_parts_of_k((int)M, (int)N, (int)K); });
   m.def("gemm_plan", [](int64_t sms, int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn, int64_t out_mode, int64_t max_ctas) {
     std::array<int, 4> plan;
-    check(pico_gemm_plan((int)sms, (int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, (int)max_ctas, plan.data()), "gemm_plan");
+    check(pico_gemm_plan((int)sms, (int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, (int)max_ctas, 1, plan.data()), "gemm_plan");
     return plan;
   });
   m.def("gemm_new", &gemm_new);

@@ -2,6 +2,7 @@
 // function returns 0 on success and leaves a message in pico_last_error() otherwise.
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 #ifdef __cplusplus
 extern "C" {
@@ -13,14 +14,18 @@ extern "C" {
 //   out_mode  : 0 -> D bf16, 1 -> D fp32, 2 -> D fp32 accumulated in place (D += ...)
 //   max_ctas  : cap on the persistent grid (0 = one CTA per SM); lets a caller leave SMs
 //               free for a kernel running beside the GEMM on another stream
+//   scratch   : NULL, or pico_gemm_scratch floats, 16-byte aligned, where that is not 0: the accumulating form then
+//               splits its last round over all SMs. Results are the same bits on each run with or without it.
 int pico_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
                    int ldd, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
-                   cudaStream_t stream);
+                   float* scratch, cudaStream_t stream);
+int64_t pico_gemm_scratch(int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas);
 
 // What pico_gemm_bf16 runs such a product on, given `sms` SMs (0: those of the current device): plan[0] the CTA pairs
 // at work (0: one-CTA tiles), plan[1] the tile width, and for pairs plan[2] the 256 x 256 output tiles and plan[3] how
 // many of them are not cut along K.
-int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas, int plan[4]);
+int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
+                   int has_scratch, int plan[4]);
 
 // D[M,N] (bf16, row stride ldd) = A[M,K] * op(B) summed in `parts` stretches of K, each by its own CTAs into its
 // own fp32 slab, the slabs then added in order (deterministic) and rounded once. For products with few tiles and

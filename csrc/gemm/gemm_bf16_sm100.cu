@@ -593,9 +593,13 @@ static int dispatch_bn(const void* A, const void* B, void* D, int M, int N, int 
 // one-CTA kernels lose against the pair kernel at large sizes (8192 x 16384 x 2048: pair 1564 TFLOP/s,
 // one CTA 128 x 256 1394). Pair tiles win when there are many of them; narrower ones when a nearly
 // empty last round would cost more than their extra operand traffic.
-// The accumulating form may cut the tiles of its last, partial round along K (partial sums can be added to D as
-// they are) when each pair gets at least 3 blocks of them: the one more epilogue that it costs is about 5 blocks.
-GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn, int b_mn, int out_mode, int max_ctas) {
+// The accumulating form may cut the tiles of its last, partial round along K when each pair gets at least 3 blocks of
+// them. kCutCycles is what the one more epilogue and the kernel that adds the pieces cost: 15 to 17 thousand cycles in
+// 2048 x 1024 x 2048, 2560 x 960 x 1999 and 6144 x 2048 x 8192. Nothing is cut beside another kernel (max_ctas): the
+// adding kernel would take the SMs that the caller leaves free.
+constexpr double kCutCycles = 16000;
+GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn, int b_mn, int out_mode, int max_ctas, bool has_scratch) {
+  const bool may_cut = has_scratch && out_mode == OUT_F32_ACC && max_ctas <= 0;
   if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
   const int64_t kb = (K + BK - 1) / BK;
   auto tiles = [&](int tm, int tn) { return (int64_t)((M + tm - 1) / tm) * ((N + tn - 1) / tn); };
@@ -612,9 +616,13 @@ GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn, int b_mn, int out_mod
   const int64_t t = tiles(2 * BM, 256);
   if (sms >= 2 && M > BM && N > 128 && gemm_pair_has(a_mn, b_mn, out_mode) && t < INT32_MAX) {
     const int64_t pairs = sms / 2, rest = t % pairs;
-    const bool cut = out_mode == OUT_F32_ACC && rest * kb / pairs >= 3;
-    const double cost = cut ? (double)(t / pairs * kb + rounds(rest * kb, pairs)) * 512 + 5000
-                            : (double)(rounds(t, pairs) * kb) * 512 + 2500;
+    double cost = (double)(rounds(t, pairs) * kb) * 512 + 2500;
+    bool cut = false;
+    if (may_cut && rest * kb / pairs >= 3) {
+      const double cut_cost = (double)(t / pairs * kb + rounds(rest * kb, pairs)) * 512 + kCutCycles;
+      cut = cut_cost < cost;
+      if (cut) cost = cut_cost;
+    }
     if (cost < best_cost) best = GemmPlan{true, 256, (int)pairs, (int)t, (int)(cut ? t - rest : t)};
   }
   return best;
@@ -686,27 +694,39 @@ extern "C" int pico_gemm_bf16_parts(const void* A, const void* B, void* D, float
   return 0;
 }
 
-extern "C" int pico_gemm_bf16_ex(const void* A, const void* B, void* D, int M, int N, int K, int lda,
-                                 int ldb, int ldd, int a_mn_major, int b_mn_major, int out_mode,
-                                 int max_ctas, const PicoGemmComm* comm, cudaStream_t stream) {
+static int run_gemm(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int a_mn_major,
+                    int b_mn_major, int out_mode, int max_ctas, const PicoGemmComm* comm, float* scratch,
+                    cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   pico::GemmPlan plan{false, 256, 0, 0, 0};
   if (comm == nullptr)
-    plan = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas);
+    plan = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas, scratch != nullptr);
   else if (N <= 64)
     plan.bn = 64;
   else if (N <= 128 || ((N + 127) / 128) * ((M + 127) / 128) <= pico_host::num_sms())
     plan.bn = 128;   // no more 128 x 128 tiles than SMs: one wave either way
   if (plan.pair)
-    return pico::gemm_pair(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, stream);
+    return pico::gemm_pair(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, scratch, stream);
   auto one_cta = plan.bn == 64 ? pico::dispatch_bn<64> : plan.bn == 128 ? pico::dispatch_bn<128> : pico::dispatch_bn<256>;
   return one_cta(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, comm, stream);
 }
 
+extern "C" int pico_gemm_bf16_ex(const void* A, const void* B, void* D, int M, int N, int K, int lda,
+                                 int ldb, int ldd, int a_mn_major, int b_mn_major, int out_mode,
+                                 int max_ctas, const PicoGemmComm* comm, cudaStream_t stream) {
+  return run_gemm(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, comm, nullptr, stream);
+}
+
+extern "C" int pico_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,
+                              int ldb, int ldd, int a_mn_major, int b_mn_major, int out_mode,
+                              int max_ctas, float* scratch, cudaStream_t stream) {
+  return run_gemm(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, nullptr, scratch, stream);
+}
+
 extern "C" int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
-                              int plan[4]) {
+                              int has_scratch, int plan[4]) {
   const pico::GemmPlan p = pico::plan_gemm(sms > 0 ? sms : pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode,
-                                           max_ctas);
+                                           max_ctas, has_scratch != 0);
   plan[0] = p.pair ? p.pairs : 0;
   plan[1] = p.bn;
   plan[2] = p.tiles;
@@ -714,9 +734,8 @@ extern "C" int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int 
   return 0;
 }
 
-extern "C" int pico_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,
-                              int ldb, int ldd, int a_mn_major, int b_mn_major, int out_mode,
-                              int max_ctas, cudaStream_t stream) {
-  return pico_gemm_bf16_ex(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode,
-                           max_ctas, nullptr, stream);
+extern "C" int64_t pico_gemm_scratch(int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas) {
+  if (out_mode != pico::OUT_F32_ACC || M <= 0 || N <= 0 || K <= 0) return 0;
+  const pico::GemmPlan p = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas, true);
+  return p.pair && p.whole < p.tiles ? (int64_t)p.pairs * pico::kGemmSlab : 0;
 }

@@ -10,17 +10,21 @@ constexpr int kGemmPairUnsupported = -10;
 
 // What a plain product runs on: the CTA-pair kernel (256 x 256 tiles) or the one-CTA kernel with 128 x bn tiles.
 // Pair kernel: `whole` of the `tiles` output tiles are dealt to the pairs as they are, the others (the last, partial
-// round of an accumulating product) are cut along K into equal shares for all pairs.
+// round of an accumulating product) are cut along K into equal shares for all pairs, which takes scratch of
+// kGemmSlab floats per pair (has_scratch).
 struct GemmPlan {
   bool pair;
   int bn;
   int pairs, tiles, whole;
 };
-GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas);
+constexpr int kGemmSlab = 256 * 256;
+GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
+                   bool has_scratch);
 
-// CTA-pair kernel; operands as pico_gemm_bf16, `plan` as plan_gemm gives it for them.
+// CTA-pair kernel; operands as pico_gemm_bf16, `plan` as plan_gemm gives it for them, slabs: its scratch, 16-byte
+// aligned (not read where nothing is cut).
 bool gemm_pair_has(int a_mn_major, int b_mn_major, int out_mode);
 int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
-              int a_mn_major, int b_mn_major, int out_mode, cudaStream_t stream);
+              int a_mn_major, int b_mn_major, int out_mode, float* slabs, cudaStream_t stream);
 
 }  // namespace pico

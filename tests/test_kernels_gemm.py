@@ -264,6 +264,38 @@ def test_pair_tiles_accumulate_with_a_cut_last_round(M, N, K):
     assert ((acc.double() - ref).norm() / ref.norm()).item() < 1e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(6144, 2048, 8192), (960, 960, 8192), (5120, 960, 8192), (516, 771, 4096),
+                                   (512, 512, 16384), (3072, 2040, 7000)])
+def test_cut_last_round_gives_the_same_bits_on_each_run(M, N, K):
+    """Pieces of a tile come from different pairs, two to eighteen of them: D, the first piece and the others are added
+    in that order whoever is done first. Column slices of wider buffers, N without a factor of 4; another stream's
+    work moves the pairs' finishing order about. fp32 sums: 1e-5 of the 64-bit result, nothing beside the slice."""
+    ops, gemm = _ops()
+    pairs, _, tiles, whole = ops.ext().gemm_plan(0, M, N, K, True, True, 2, 0)
+    assert pairs and whole < tiles
+    torch.manual_seed(M + K)
+    a = torch.randn(K, (M + 63) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, 32:32 + M]
+    b = torch.randn(K, (N + 15) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :N]
+    before = torch.randn(M, (N + 7) // 4 * 4 + 4, device="cuda")
+    wide, side, noise = before.clone(), torch.cuda.Stream(), torch.randn(2 ** 24, device="cuda")
+    first = None
+    for run in range(6):
+        wide.copy_(before)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for _ in range(run):
+                noise.mul_(1.0)
+        gemm.gemm_tn(a, b, out=wide[:, 4:4 + N], accumulate=True)
+        torch.cuda.current_stream().wait_stream(side)
+        first = wide.clone() if first is None else first
+        assert torch.equal(wide, first)
+    ops.check_status("pair gemm, cut")
+    ref = before.double()
+    ref[:, 4:4 + N] += a.double().t() @ b.double()
+    assert torch.equal(first[:, :4], before[:, :4]) and torch.equal(first[:, 4 + N:], before[:, 4 + N:])
+    assert ((first.double() - ref).norm() / ref.norm()).item() < 1e-5
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 576, 49152), (1, 64, 8192), (33, 960, 20000), (1000, 520, 32768), (130, 136, 6400)])
 def test_products_summed_in_parts_of_k(M, N, K):
     """Few tiles and a long reduction: parts of K added in fp32 in order, rounded once; the same bits again: 2^-8 of the value for the rounding. The

@@ -193,7 +193,8 @@ def test_untracked_only_where_nothing_watches_the_call():
 
 def test_gemm_plan_cuts_what_it_prices_as_cut():
     """The model that chooses a product's tiles and the launch share one decision about cutting the last round along K:
-    no tile, or every tile of the partial round, each pair's share at least 3 blocks, accumulating products only."""
+    no tile, or every tile of the partial round, each pair's share at least 3 blocks, accumulating products that have
+    the device to themselves only."""
     from picotron_b200 import ops
     if not ops.ext_available():
         pytest.skip("extension not built")
@@ -213,13 +214,17 @@ def test_gemm_plan_cuts_what_it_prices_as_cut():
                             pairs_seen += 1
                             assert pairs == at_work and bn == 256 and tiles == -(-M // 256) * -(-N // 256)
                             rest, blocks = tiles % pairs, -(-K // 64)
-                            cut = acc and rest * blocks // pairs >= 3
-                            assert whole == (tiles - rest if cut else tiles)
-                            cuts += cut
-    assert pairs_seen > 1000 and cuts > 100
+                            if whole != tiles:
+                                cuts += 1
+                                assert whole == tiles - rest and acc and max_ctas == 0 and rest * blocks // pairs >= 3
+                                # shorter than the round that it replaces by what the adding kernel costs
+                                assert (blocks - -(-rest * blocks // pairs)) * 512 > 13500
+                            elif acc and max_ctas == 0 and rest * blocks // pairs >= 3:
+                                assert (blocks - -(-rest * blocks // pairs)) * 512 <= 13500
+    assert pairs_seen > 1000 and cuts > 40
     # 80 tiles of 32 blocks on 74 pairs: the 6 left over give each pair 2 blocks, too few to cut, and a second round for
     # them costs more (2 x 32 x 512 cycles) than three rounds of 128 x 128 tiles (3 x 32 x 333)
     assert plan(148, 5120, 960, 2048, True, True, 2, 0)[:2] == [0, 128]
     assert plan(148, 5120, 960, 8192, True, True, 2, 0) == [74, 256, 80, 74]      # 10 blocks each
-    assert plan(148, 4736, 1024, 8192, True, True, 2, 0)[2:] == [76, 74]
+    assert plan(148, 2048, 2048, 8192, True, True, 2, 0) == [74, 256, 64, 64]     # 110 of 128 blocks: not worth it
     assert plan(148, 9472, 512, 8192, True, True, 2, 0)[2:] == [74, 74]           # whole rounds: nothing left to cut
