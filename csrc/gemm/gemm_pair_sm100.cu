@@ -209,6 +209,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           }
         }
       }
+      // The commits that release the last stages arrive here from the first CTA's tensor core, which no barrier of its
+      // threads orders: neither CTA may go away before they have (a stage that was never filled counts as released).
+      for (int i = 0; ok && i < C::kStages; ++i) {
+        ok = mbar_wait(&empty_bar[s], phase ^ 1, abort_word, status, 150 + s);
+        if (++s == C::kStages) {
+          s = 0;
+          phase ^= 1;
+        }
+      }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (converged warp)

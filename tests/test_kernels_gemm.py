@@ -248,6 +248,40 @@ def test_pair_tiles_all_layouts(M, N, K):
         assert ((out.double() - ref).abs() / scale).max().item() < 2 ** -8 + 2e-4
 
 
+@pytest.mark.parametrize("M,N,K,max_ctas", [(4000, 4104, 520, 0), (8192, 2056, 1000, 0), (1016, 1528, 8, 2),
+                                            (504, 760, 72, 2), (512, 744, 384, 7), (496, 504, 392, 5), (1488, 760, 1000, 37)])
+def test_pair_tiles_with_pitched_operands_and_limited_grids(M, N, K, max_ctas):
+    """Column slices of wider matrices as operands and results (fused projections have them), one pair, an odd number of
+    CTAs, from one K block to more than the six stages. Limits as in test_pair_tiles_all_layouts; what lies beside a
+    result stays."""
+    ops, gemm = _ops()
+    plan = ops.ext().gemm_plan
+    for a_mn, b_mn, mode in ((False, False, 0), (False, True, 0), (True, True, 0), (True, True, 2)):
+        pairs, bn, tiles, whole = plan(0, M, N, K, a_mn, b_mn, mode, max_ctas)
+        assert pairs > 0 and (max_ctas == 0 or (pairs == max_ctas // 2 and whole == tiles))
+    torch.manual_seed(M + K)
+
+    def sliced(rows, cols, dtype=torch.bfloat16):
+        return torch.randn(rows, (cols + 31) // 8 * 8, device="cuda").to(dtype)[:, 16:16 + cols]
+    a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, K, device="cuda").to(torch.bfloat16)
+    a_k, a_m, b_k, b_n = sliced(M, K), sliced(K, M), sliced(N, K), sliced(K, N)
+    for view, dense in ((a_k, a), (a_m, a.t()), (b_k, b), (b_n, b.t())):
+        view.copy_(dense)
+    ref = a.double() @ b.double().t()
+    scale = ref.abs().clamp_min(ref.pow(2).mean().sqrt() * 1e-2)
+    for product, x, y in ((gemm.gemm_nt, a_k, b_k), (gemm.gemm_nn, a_k, b_n), (gemm.gemm_tn, a_m, b_n)):
+        wide = torch.full((M, N + 24), 7.0, device="cuda", dtype=torch.bfloat16)
+        product(x, y, out=wide[:, 8:8 + N], max_ctas=max_ctas)
+        ops.check_status("pair gemm")
+        assert ((wide[:, 8:8 + N].double() - ref).abs() / scale).max().item() < 2 ** -8 + 2e-4
+        assert (wide[:, :8] == 7).all() and (wide[:, 8 + N:] == 7).all()
+    acc = sliced(M, N, torch.float32)
+    want = acc.double() + ref
+    gemm.gemm_tn(a_m, b_n, out=acc, accumulate=True, max_ctas=max_ctas)
+    ops.check_status("pair gemm accumulate")
+    assert ((acc.double() - want).norm() / want.norm()).item() < 1e-5
+
+
 @pytest.mark.parametrize("M,N,K", [(520, 776, 4096), (2048, 2048, 1999), (5120, 960, 8192), (576, 264, 16384)])
 def test_pair_tiles_accumulate_with_a_cut_last_round(M, N, K):
     """The last round's tiles are cut along K and added in pieces: fp32 sums, 1e-5 of the 64-bit result, and
