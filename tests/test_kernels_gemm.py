@@ -282,6 +282,19 @@ def test_pair_tiles_with_pitched_operands_and_limited_grids(M, N, K, max_ctas):
     assert ((acc.double() - want).norm() / want.norm()).item() < 1e-5
 
 
+def test_sizes_of_the_pair_tests_run_on_pairs():
+    """The tests of the pair kernel that take their kernel from the size rule, and the cut ones from its cut."""
+    ops, _ = _ops()
+    plan = ops.ext().gemm_plan
+    for M, N, K in ((4000, 4104, 520), (4104, 4000, 72), (8192, 2056, 1000)):
+        assert all(plan(0, M, N, K, a, b, 0, 0)[0] > 0 for a, b in ((False, False), (False, True), (True, True)))
+    for M, N, K in ((520, 776, 4096), (5120, 960, 8192), (576, 264, 16384)):
+        pairs, _, tiles, whole = plan(0, M, N, K, True, True, 2, 0)
+        assert pairs > 0 and whole < tiles
+    pairs, _, tiles, whole = plan(0, 2048, 2048, 1999, True, True, 2, 0)       # 64 tiles on 74 pairs: as they are
+    assert pairs > 0 and whole == tiles
+
+
 @pytest.mark.parametrize("M,N,K", [(520, 776, 4096), (2048, 2048, 1999), (5120, 960, 8192), (576, 264, 16384)])
 def test_pair_tiles_accumulate_with_a_cut_last_round(M, N, K):
     """The last round's tiles are cut along K and added in pieces: fp32 sums, 1e-5 of the 64-bit result, and
