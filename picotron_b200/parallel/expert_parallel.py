@@ -130,7 +130,9 @@ class MoELayer(nn.Module):
 
     # ------------------------------------------------------------------------------ routing
     def _route(self, tokens):
-        logits = self.gate(tokens)
+        return self._route_logits(self.gate(tokens), tokens.dtype)
+
+    def _route_logits(self, logits, dtype):
         if logits.is_cuda and logits.dtype == torch.bfloat16 and self.num_experts <= 256 and self.top_k <= 8 \
                 and os.environ.get("PICO_MOE_DEVICE_ROUTING", "1") != "0":
             # one kernel for softmax + bias + top-k + renormalisation + counts (ops/moe_route.py)
@@ -138,7 +140,7 @@ class MoELayer(nn.Module):
             probs, idx, w, counts = mr.route(logits, self.expert_bias if self.use_loss_free else None, self.top_k,
                                              self.norm_topk_prob)
             self._balance(probs, idx, counts)
-            return idx.long(), w.to(tokens.dtype)
+            return idx.long(), w.to(dtype)
         probs = F.softmax(logits, dim=-1, dtype=torch.float32)
         scores = probs + self.expert_bias.to(probs.dtype) if self.use_loss_free else probs
         topk_idx = torch.topk(scores, self.top_k, dim=-1).indices
@@ -146,7 +148,7 @@ class MoELayer(nn.Module):
         if self.norm_topk_prob and self.top_k > 1:
             topk_w = topk_w / topk_w.sum(dim=-1, keepdim=True)
         self._balance(probs, topk_idx)
-        return topk_idx, topk_w.to(tokens.dtype)
+        return topk_idx, topk_w.to(dtype)
 
     def _balance(self, probs, topk_idx, counts=None):
         """Auxiliary balancing loss and loss-free bias update from this forward pass's routing;
@@ -343,7 +345,7 @@ class MoELayer(nn.Module):
         grouped GEMM take. Nothing of it reads a device value on the host."""
         if self.ep_world_size != 1 or self.ep_capacity_factor > 0 or not tokens.is_cuda \
                 or tokens.dtype != torch.bfloat16 or tokens.shape[0] == 0 or self.num_experts > 256 \
-                or self.top_k > 8 or self.gate.weight.dtype != torch.bfloat16:
+                or self.top_k > 8:
             return False
         if os.environ.get("PICO_MOE_DEVICE_ROUTING", "1") == "0" or self.fused_ep_var is not None:
             return False
@@ -356,6 +358,9 @@ class MoELayer(nn.Module):
         moved each routed row a dozen times and read the counts on the host."""
         from ..ops import moe_route as mr
         logits = self.gate(tokens)
+        if not (logits.is_cuda and logits.dtype == torch.bfloat16 and logits.stride(-1) == 1):
+            # a gate of another kind, or a hook on it, that gives wider logits: they are not rounded for the kernel
+            return self._moe_given_routing(tokens, *self._route_logits(logits, tokens.dtype), False)
         probs, idx, w, counts = mr.route(logits, self.expert_bias if self.use_loss_free else None, self.top_k,
                                          self.norm_topk_prob)
         self._balance(probs, idx, counts)

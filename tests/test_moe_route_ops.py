@@ -323,3 +323,41 @@ def test_tokens_that_are_not_finite_stay_among_themselves(E, k):
     same[[3, 200]] = False
     for a, b in zip(*got):
         assert torch.isnan(b[~same]).all() and torch.equal(a[same], b[same])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["hook", "module"])
+def test_a_gate_that_gives_fp32_logits_keeps_its_route(how, monkeypatch):
+    """Logits that are not bf16 (a forward hook, a gate of the user's own without a ``weight``) are routed in fp32 by
+    the tensor path, as before the local experts had kernels of their own."""
+    from types import SimpleNamespace
+    from picotron_b200 import ops
+    from picotron_b200 import process_group_manager as pgm
+    from picotron_b200.parallel.expert_parallel import MoELayer
+    if pgm.process_group_manager is None:
+        pgm.setup_process_group_manager(1, 1, 1, 1, 1)
+    torch.manual_seed(11)
+    with torch.device("cuda"):
+        layer = MoELayer(SimpleNamespace(hidden_size=256, intermediate_size=256, num_experts=8,
+                                         num_experts_per_tok=2)).to(torch.bfloat16)
+    if how == "hook":
+        layer.gate.register_forward_hook(lambda mod, args, out: out.float() * 1.0009765625)
+    else:
+        class Gate(torch.nn.Module):
+            def __init__(self):
+                super().__init__()
+                self.table = torch.nn.Parameter(torch.randn(256, 8, device="cuda"))
+
+            def forward(self, x):
+                return x.float() @ self.table
+        layer.gate = Gate()
+    x = torch.randn(300, 256, device="cuda", dtype=torch.bfloat16)
+    got = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("PICO_MOE_DEVICE_ROUTING", flag)
+        layer.zero_grad(set_to_none=True)
+        y = layer(x)
+        y.float().square().sum().backward()
+        got.append([y.detach()] + [p.grad.clone() for p in layer.parameters()])
+    ops.check_status("moe layer")
+    assert all(torch.equal(a, b) for a, b in zip(*got))
