@@ -361,3 +361,50 @@ def test_a_gate_that_gives_fp32_logits_keeps_its_route(how, monkeypatch):
         got.append([y.detach()] + [p.grad.clone() for p in layer.parameters()])
     ops.check_status("moe layer")
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("renorm,aux,bias_rate", [(False, 0.0, 0.0), (True, 0.01, 0.0), (True, 0.0, 0.05), (False, 0.02, 0.1)])
+def test_local_experts_layer_balances_like_the_tensor_path(renorm, aux, bias_rate, monkeypatch):
+    """Raw router probabilities as weights, the auxiliary loss (its dense gradient enters the router beside the
+    weights') and the loss-free bias (selection by probability + bias, update from the kernel's counts): outputs,
+    gradients, loss and bias against the layer on sorted, padded tensors over three steps. The tensor path rounds the
+    weights to bf16, so outputs and gradients may differ by that and their own rounding, 2^-8 each."""
+    from types import SimpleNamespace
+    from picotron_b200 import ops
+    from picotron_b200 import process_group_manager as pgm
+    from picotron_b200.parallel.expert_parallel import MoELayer
+    if pgm.process_group_manager is None:
+        pgm.setup_process_group_manager(1, 1, 1, 1, 1)
+    torch.manual_seed(7)
+    with torch.device("cuda"):
+        layer = MoELayer(SimpleNamespace(hidden_size=256, intermediate_size=256, num_experts=16, num_experts_per_tok=3,
+                                         norm_topk_prob=renorm, router_aux_loss_coef=aux,
+                                         router_bias_update_rate=bias_rate)).to(torch.bfloat16)
+    layer.train()
+    layer.expert_bias = layer.expert_bias.float()
+    xs = [torch.randn(700, 256, device="cuda", dtype=torch.bfloat16) for _ in range(3)]
+    dy = torch.randn(700, 256, device="cuda", dtype=torch.bfloat16)
+    got = []
+    for flag in ("1", "0"):
+        monkeypatch.setenv("PICO_MOE_DEVICE_ROUTING", flag)
+        layer.expert_bias.zero_()
+        layer.zero_grad(set_to_none=True)
+        values, exact = [], []
+        for x0 in xs:
+            x = x0.clone().requires_grad_()
+            assert layer._local_routed_ok(x) == (flag == "1")
+            y = layer(x)
+            loss = (y * dy).float().sum()
+            assert (layer.aux_loss is not None) == (aux > 0)
+            if aux > 0:
+                values.append(layer.aux_loss.detach().reshape(1))
+                loss = loss + 1000.0 * layer.aux_loss
+            loss.backward()
+            values += [y.detach(), x.grad]
+            exact.append(layer.expert_bias.clone())
+        got.append((values + [p.grad.clone() for p in layer.parameters()], exact))
+    ops.check_status("moe layer")
+    for a, b in zip(got[0][0], got[1][0]):
+        assert ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)).item() < 2 ** -6
+    assert all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1])) and (got[0][1][-1].any().item() == (bias_rate > 0))
