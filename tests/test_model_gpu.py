@@ -63,3 +63,77 @@ def test_logits_without_gradients_are_the_same_bits(batch, seq):
         without = engine.model(ids)
     ops.check_status("forward")
     assert not without.requires_grad and torch.equal(with_grad, without)
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_launches_ahead_keep_the_order_of_forked_streams(captured):
+    """Kernels set up beside their predecessor wait for everything their stream waits for: a long product, a fork to
+    another stream that reads it, work on both, and a join, launched right behind the event waits as the captured
+    tensor-parallel micro-batches do. Eager and replayed, with new inputs each time, against one stream with a
+    synchronisation after every step (the same kernels, so the same bits)."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import gemm, norm, swiglu
+    torch.manual_seed(0)
+    d = 2048
+
+    def new():
+        return torch.randn(d, d, device="cuda", dtype=torch.bfloat16)
+    x, w1, w2, w3, scale = new(), new() * 0.02, new() * 0.02, new() * 0.02, torch.ones(d, device="cuda", dtype=torch.bfloat16)
+    side = torch.cuda.Stream()
+    big = torch.randn(6144, 6144, device="cuda", dtype=torch.bfloat16)
+
+    def steps(fork, join, sync):
+        with torch.no_grad():
+            out = []
+            for _ in range(3):
+                gemm.gemm_nt(big, big)                   # holds the SMs while the next ones are set up
+                a = gemm.gemm_nt(x, w1)
+                sync()
+                with fork():
+                    b = norm.rmsnorm(a, scale, 1e-5)     # launched ahead behind an event wait only
+                    c = gemm.gemm_nt(b, w2)
+                e = swiglu.swiglu(a)
+                f = gemm.gemm_nt(a, w3)
+                sync()
+                join()
+                g = gemm.gemm_nt(c, f)                   # launched ahead behind a kernel of each stream
+                h, r = norm.add_rmsnorm(g, c, scale, 1e-5)
+                sync()
+                out += [a, b, c, e, f, g, h, r]
+            return out
+
+    class on_side:
+        def __enter__(self):
+            side.wait_stream(torch.cuda.current_stream())
+            self.ctx = torch.cuda.stream(side)
+            self.ctx.__enter__()
+
+        def __exit__(self, *args):
+            self.ctx.__exit__(*args)
+
+    def back():
+        torch.cuda.current_stream().wait_stream(side)
+
+    def forked():
+        return steps(on_side, back, lambda: None)
+
+    def alone():
+        import contextlib
+        return steps(contextlib.nullcontext, lambda: None, torch.cuda.synchronize)
+    forked()
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            held = forked()
+    for _ in range(4):
+        x.copy_(new())
+        want = [t.clone() for t in alone()]
+        if captured:
+            graph.replay()
+            got = held
+        else:
+            got = forked()
+        torch.cuda.synchronize()
+        assert all(torch.equal(p, q) for p, q in zip(want, got))
+    ops.check_status("forked streams")
