@@ -402,18 +402,18 @@ moe_scatter_sum_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __res
   for (int t = warp; t < T; t += nwarps) {
     int slot[kMaxTopK];
     float wt[kMaxTopK];
+    bool lost = false;
 #pragma unroll
     for (int j = 0; j < kMaxTopK; ++j) {
       slot[j] = j < k ? slot_of_row[(int64_t)t * k + j] : 0;
       wt[j] = kHasW && j < k ? w[(int64_t)t * k + j] : 1.f;
+      lost |= slot[j] < 0;
     }
     for (int v = lane; v < nvec; v += 32) {
       uint4 raw[kMaxTopK];               // all k rows' loads in flight
 #pragma unroll
       for (int j = 0; j < kMaxTopK; ++j)
-        if (j < k)
-          raw[j] = slot[j] >= 0 ? reinterpret_cast<const uint4*>(x + (int64_t)slot[j] * d)[v]
-                                : make_uint4(~0u, ~0u, ~0u, ~0u);     // bf16 NaNs
+        if (j < k) raw[j] = reinterpret_cast<const uint4*>(x + (int64_t)max(slot[j], 0) * d)[v];
       float acc[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -433,6 +433,7 @@ moe_scatter_sum_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __res
       __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
 #pragma unroll
       for (int i = 0; i < 4; ++i) oh[i] = __floats2bfloat162_rn(acc[2 * i], acc[2 * i + 1]);
+      if (lost) o = make_uint4(~0u, ~0u, ~0u, ~0u);       // bf16 NaNs
       reinterpret_cast<uint4*>(y + (int64_t)t * d)[v] = o;
     }
   }
