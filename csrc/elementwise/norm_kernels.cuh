@@ -266,9 +266,10 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
       rstd[r] = row < rows ? rstd_in[row] : 0.f;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        const size_t off = (size_t)min(row, rows - 1) * nvec + threadIdx.x + i * kNormThreads;
-        draw[r][i] = reinterpret_cast<const uint4*>(dy)[off];
-        hraw[r][i] = reinterpret_cast<const uint4*>(h)[off];
+        // zeros past the end: a copy of the last row times rstd = 0 would be NaN where that row has an infinity
+        const size_t off = (size_t)row * nvec + threadIdx.x + i * kNormThreads;
+        draw[r][i] = row < rows ? reinterpret_cast<const uint4*>(dy)[off] : make_uint4(0, 0, 0, 0);
+        hraw[r][i] = row < rows ? reinterpret_cast<const uint4*>(h)[off] : make_uint4(0, 0, 0, 0);
       }
     }
     float dot[R];
@@ -283,7 +284,7 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat1
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           dot[r] += d[j] * wv[i][j] * hv[j];
-          dw_acc[i][j] += d[j] * hv[j] * rstd[r];      // rstd = 0 for rows past the end
+          dw_acc[i][j] += d[j] * hv[j] * rstd[r];
         }
       }
       dot[r] = warp_sum(dot[r]);
@@ -369,9 +370,9 @@ rmsnorm_bwd_rows_pf_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
       rnext[r] = row < rows ? rstd_in[row] : 0.f;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        const size_t off = (size_t)min(row, rows - 1) * nvec + col;
-        dnext[r][i] = reinterpret_cast<const uint4*>(dy)[off];
-        hnext[r][i] = reinterpret_cast<const uint4*>(h)[off];
+        const size_t off = (size_t)row * nvec + col;      // zeros past the end, as above
+        dnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(dy)[off] : make_uint4(0, 0, 0, 0);
+        hnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(h)[off] : make_uint4(0, 0, 0, 0);
       }
     }
   }
@@ -395,9 +396,9 @@ rmsnorm_bwd_rows_pf_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
         rnext[r] = row < rows ? rstd_in[row] : 0.f;
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
-          const size_t off = (size_t)min(row, rows - 1) * nvec + col;
-          dnext[r][i] = reinterpret_cast<const uint4*>(dy)[off];
-          hnext[r][i] = reinterpret_cast<const uint4*>(h)[off];
+          const size_t off = (size_t)row * nvec + col;      // zeros past the end, as above
+          dnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(dy)[off] : make_uint4(0, 0, 0, 0);
+          hnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(h)[off] : make_uint4(0, 0, 0, 0);
         }
       }
     }
@@ -413,7 +414,7 @@ rmsnorm_bwd_rows_pf_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           if (act) dot[r] += d[j] * wv[i][j] * hv[j];
-          dw_acc[i][j] += d[j] * hv[j] * rstd[r];      // rstd = 0 for rows past the end
+          dw_acc[i][j] += d[j] * hv[j] * rstd[r];
         }
       }
       dot[r] = warp_sum(dot[r]);

@@ -192,3 +192,22 @@ def test_rmsnorm_row_widths_against_64_bits(rows, H, residual):
     for got, exp in ((y, y6.detach()), (grads[0], want[0]), (grads[1], want[1])):
         scale = exp.abs().clamp_min(exp.pow(2).mean().sqrt())
         assert ((got.double() - exp).abs() / scale).max().item() < 2 ** -8 + 1e-5
+
+
+@pytest.mark.parametrize("rows,H", [(1, 576), (3, 960), (301, 2048), (5, 4096), (5, 1032), (7, 2056)])
+def test_rmsnorm_backward_keeps_infinities_where_they_are(rows, H):
+    """An infinity in the last row's gradient (rows are worked on two at a time) makes its own column of the weight
+    gradient infinite, not NaN, and leaves the other columns and rows alone."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import norm
+    torch.manual_seed(H)
+    x = torch.randn(rows, H, device="cuda", dtype=torch.bfloat16).abs_().add_(0.5).requires_grad_()
+    w = torch.ones(H, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    dy = torch.randn(rows, H, device="cuda", dtype=torch.bfloat16)
+    clean = torch.autograd.grad(norm.rmsnorm(x, w, 1e-5), (x, w), dy)
+    dy[-1, 5] = float("inf")
+    dx, dw = torch.autograd.grad(norm.rmsnorm(x, w, 1e-5), (x, w), dy)
+    ops.check_status("rmsnorm")
+    others = torch.arange(H, device="cuda") != 5
+    assert dw[5].item() == float("inf") and torch.equal(dw[others], clean[1][others])
+    assert torch.equal(dx[:-1], clean[0][:-1]) and not dx[-1].isfinite().any()
