@@ -21,7 +21,8 @@
 // threads per key row, 32 queries each, 704 threads of 80 registers): with 8 the exponentials of a tile took
 // 1800 cycles against 1024 for the special-function unit (a warp's dependent instructions issue every 3
 // cycles; 16384 tokens: 3510 and 3284 us). W = 8 at head_dim 128, where the tensor cores have more to do and the
-// drain, which dP of the next step waits for, holds two chunks in registers (437 us; with 16 warps 499). The MMA warp issues
+// drain, which dP of the next step waits for, holds two chunks in registers (437 us; with 16 warps 499).
+// The MMA warp issues
 //   dV(i) S(i+1) | dK(i) dQ(i) dP(i+1)
 // so that the exponentials of step i+1 run under dK(i) / dQ(i) / dP(i+1) and the dS arithmetic under
 // dV(i+1) / S(i+2); the two score tiles need no second buffer:
@@ -63,7 +64,8 @@ struct BwdCfg {
   static constexpr int kStaging = 2 * 128 * 128;            // two fp32 dQ chunks of 32 columns
   static constexpr int kTiles = (2 + kQStages + kDoStages) * kTile + kDs + kStaging;
   static constexpr int kStats = 2 * 2 * 128 * 4;            // lse and delta of the queries, two stages
-  // kv_full, q_full/q_empty, do_full/do_empty, stat_full[2], s_full, p_ready, dp_full, ds_ready, dq_full, dq_free, all_done
+  // kv_full, q_full/q_empty, do_full/do_empty, stat_full[2], s_full, p_ready, dp_full, ds_ready, dq_full, dq_free,
+  // all_done
   static constexpr int kNumBars = 1 + 2 * kQStages + 2 * kDoStages + 2 + 7;
   static constexpr int kSmemBytes = kTiles + kStats + kNumBars * 8 + 16;
   static constexpr int kPanels = D / 64;
@@ -316,7 +318,8 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
           tc_mma_f16_ss_warp(d_tmem, a_d + off, b_d + off, idesc_s, kk != 0 ? 1u : 0u);
         }
       };
-      bool ok = mbar_wait_warp(kv_full, 0, abort_word, status, 2000) && mbar_wait_warp(&q_full[0], 0, abort_word, status, 2020);
+      bool ok = mbar_wait_warp(kv_full, 0, abort_word, status, 2000) &&
+                mbar_wait_warp(&q_full[0], 0, abort_word, status, 2020);
       if (ok) {
         tc_fence_after();
         issue_scores(tmem_base + Cfg::kTmS, k_d, q_d);
@@ -334,8 +337,9 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)   // contraction over the 128 queries, 16 (8 packed columns) per step
-          tc_mma_f16_ts_warp(tmem_base + Cfg::kTmDv, tmem_base + Cfg::kTmP + kk / Cfg::kSteps * Cfg::kTmPPart + kk % Cfg::kSteps * 8,
-                        do_mn + ds * kStep + (kk * 2048 >> 4), idesc_v, (it | kk) != 0 ? 1u : 0u);
+          tc_mma_f16_ts_warp(tmem_base + Cfg::kTmDv,
+                             tmem_base + Cfg::kTmP + kk / Cfg::kSteps * Cfg::kTmPPart + kk % Cfg::kSteps * 8,
+                             do_mn + ds * kStep + (kk * 2048 >> 4), idesc_v, (it | kk) != 0 ? 1u : 0u);
         tc_commit_warp(&do_empty[ds]);
         if (it + 1 < total) {
           const int nq = (it + 1) % Cfg::kQStages;
@@ -348,8 +352,9 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
         tc_fence_after();
 #pragma unroll
         for (int kk = 0; kk < 8; ++kk)
-          tc_mma_f16_ts_warp(tmem_base + Cfg::kTmDk, tmem_base + Cfg::kTmDp + kk / Cfg::kSteps * Cfg::kCols + kk % Cfg::kSteps * 8,
-                        q_mn + qs * kStep + (kk * 2048 >> 4), idesc_v, (it | kk) != 0 ? 1u : 0u);
+          tc_mma_f16_ts_warp(tmem_base + Cfg::kTmDk,
+                             tmem_base + Cfg::kTmDp + kk / Cfg::kSteps * Cfg::kCols + kk % Cfg::kSteps * 8,
+                             q_mn + qs * kStep + (kk * 2048 >> 4), idesc_v, (it | kk) != 0 ? 1u : 0u);
         tc_commit_warp(&q_empty[qs]);
         // dQ has its own columns at head_dim 64: the previous tile must have been drained; at head_dim 128
         // that wait came before dP(it), whose columns it shares
@@ -493,8 +498,10 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
       for (int c = 0; c < kCols; c += 4) {
         const float4 nl = *reinterpret_cast<const float4*>(st + c);     // -lse * log2(e), the same for all lanes
         float e0, e1, e2, e3;
-        f2_unpack(f2_fma(f2_pack(__uint_as_float(pr[c]), __uint_as_float(pr[c + 1])), scale2, f2_pack(nl.x, nl.y)), e0, e1);
-        f2_unpack(f2_fma(f2_pack(__uint_as_float(pr[c + 2]), __uint_as_float(pr[c + 3])), scale2, f2_pack(nl.z, nl.w)), e2, e3);
+        const uint64_t s01 = f2_pack(__uint_as_float(pr[c]), __uint_as_float(pr[c + 1]));
+        const uint64_t s23 = f2_pack(__uint_as_float(pr[c + 2]), __uint_as_float(pr[c + 3]));
+        f2_unpack(f2_fma(s01, scale2, f2_pack(nl.x, nl.y)), e0, e1);
+        f2_unpack(f2_fma(s23, scale2, f2_pack(nl.z, nl.w)), e2, e3);
         e0 = exp2f(e0);
         e1 = exp2f(e1);
         e2 = exp2f(e2);
@@ -531,12 +538,12 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
         for (int c = 0; c < 32; c += 4) {
           const float4 nd = *reinterpret_cast<const float4*>(st + 128 + h + c);   // -delta
           float s0, s1, s2, s3;
-          f2_unpack(f2_mul(f2_pack(__uint_as_float(pr[h + c]), __uint_as_float(pr[h + c + 1])),
-                           f2_add(f2_pack(__uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1])), f2_pack(nd.x, nd.y))),
-                    s0, s1);
-          f2_unpack(f2_mul(f2_pack(__uint_as_float(pr[h + c + 2]), __uint_as_float(pr[h + c + 3])),
-                           f2_add(f2_pack(__uint_as_float(dpv[c + 2]), __uint_as_float(dpv[c + 3])), f2_pack(nd.z, nd.w))),
-                    s2, s3);
+          const uint64_t p01 = f2_pack(__uint_as_float(pr[h + c]), __uint_as_float(pr[h + c + 1]));
+          const uint64_t p23 = f2_pack(__uint_as_float(pr[h + c + 2]), __uint_as_float(pr[h + c + 3]));
+          const uint64_t d01 = f2_pack(__uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1]));
+          const uint64_t d23 = f2_pack(__uint_as_float(dpv[c + 2]), __uint_as_float(dpv[c + 3]));
+          f2_unpack(f2_mul(p01, f2_add(d01, f2_pack(nd.x, nd.y))), s0, s1);
+          f2_unpack(f2_mul(p23, f2_add(d23, f2_pack(nd.z, nd.w))), s2, s3);
           dsp[c / 2] = pack_bf16x2(s0, s1);
           dsp[c / 2 + 1] = pack_bf16x2(s2, s3);
         }
@@ -639,9 +646,9 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
     attr_dev = dev;
   }
   dim3 grid(p->kv_heads, p->batch, (p->seq_k + kBN - 1) / kBN);
-  pico_host::launch_ahead(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, maps, lse, delta, (__nv_bfloat16*)dk, (__nv_bfloat16*)dv,
-                                                      *p, dk_batch_stride, dk_row_stride, dv_batch_stride,
-                                                      dv_row_stride, pico_status_buffer());
+  pico_host::launch_ahead(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, maps, lse, delta, (__nv_bfloat16*)dk,
+                          (__nv_bfloat16*)dv, *p, dk_batch_stride, dk_row_stride, dv_batch_stride, dv_row_stride,
+                          pico_status_buffer());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     pico_host::set_error("attention bwd launch: %s", cudaGetErrorString(e));
@@ -673,8 +680,8 @@ extern "C" int pico_attention_bwd(const void* q, const void* k, const void* v, c
   {
     int64_t blocks = (rows * (p->head_dim / 8) + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    pico_host::launch_ahead(attn_delta_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)out, (const __nv_bfloat16*)dout, delta,
-                                                      dq_accum, *p, do_batch_stride, do_row_stride);
+    pico_host::launch_ahead(attn_delta_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)out,
+                            (const __nv_bfloat16*)dout, delta, dq_accum, *p, do_batch_stride, do_row_stride);
   }
   int rc;
   if (p->head_dim == 64)
@@ -688,8 +695,8 @@ extern "C" int pico_attention_bwd(const void* q, const void* k, const void* v, c
     int64_t nvec = rows * p->head_dim / 8;
     int64_t blocks = (nvec + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    pico_host::launch_ahead(attn_dq_convert_kernel, (int)blocks, 256, 0, stream, dq_accum, (__nv_bfloat16*)dq, *p, dq_batch_stride,
-                                                           dq_row_stride);
+    pico_host::launch_ahead(attn_dq_convert_kernel, (int)blocks, 256, 0, stream, dq_accum, (__nv_bfloat16*)dq, *p,
+                            dq_batch_stride, dq_row_stride);
   }
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

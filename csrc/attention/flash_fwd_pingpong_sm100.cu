@@ -504,7 +504,8 @@ static int launch(const void* q, const void* k, const void* v, void* out, float*
     attr_dev = dev;
   }
   dim3 grid(p->heads, p->batch, (p->seq_q + kCtaM - 1) / kCtaM);
-  pico_host::launch_ahead(kern, grid, kThreads, C::kSmemBytes, stream, maps, (__nv_bfloat16*)out, lse, *p, pico_status_buffer());
+  pico_host::launch_ahead(kern, grid, kThreads, C::kSmemBytes, stream, maps, (__nv_bfloat16*)out, lse, *p,
+                          pico_status_buffer());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     pico_host::set_error("attention fwd launch: %s", cudaGetErrorString(e));

@@ -5,6 +5,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <array>
 #include <cstring>
 
 #include "attention/attention.h"
@@ -56,16 +57,28 @@ void gemm(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, int64_t M, in
         "gemm");
 }
 
-void gemm_parts(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, at::Tensor& slabs, int64_t M, int64_t N, int64_t K,
-                bool b_mn_major, int64_t parts) {
+// (pairs at work or 0, tile width, 256 x 256 tiles, tiles that are not cut) of such a product on `sms` SMs (0: this
+// device's)
+std::array<int, 4> gemm_plan(int64_t sms, int64_t M, int64_t N, int64_t K, bool a_mn_major, bool b_mn_major,
+                             int64_t out_mode, int64_t max_ctas) {
+  std::array<int, 4> plan;
+  check(pico_gemm_plan((int)sms, (int)M, (int)N, (int)K, a_mn_major, b_mn_major, (int)out_mode, (int)max_ctas, 1,
+                       plan.data()),
+        "gemm_plan");
+  return plan;
+}
+
+void gemm_parts(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, at::Tensor& slabs, int64_t M, int64_t N,
+                int64_t K, bool b_mn_major, int64_t parts) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda() && D.is_cuda() && slabs.is_cuda(), "gemm_parts: CUDA tensors required");
-  TORCH_CHECK(A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16 && D.scalar_type() == at::kBFloat16 &&
-                  slabs.scalar_type() == at::kFloat && slabs.is_contiguous(),
+  TORCH_CHECK(A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16 &&
+                  D.scalar_type() == at::kBFloat16 && slabs.scalar_type() == at::kFloat && slabs.is_contiguous(),
               "gemm_parts: bf16 operands, fp32 scratch");
   TORCH_CHECK(slabs.numel() >= parts * ((M + 127) / 128) * 128 * N, "gemm_parts: scratch too small");
   c10::cuda::CUDAGuard guard(A.device());
   check(pico_gemm_bf16_parts(A.data_ptr(), B.data_ptr(), D.data_ptr(), slabs.data_ptr<float>(), (int)M, (int)N, (int)K,
-                             (int)A.stride(0), (int)B.stride(0), (int)D.stride(0), b_mn_major, (int)parts, stream_of(A)),
+                             (int)A.stride(0), (int)B.stride(0), (int)D.stride(0), b_mn_major, (int)parts,
+                             stream_of(A)),
         "gemm_parts");
 }
 
@@ -111,11 +124,12 @@ std::tuple<at::Tensor, at::Tensor, int64_t> linear_fwd(const at::Tensor& x, cons
 }
 
 // (norm(x + residual), x + residual or x, 1 / rms) of [rows, H] rows
-std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_new(const at::Tensor& x, const c10::optional<at::Tensor>& residual,
+std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_new(const at::Tensor& x,
+                                                           const c10::optional<at::Tensor>& residual,
                                                            const at::Tensor& w, double eps) {
   const int64_t H = x.size(-1);
-  TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && w.is_contiguous() && w.numel() == H &&
-                  x.is_cuda() && w.is_cuda(),
+  TORCH_CHECK(x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 && w.is_contiguous() &&
+                  w.numel() == H && x.is_cuda() && w.is_cuda(),
               "rmsnorm: bf16 CUDA rows and a weight of their width");
   c10::cuda::CUDAGuard guard(x.device());
   at::Tensor x2 = x.reshape({-1, H}).contiguous();
@@ -323,7 +337,8 @@ void moe_layout(const at::Tensor& idx, const at::Tensor& counts, at::Tensor& slo
         "moe_layout");
 }
 
-void moe_gather(const at::Tensor& x, const at::Tensor& row_of_slot, const at::Tensor& used, at::Tensor& out, int64_t k) {
+void moe_gather(const at::Tensor& x, const at::Tensor& row_of_slot, const at::Tensor& used, at::Tensor& out,
+                int64_t k) {
   c10::cuda::CUDAGuard guard(x.device());
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && x.is_contiguous() && out.scalar_type() == at::kBFloat16 &&
                   out.is_contiguous() && x.dim() == 2 && out.dim() == 2 && x.size(1) == out.size(1) &&
@@ -342,7 +357,8 @@ void moe_scatter_sum(const at::Tensor& x, const at::Tensor& slot_of_row, const c
   const bool has_w = w.has_value() && w->defined();
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && x.is_contiguous() && y.scalar_type() == at::kBFloat16 &&
                   y.is_contiguous() && x.dim() == 2 && y.dim() == 2 && x.size(1) == y.size(1) &&
-                  slot_of_row.scalar_type() == at::kInt && slot_of_row.is_contiguous() && slot_of_row.numel() == T * k &&
+                  slot_of_row.scalar_type() == at::kInt && slot_of_row.is_contiguous() &&
+                  slot_of_row.numel() == T * k &&
                   (!has_w || (w->scalar_type() == at::kFloat && w->is_contiguous() && w->numel() == T * k)),
               "moe_scatter_sum: tensors of the wrong type or size");
   check(pico_moe_scatter_sum(x.data_ptr(), slot_of_row.data_ptr<int>(), has_w ? w->data_ptr<float>() : nullptr,
@@ -810,7 +826,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
                                                                  const at::Tensor& out_, const at::Tensor& lse,
                                                                  double sm_scale, bool causal, int64_t q_pos0,
                                                                  int64_t k_pos0) {
-  at::Tensor q = pack_heads(q_), k = pack_heads(k_), v = pack_heads(v_), out = pack_heads(out_), dout = pack_heads(dout_);
+  at::Tensor q = pack_heads(q_), k = pack_heads(k_), v = pack_heads(v_);
+  at::Tensor out = pack_heads(out_), dout = pack_heads(dout_);
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && dout.sizes() == q.sizes() &&
                   out.sizes() == q.sizes(),
               "attention_bwd: out and its gradient have the shape of q, fp32 contiguous lse");
@@ -845,12 +862,9 @@ std::vector<int64_t> status_fetch() {
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm", &gemm);
   m.def("gemm_parts", &gemm_parts);
-  m.def("gemm_parts_of_k", [](int64_t M, int64_t N, int64_t K) { return pico_gemm_parts_of_k((int)M, (int)N, (int)K); });
-  m.def("gemm_plan", [](int64_t sms, int64_t M, int64_t N, int64_t K, bool a_mn, bool b_mn, int64_t out_mode, int64_t max_ctas) {
-    std::array<int, 4> plan;
-    check(pico_gemm_plan((int)sms, (int)M, (int)N, (int)K, a_mn, b_mn, (int)out_mode, (int)max_ctas, 1, plan.data()), "gemm_plan");
-    return plan;
-  });
+  m.def("gemm_parts_of_k",
+        [](int64_t M, int64_t N, int64_t K) { return pico_gemm_parts_of_k((int)M, (int)N, (int)K); });
+  m.def("gemm_plan", &gemm_plan);
   m.def("gemm_new", &gemm_new);
   m.def("linear_fwd", &linear_fwd);
   m.def("rmsnorm_new", &rmsnorm_new);

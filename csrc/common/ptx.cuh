@@ -90,7 +90,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-
 // Bounded wait. `abort_word` lives in shared memory; once any role sets it, every wait
 // in the CTA gives up immediately. Returns false when the wait was abandoned.
 constexpr uint64_t PICO_MBAR_TIMEOUT_NS = 2000ull * 1000ull * 1000ull;  // 2 s
@@ -416,7 +415,7 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
       : "memory");
 }
 // D[256 x N over both CTAs' tensor memory] (+)= A[256 x 16] * B[16 x N]; an elected lane of the first CTA's
-// converged warp issues, the // descriptors hold for both CTAs (each holds 128 rows of A and N/2 columns of B)
+// converged warp issues, the descriptors hold for both CTAs (each holds 128 rows of A and N/2 columns of B)
 __device__ __forceinline__ void tc_mma_f16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b,
                                                    uint32_t idesc, uint32_t accumulate) {
   asm volatile(

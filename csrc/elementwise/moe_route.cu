@@ -608,7 +608,8 @@ extern "C" int pico_moe_combine_bwd(const void* dy, const void* out, const int32
   }
   if (slots <= 0) return 0;
   moe_combine_bwd_kernel<<<warp_grid(slots), 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)out,
-                                                              row_of_slot, w, used, (__nv_bfloat16*)dout, dw, slots, k, d);
+                                                              row_of_slot, w, used, (__nv_bfloat16*)dout, dw, slots,
+                                                              k, d);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) pico_host::set_error("moe_combine_bwd: %s", cudaGetErrorString(e));
   return (int)e;

@@ -5,9 +5,10 @@
 //   backward:  g = dy * w;  dh = rstd * g - h * rstd^3 * mean(g * h) (+ dres);
 //              dw = sum_rows(dy * h * rstd)
 //
-// One CTA of 256 threads owns a row at a time (persistent over rows in the backward so
-// the weight-gradient partials stay in registers); all global traffic is 16-byte vectors.
-// The hidden size must be a multiple of 8.
+// Forward: a warp per row where rows are narrow and many, else a CTA of 256 threads per row. Backward: persistent
+// CTAs, so the weight-gradient partials stay in registers; up to H = 2048 and at 4096 two rows at a time, with the
+// threads that the width needs up to 2048. All global traffic is 16-byte vectors; the hidden size must be a multiple
+// of 8.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -50,7 +51,11 @@ extern "C" int pico_rmsnorm_fwd(const void* x, const void* residual, const void*
     const __nv_bfloat16* b = (const __nv_bfloat16*)residual;
     const __nv_bfloat16* c = (const __nv_bfloat16*)w;
     switch ((H / 8 + 31) / 32) {
-#define PICO_W(N) case N: pico_host::launch_ahead(pico::rmsnorm_fwd_warp_kernel<N>, warp_grid, pico::kNormThreads, 0, stream, a, b, c, (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, H, eps); break;
+#define PICO_W(N)                                                                                               \
+  case N:                                                                                                       \
+    pico_host::launch_ahead(pico::rmsnorm_fwd_warp_kernel<N>, warp_grid, pico::kNormThreads, 0, stream, a, b, c, \
+                            (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, H, eps);                      \
+    break;
       PICO_W(1) PICO_W(2) PICO_W(3) PICO_W(4)
 #undef PICO_W
     }
@@ -60,9 +65,9 @@ extern "C" int pico_rmsnorm_fwd(const void* x, const void* residual, const void*
   }
   int grid = rows < pico_host::num_sms() * 8 ? rows : pico_host::num_sms() * 8;
   int rc = pico::pick_nv(H, [&](auto nv) {
-    pico_host::launch_ahead(pico::rmsnorm_fwd_kernel<decltype(nv)::value>, grid, pico::kNormThreads, 0, stream, 
-        (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w,
-        (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, H, eps);
+    pico_host::launch_ahead(pico::rmsnorm_fwd_kernel<decltype(nv)::value>, grid, pico::kNormThreads, 0, stream,
+                            (const __nv_bfloat16*)x, (const __nv_bfloat16*)residual, (const __nv_bfloat16*)w,
+                            (__nv_bfloat16*)y, (__nv_bfloat16*)h_out, rstd, rows, H, eps);
     return 0;
   });
   if (rc) return rc;
@@ -92,11 +97,13 @@ extern "C" int pico_rmsnorm_bwd(const void* dy, const void* h, const void* w, co
     const __nv_bfloat16* c = (const __nv_bfloat16*)w;
     const __nv_bfloat16* d = (const __nv_bfloat16*)dres;
     __nv_bfloat16* o = (__nv_bfloat16*)dh;
-    // two rows per step with the next two in flight: 78 registers at 256 threads, three CTAs resident per SM and
+    // two rows per step with the next two in flight: 80 registers at 256 threads, three CTAs resident per SM and
     // exactly that many launched (48 us against 58 us for four rows per step without prefetch)
     const int most = H > 1536 && H <= 2048 ? pico_host::num_sms() * 3 : max_parts;
     const int parts = (rows + 1) / 2 < most ? (rows + 1) / 2 : most;
-#define PICO_ROWS(T) pico_host::launch_ahead(pico::rmsnorm_bwd_rows_pf_kernel<T, 2>, parts, T, 0, stream, a, b, c, rstd, d, o, dw_partial, rows, H)
+#define PICO_ROWS(T)                                                                                         \
+  pico_host::launch_ahead(pico::rmsnorm_bwd_rows_pf_kernel<T, 2>, parts, T, 0, stream, a, b, c, rstd, d, o, \
+                          dw_partial, rows, H)
     if (H <= 512)
       PICO_ROWS(64);
     else if (H <= 768)
@@ -108,23 +115,24 @@ extern "C" int pico_rmsnorm_bwd(const void* dy, const void* h, const void* w, co
     else if (H <= 2048)
       PICO_ROWS(256);
     else
-      pico_host::launch_ahead(pico::rmsnorm_bwd_rows_kernel<2, 2>, parts, pico::kNormThreads, 0, stream, a, b, c, rstd, d, o, dw_partial, rows, H);
+      pico_host::launch_ahead(pico::rmsnorm_bwd_rows_kernel<2, 2>, parts, pico::kNormThreads, 0, stream, a, b, c, rstd,
+                              d, o, dw_partial, rows, H);
 #undef PICO_ROWS
     pico_host::launch_ahead(pico::colsum_kernel, (H + 31) / 32, 1024, 0, stream, dw_partial, parts, H, dw_f32,
-                                                             (__nv_bfloat16*)dw_bf16, accumulate);
+                            (__nv_bfloat16*)dw_bf16, accumulate);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) pico_host::set_error("rmsnorm_bwd: %s", cudaGetErrorString(e));
     return (int)e;
   }
   int rc = pico::pick_nv(H, [&](auto nv) {
-    pico_host::launch_ahead(pico::rmsnorm_bwd_kernel<decltype(nv)::value>, grid, pico::kNormThreads, 0, stream, 
-        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd,
-        (const __nv_bfloat16*)dres, (__nv_bfloat16*)dh, dw_partial, rows, H);
+    pico_host::launch_ahead(pico::rmsnorm_bwd_kernel<decltype(nv)::value>, grid, pico::kNormThreads, 0, stream,
+                            (const __nv_bfloat16*)dy, (const __nv_bfloat16*)h, (const __nv_bfloat16*)w, rstd,
+                            (const __nv_bfloat16*)dres, (__nv_bfloat16*)dh, dw_partial, rows, H);
     return 0;
   });
   if (rc) return rc;
   pico_host::launch_ahead(pico::colsum_kernel, (H + 31) / 32, 1024, 0, stream, dw_partial, grid, H, dw_f32,
-                                                           (__nv_bfloat16*)dw_bf16, accumulate);
+                          (__nv_bfloat16*)dw_bf16, accumulate);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) pico_host::set_error("rmsnorm_bwd: %s", cudaGetErrorString(e));
   return (int)e;

@@ -234,8 +234,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // Row-group variant for H = 2048 * NV: one CTA works on R rows at a time, every thread owning NV
 // vectors of 8 columns of each row. The R row dot products share one pair of barriers, the
 // weight-gradient partials are 8 * NV registers per thread, so many CTAs fit an SM and enough
-// loads are in flight to keep the memory system busy (the warp-per-row kernel holds 64 partials per
-// lane and runs at a quarter of the copy bandwidth).
+// loads are in flight to keep the memory system busy (a warp per row would hold 8 * H / 256 partials per
+// lane: 64 at H = 2048, which measured a quarter of the copy bandwidth).
 template <int NV, int R>
 __global__ void __launch_bounds__(kNormThreads)
 rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ h,
@@ -343,79 +343,53 @@ rmsnorm_bwd_rows_pf_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
                            float* __restrict__ dw_partial, int rows, int H) {
   ahead_wait();
   ahead_next();
-  constexpr int NV = 1;
   constexpr int kWarps = kThreads / 32;
   __shared__ float red[R][kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int nvec = H / 8;                       // <= kThreads
   const bool act = (int)threadIdx.x < nvec;
   const int col = act ? (int)threadIdx.x : 0;     // idle threads read column 0 and add nothing
-  float dw_acc[NV][8];
-  float wv[NV][8];
+  float dw_acc[8], wv[8];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dw_acc[i][j] = 0.f;
-    unpack8(reinterpret_cast<const uint4*>(w)[col], wv[i]);
-  }
+  for (int j = 0; j < 8; ++j) dw_acc[j] = 0.f;
+  unpack8(reinterpret_cast<const uint4*>(w)[col], wv);
   const float inv_h = 1.f / (float)H;
-  uint4 dnext[R][NV], hnext[R][NV];
+  uint4 dnext[R], hnext[R];
   float rnext[R];
-  const int stride = gridDim.x * R;
-  int row0 = blockIdx.x * R;
-  if (row0 < rows) {
+  auto load = [&](int row0) {                   // zeros past the end, as above
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int row = row0 + r;
+      const size_t off = (size_t)row * nvec + col;
       rnext[r] = row < rows ? rstd_in[row] : 0.f;
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const size_t off = (size_t)row * nvec + col;      // zeros past the end, as above
-        dnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(dy)[off] : make_uint4(0, 0, 0, 0);
-        hnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(h)[off] : make_uint4(0, 0, 0, 0);
-      }
+      dnext[r] = row < rows ? reinterpret_cast<const uint4*>(dy)[off] : make_uint4(0, 0, 0, 0);
+      hnext[r] = row < rows ? reinterpret_cast<const uint4*>(h)[off] : make_uint4(0, 0, 0, 0);
     }
-  }
+  };
+  const int stride = gridDim.x * R;
+  int row0 = blockIdx.x * R;
+  if (row0 < rows) load(row0);
   for (; row0 < rows; row0 += stride) {
-    uint4 draw[R][NV], hraw[R][NV];
+    uint4 draw[R], hraw[R];
     float rstd[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       rstd[r] = rnext[r];
-#pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        draw[r][i] = dnext[r][i];
-        hraw[r][i] = hnext[r][i];
-      }
+      draw[r] = dnext[r];
+      hraw[r] = hnext[r];
     }
-    const int next0 = row0 + stride;
-    if (next0 < rows) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int row = next0 + r;
-        rnext[r] = row < rows ? rstd_in[row] : 0.f;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-          const size_t off = (size_t)row * nvec + col;      // zeros past the end, as above
-          dnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(dy)[off] : make_uint4(0, 0, 0, 0);
-          hnext[r][i] = row < rows ? reinterpret_cast<const uint4*>(h)[off] : make_uint4(0, 0, 0, 0);
-        }
-      }
-    }
+    if (row0 + stride < rows) load(row0 + stride);
     float dot[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       dot[r] = 0.f;
+      float d[8], hv[8];
+      unpack8(draw[r], d);
+      unpack8(hraw[r], hv);
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        float d[8], hv[8];
-        unpack8(draw[r][i], d);
-        unpack8(hraw[r][i], hv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if (act) dot[r] += d[j] * wv[i][j] * hv[j];
-          dw_acc[i][j] += d[j] * hv[j] * rstd[r];
-        }
+      for (int j = 0; j < 8; ++j) {
+        if (act) dot[r] += d[j] * wv[j] * hv[j];
+        dw_acc[j] += d[j] * hv[j] * rstd[r];
       }
       dot[r] = warp_sum(dot[r]);
     }
@@ -433,32 +407,25 @@ rmsnorm_bwd_rows_pf_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bflo
 #pragma unroll
       for (int k = 0; k < kWarps; ++k) tot += red[r][k];
       const float c = tot * inv_h * rstd[r] * rstd[r] * rstd[r];
+      float d[8], hv[8], o[8];
+      unpack8(draw[r], d);
+      unpack8(hraw[r], hv);
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        float d[8], hv[8], o[8];
-        unpack8(draw[r][i], d);
-        unpack8(hraw[r][i], hv);
+      for (int j = 0; j < 8; ++j) o[j] = rstd[r] * d[j] * wv[j] - hv[j] * c;
+      const size_t off = (size_t)row * nvec + col;
+      if (dres) {
+        float rr[8];
+        unpack8(reinterpret_cast<const uint4*>(dres)[off], rr);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = rstd[r] * d[j] * wv[i][j] - hv[j] * c;
-        const size_t off = (size_t)row * nvec + col;
-        if (dres) {
-          float rr[8];
-          unpack8(reinterpret_cast<const uint4*>(dres)[off], rr);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += rr[j];
-        }
-        if (act) reinterpret_cast<uint4*>(dh)[off] = pack8(o);
+        for (int j = 0; j < 8; ++j) o[j] += rr[j];
       }
+      if (act) reinterpret_cast<uint4*>(dh)[off] = pack8(o);
     }
   }
   if (!act) return;
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    float4* out = reinterpret_cast<float4*>(dw_partial + (size_t)blockIdx.x * H +
-                                            (size_t)col * 8);
-    out[0] = make_float4(dw_acc[i][0], dw_acc[i][1], dw_acc[i][2], dw_acc[i][3]);
-    out[1] = make_float4(dw_acc[i][4], dw_acc[i][5], dw_acc[i][6], dw_acc[i][7]);
-  }
+  float4* out = reinterpret_cast<float4*>(dw_partial + (size_t)blockIdx.x * H + (size_t)col * 8);
+  out[0] = make_float4(dw_acc[0], dw_acc[1], dw_acc[2], dw_acc[3]);
+  out[1] = make_float4(dw_acc[4], dw_acc[5], dw_acc[6], dw_acc[7]);
 }
 
 // dw[H] (=|+=) sum_p partial[p][H]; fixed summation order (deterministic)

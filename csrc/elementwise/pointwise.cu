@@ -337,7 +337,8 @@ extern "C" int pico_scale_unless_one(void* x_bf16, int64_t n, const float* scale
     pico_host::set_error("scale_unless_one: %lld elements, need a multiple of 8", (long long)n);
     return -2;
   }
-  pico_host::launch_ahead(scale_unless_one_kernel, grid_for(n / 8, 256), 256, 0, stream, (uint4*)x_bf16, n / 8, scale_dev);
+  pico_host::launch_ahead(scale_unless_one_kernel, grid_for(n / 8, 256), 256, 0, stream, (uint4*)x_bf16, n / 8,
+                          scale_dev);
   return finish("scale_unless_one");
 }
 
@@ -352,8 +353,7 @@ extern "C" int pico_rope_inplace(void* x, int64_t row_stride, int rows, int seq,
   }
   const int64_t total = (int64_t)rows * nheads * (d / 16);
   pico_host::launch_ahead(rope_kernel, grid_for(total, 256), 256, 0, stream, (__nv_bfloat16*)x, row_stride, rows, seq,
-                                                        pos_offset, nheads, d, cos, sin,
-                                                        sign >= 0 ? 1.f : -1.f);
+                          pos_offset, nheads, d, cos, sin, sign >= 0 ? 1.f : -1.f);
   return finish("rope");
 }
 
@@ -364,7 +364,8 @@ extern "C" int pico_swiglu_fwd(const void* gu, int64_t ld_gu, void* y, int rows,
     pico_host::set_error("swiglu: width %d and stride %lld must be multiples of 8", I, (long long)ld_gu);
     return -2;
   }
-  pico_host::launch_ahead(swiglu_fwd_kernel, grid_for((int64_t)rows * (I / 8), 256), 256, 0, stream, (const __nv_bfloat16*)gu, ld_gu, (__nv_bfloat16*)y, rows, I, rows_dev);
+  pico_host::launch_ahead(swiglu_fwd_kernel, grid_for((int64_t)rows * (I / 8), 256), 256, 0, stream,
+                          (const __nv_bfloat16*)gu, ld_gu, (__nv_bfloat16*)y, rows, I, rows_dev);
   return finish("swiglu_fwd");
 }
 
@@ -375,7 +376,9 @@ extern "C" int pico_swiglu_bwd(const void* dy, const void* gu, int64_t ld_gu, vo
     pico_host::set_error("swiglu: width and strides must be multiples of 8");
     return -2;
   }
-  pico_host::launch_ahead(swiglu_bwd_kernel, grid_for((int64_t)rows * (I / 8), 256), 256, 0, stream, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, ld_gu, (__nv_bfloat16*)dgu, ld_dgu, rows, I, rows_dev);
+  pico_host::launch_ahead(swiglu_bwd_kernel, grid_for((int64_t)rows * (I / 8), 256), 256, 0, stream,
+                          (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, ld_gu, (__nv_bfloat16*)dgu, ld_dgu,
+                          rows, I, rows_dev);
   return finish("swiglu_bwd");
 }
 
@@ -388,8 +391,8 @@ extern "C" int pico_adamw(void* p_bf16, float* master, float* g, float* m, float
     pico_host::set_error("adamw: need bf16 params or fp32 master params");
     return -2;
   }
-  pico_host::launch_ahead(adamw_kernel, grid_for(n / 4 + 1, 256), 256, 0, stream, (__nv_bfloat16*)p_bf16, master, g, m, v, n, lr, beta1, beta2, eps, weight_decay, bias_corr1,
-      bias_corr2, grad_scale, zero_grad);
+  pico_host::launch_ahead(adamw_kernel, grid_for(n / 4 + 1, 256), 256, 0, stream, (__nv_bfloat16*)p_bf16, master, g, m,
+                          v, n, lr, beta1, beta2, eps, weight_decay, bias_corr1, bias_corr2, grad_scale, zero_grad);
   return finish("adamw");
 }
 
@@ -400,7 +403,8 @@ extern "C" int pico_embedding_fwd(const void* W, const int64_t* ids, void* out, 
     pico_host::set_error("embedding: hidden size %d must be a multiple of 8", H);
     return -2;
   }
-  pico_host::launch_ahead(embedding_fwd_kernel, grid_for((int64_t)rows * (H / 8), 256), 256, 0, stream, (const __nv_bfloat16*)W, ids, (__nv_bfloat16*)out, rows, H, Vlocal, vocab_start);
+  pico_host::launch_ahead(embedding_fwd_kernel, grid_for((int64_t)rows * (H / 8), 256), 256, 0, stream,
+                          (const __nv_bfloat16*)W, ids, (__nv_bfloat16*)out, rows, H, Vlocal, vocab_start);
   return finish("embedding_fwd");
 }
 
@@ -411,7 +415,8 @@ extern "C" int pico_embedding_bwd(const void* dout, const int64_t* ids, float* d
     pico_host::set_error("embedding: hidden size %d must be a multiple of 8", H);
     return -2;
   }
-  pico_host::launch_ahead(embedding_bwd_kernel, grid_for((int64_t)rows * (H / 8), 256), 256, 0, stream, (const __nv_bfloat16*)dout, ids, dW, rows, H, Vlocal, vocab_start);
+  pico_host::launch_ahead(embedding_bwd_kernel, grid_for((int64_t)rows * (H / 8), 256), 256, 0, stream,
+                          (const __nv_bfloat16*)dout, ids, dW, rows, H, Vlocal, vocab_start);
   return finish("embedding_bwd");
 }
 

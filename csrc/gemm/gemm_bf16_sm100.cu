@@ -5,8 +5,8 @@
 // One CTA per SM walks output tiles of 128 x BN. Roles:
 //   warp 0    : TMA producer  - streams 64-deep K slices of A and B into a ring of shared
 //                               memory stages (128-byte swizzle), one mbarrier per stage
-//   warp 1    : MMA issuer    - one elected thread issues tcgen05.mma (128 x BN x 16) per
-//                               K step; accumulators live in TMEM, double buffered so the
+//   warp 1    : MMA issuer    - a converged warp, one elected lane issues tcgen05.mma
+//                               (128 x BN x 16) per K step; accumulators live in TMEM, double buffered so the
 //                               epilogue of tile i overlaps the main loop of tile i+1
 //   warps 2-5 : epilogue      - tcgen05.ld the accumulator, convert, stage in swizzled
 //                               shared memory, TMA store (or TMA reduce-add for D +=)
@@ -557,7 +557,8 @@ static int launch(const void* A, const void* B, void* D, int M, int N, int K, in
   if (scatter || gather)
     kern<<<ctas, kNumThreads, Cfg::kSmemBytes, stream>>>(ta, tb, dm, comm, M, N, K, pico_status_buffer());
   else
-    pico_host::launch_ahead(kern, ctas, kNumThreads, Cfg::kSmemBytes, stream, ta, tb, dm, comm, M, N, K, pico_status_buffer());
+    pico_host::launch_ahead(kern, ctas, kNumThreads, Cfg::kSmemBytes, stream, ta, tb, dm, comm, M, N, K,
+                            pico_status_buffer());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     pico_host::set_error("gemm launch: %s", cudaGetErrorString(e));
@@ -673,8 +674,8 @@ extern "C" int pico_gemm_bf16_parts(const void* A, const void* B, void* D, float
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const int num_kb = (K + pico::BK - 1) / pico::BK;
   if (parts < 1 || parts > num_kb || N % 4 != 0 || ldd % 4 != 0 || (reinterpret_cast<uintptr_t>(D) & 7) != 0) {
-    pico_host::set_error("gemm in parts: 1 <= parts (%d) <= K blocks (%d), N (%d) and ldd (%d) multiples of 4, D 8-byte "
-                         "aligned", parts, num_kb, N, ldd);
+    pico_host::set_error("gemm in parts: 1 <= parts (%d) <= K blocks (%d), N (%d) and ldd (%d) multiples of 4, D "
+                         "8-byte aligned", parts, num_kb, N, ldd);
     return -2;
   }
   const int rc = b_mn_major
@@ -684,8 +685,8 @@ extern "C" int pico_gemm_bf16_parts(const void* A, const void* B, void* D, float
   const int64_t items = (int64_t)M * (N / 4);
   int64_t blocks = (items + 255) / 256;
   if (blocks > pico_host::num_sms() * 8) blocks = pico_host::num_sms() * 8;
-  pico_host::launch_ahead(pico::sum_parts_kernel, (int)blocks, 256, 0, stream, slabs, (__nv_bfloat16*)D, ldd, M, N, parts,
-                                                         (int64_t)((M + pico::BM - 1) / pico::BM) * pico::BM * N);
+  pico_host::launch_ahead(pico::sum_parts_kernel, (int)blocks, 256, 0, stream, slabs, (__nv_bfloat16*)D, ldd, M, N,
+                          parts, (int64_t)((M + pico::BM - 1) / pico::BM) * pico::BM * N);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     pico_host::set_error("gemm in parts: %s", cudaGetErrorString(e));
@@ -694,20 +695,23 @@ extern "C" int pico_gemm_bf16_parts(const void* A, const void* B, void* D, float
   return 0;
 }
 
-static int run_gemm(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int a_mn_major,
-                    int b_mn_major, int out_mode, int max_ctas, const PicoGemmComm* comm, float* scratch,
-                    cudaStream_t stream) {
+static int run_gemm(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
+                    int a_mn_major, int b_mn_major, int out_mode, int max_ctas, const PicoGemmComm* comm,
+                    float* scratch, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   pico::GemmPlan plan{false, 256, 0, 0, 0};
   if (comm == nullptr)
-    plan = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas, scratch != nullptr);
+    plan = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas,
+                           scratch != nullptr);
   else if (N <= 64)
     plan.bn = 64;
   else if (N <= 128 || ((N + 127) / 128) * ((M + 127) / 128) <= pico_host::num_sms())
     plan.bn = 128;   // no more 128 x 128 tiles than SMs: one wave either way
   if (plan.pair)
     return pico::gemm_pair(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, scratch, stream);
-  auto one_cta = plan.bn == 64 ? pico::dispatch_bn<64> : plan.bn == 128 ? pico::dispatch_bn<128> : pico::dispatch_bn<256>;
+  auto one_cta = plan.bn == 64    ? pico::dispatch_bn<64>
+                 : plan.bn == 128 ? pico::dispatch_bn<128>
+                                  : pico::dispatch_bn<256>;
   return one_cta(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, comm, stream);
 }
 
@@ -720,13 +724,14 @@ extern "C" int pico_gemm_bf16_ex(const void* A, const void* B, void* D, int M, i
 extern "C" int pico_gemm_bf16(const void* A, const void* B, void* D, int M, int N, int K, int lda,
                               int ldb, int ldd, int a_mn_major, int b_mn_major, int out_mode,
                               int max_ctas, float* scratch, cudaStream_t stream) {
-  return run_gemm(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, nullptr, scratch, stream);
+  return run_gemm(A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, max_ctas, nullptr, scratch,
+                  stream);
 }
 
 extern "C" int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas,
                               int has_scratch, int plan[4]) {
-  const pico::GemmPlan p = pico::plan_gemm(sms > 0 ? sms : pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode,
-                                           max_ctas, has_scratch != 0);
+  const pico::GemmPlan p = pico::plan_gemm(sms > 0 ? sms : pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major,
+                                           out_mode, max_ctas, has_scratch != 0);
   plan[0] = p.pair ? p.pairs : 0;
   plan[1] = p.bn;
   plan[2] = p.tiles;
@@ -736,6 +741,7 @@ extern "C" int pico_gemm_plan(int sms, int M, int N, int K, int a_mn_major, int 
 
 extern "C" int64_t pico_gemm_scratch(int M, int N, int K, int a_mn_major, int b_mn_major, int out_mode, int max_ctas) {
   if (out_mode != pico::OUT_F32_ACC || M <= 0 || N <= 0 || K <= 0) return 0;
-  const pico::GemmPlan p = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas, true);
+  const pico::GemmPlan p =
+      pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas, true);
   return p.pair && p.whole < p.tiles ? (int64_t)p.pairs * pico::kGemmSlab : 0;
 }

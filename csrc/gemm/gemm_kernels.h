@@ -24,7 +24,7 @@ GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn_major, int b_mn_major,
 // CTA-pair kernel; operands as pico_gemm_bf16, `plan` as plan_gemm gives it for them, slabs: its scratch, 16-byte
 // aligned (not read where nothing is cut).
 bool gemm_pair_has(int a_mn_major, int b_mn_major, int out_mode);
-int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
-              int a_mn_major, int b_mn_major, int out_mode, float* slabs, cudaStream_t stream);
+int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
+              int ldd, int a_mn_major, int b_mn_major, int out_mode, float* slabs, cudaStream_t stream);
 
 }  // namespace pico

@@ -20,10 +20,10 @@
 // Work split: output tiles are dealt to the pairs in whole rounds; where D is accumulated (weight
 // gradients) the tiles of the last, partial round are cut along K into equal shares for all pairs, so that
 // round costs its share and not a whole one (256 tiles on 74 pairs: 3.46 rounds instead of 4). A share is
-// shorter than a tile, so a pair has at most one piece that does not begin its tile. That one goes to the pair's own fp32
-// slab; the first piece of a tile is added to D like a whole tile, and add_pieces_kernel then adds the slabs to D
-// in the order of K: the same bits on each run. (Reduce-adding every piece to D needs no second kernel, but then the sums
-// depend on which pair is done first.) Measured, dW += dY^T X of 8192 tokens, uncut, cut, cut without an order:
+// shorter than a tile, so a pair has at most one piece that does not begin its tile. That one goes to the pair's own
+// fp32 slab; the first piece of a tile is added to D like a whole tile, and add_pieces_kernel then adds the slabs to D
+// in the order of K: the same bits on each run. (Reduce-adding every piece to D needs no second kernel, but then the
+// sums depend on which pair is done first.) Measured, dW += dY^T X of 8192 tokens, uncut, cut, cut without an order:
 // 6144 x 2048 165, 158, 149 us; 960 x 960 (16 tiles) 52, 29, 24 us; 2048 x 2048 (64 tiles) 67, 77, 66 us.
 //
 // Operand layouts and raggedness as in gemm_bf16_sm100.cu.
@@ -119,8 +119,8 @@ struct Schedule : Tiles {
 template <int BN, int A_MN, int B_MN, int OUT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_slabs, int M, int N,
-                 int K, int whole, int* status) {
+                 const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_slabs, int M,
+                 int N, int K, int whole, int* status) {
   using C = Cfg<BN>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* staging = smem + C::kStages * C::kStageBytes;
@@ -373,8 +373,8 @@ add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_
   const Tiles tiles(M, N, K, 256);
   Work w;
   tiles.place(whole + cut, w);
-  // the pairs whose share begins inside this tile, floor(rest * num_kb * p / pairs) in (cut * num_kb, (cut + 1) * num_kb):
-  // num_kb * (rest * p - cut * pairs) >= pairs, and rest * p < (cut + 1) * pairs
+  // the pairs whose share begins inside this tile, floor(rest * num_kb * p / pairs) in (cut * num_kb,
+  // (cut + 1) * num_kb): num_kb * (rest * p - cut * pairs) >= pairs, and rest * p < (cut + 1) * pairs
   const int first = (cut * pairs + (pairs + tiles.num_kb - 1) / tiles.num_kb + rest - 1) / rest;
   const int last = ((cut + 1) * pairs + rest - 1) / rest;      // exclusive
   const int row = blockIdx.x * 4 * kRows + (threadIdx.x >> 6), col = (threadIdx.x & 63) * 4;
@@ -455,8 +455,8 @@ static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, i
       pico_host::set_error("pair gemm: tiles cut along K need an accumulated result and scratch");
       return -2;
     }
-    rc = pico_host::make_tmap_2d(&ts, slabs, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 256, (uint64_t)plan.pairs * 256, 256 * 4, 32,
-                                 BM, Swizzle::B128);
+    rc = pico_host::make_tmap_2d(&ts, slabs, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 256, (uint64_t)plan.pairs * 256,
+                                 256 * 4, 32, BM, Swizzle::B128);
     if (rc) return rc;
   }
   const int pairs = !cut && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
@@ -466,8 +466,8 @@ static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, i
     // few tiles have many pieces each: short threads there, fewer and longer ones where the tiles alone fill the SMs
     const int rest = plan.tiles - plan.whole;
     const bool few = rest < 16;
-    pico_host::launch_ahead(few ? add_pieces_kernel<1> : add_pieces_kernel<4>, dim3(few ? 64 : 16, rest), 256, 0, stream,
-                            slabs, (float*)D, (int64_t)ldd, M, N, K, plan.whole, plan.pairs);
+    pico_host::launch_ahead(few ? add_pieces_kernel<1> : add_pieces_kernel<4>, dim3(few ? 64 : 16, rest), 256, 0,
+                            stream, slabs, (float*)D, (int64_t)ldd, M, N, K, plan.whole, plan.pairs);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -498,8 +498,8 @@ bool gemm_pair_has(int a_mn, int b_mn, int out_mode) {
          (out_mode == GEMM_OUT_F32_ACC && a_mn == 1 && b_mn == 1);
 }
 
-int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
-              int a_mn, int b_mn, int out_mode, float* slabs, cudaStream_t stream) {
+int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
+              int ldd, int a_mn, int b_mn, int out_mode, float* slabs, cudaStream_t stream) {
   return pair::dispatch<256>(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, slabs, stream);
 }
 
