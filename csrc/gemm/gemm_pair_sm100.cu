@@ -364,8 +364,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 }
 
 // Pieces of the cut tiles that do not begin their tile, added to D in the order of K. blockIdx.y is the cut tile, a
-// block takes 4 * kRows rows of it, a thread four columns of kRows rows with their loads in flight.
-template <int kRows>
+// block takes 4 * kRows rows of it, a thread four columns of kRows rows; the loads of kBatch pieces are in flight at a
+// time.
+template <int kRows, int kBatch>
 __global__ void __launch_bounds__(256)
 add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_t ldd, int M, int N, int K, int whole,
                   int pairs) {
@@ -389,18 +390,26 @@ add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
       if (m + 4 * r < M) acc[r] = *reinterpret_cast<const float4*>(dst + 4 * r * ldd);
-#pragma unroll(kRows == 1 ? 8 : 2)
-    for (int p = first; p < last; ++p, src += kGemmSlab) {
-      float4 v[kRows];
+    for (int p = first; p < last; p += kBatch, src += (int64_t)kBatch * kGemmSlab) {
+      float4 v[kBatch][kRows];
 #pragma unroll
-      for (int r = 0; r < kRows; ++r)
-        if (m + 4 * r < M) v[r] = *reinterpret_cast<const float4*>(src + 4 * r * 256);
+      for (int b = 0; b < kBatch; ++b) {
 #pragma unroll
-      for (int r = 0; r < kRows; ++r) {
-        acc[r].x += v[r].x;
-        acc[r].y += v[r].y;
-        acc[r].z += v[r].z;
-        acc[r].w += v[r].w;
+        for (int r = 0; r < kRows; ++r)
+          if (p + b < last && m + 4 * r < M)
+            v[b][r] = *reinterpret_cast<const float4*>(src + (int64_t)b * kGemmSlab + 4 * r * 256);
+      }
+#pragma unroll
+      for (int b = 0; b < kBatch; ++b) {
+        if (p + b < last) {
+#pragma unroll
+          for (int r = 0; r < kRows; ++r) {
+            acc[r].x += v[b][r].x;
+            acc[r].y += v[b][r].y;
+            acc[r].z += v[b][r].z;
+            acc[r].w += v[b][r].w;
+          }
+        }
       }
     }
 #pragma unroll
@@ -463,10 +472,11 @@ static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, i
   pico_host::launch_ahead(kern, 2 * pairs, kThreads, C::kSmemBytes, stream, ta, tb, td, ts, M, N, K, plan.whole,
                           pico_status_buffer());
   if (cut) {
-    // few tiles have many pieces each: short threads there, fewer and longer ones where the tiles alone fill the SMs
+    // few tiles have many pieces each (up to 18): short threads with many loads in flight, latency binds; else two or
+    // three, and fewer and longer threads
     const int rest = plan.tiles - plan.whole;
     const bool few = rest < 16;
-    pico_host::launch_ahead(few ? add_pieces_kernel<1> : add_pieces_kernel<4>, dim3(few ? 64 : 16, rest), 256, 0,
+    pico_host::launch_ahead(few ? add_pieces_kernel<1, 8> : add_pieces_kernel<4, 1>, dim3(few ? 64 : 16, rest), 256, 0,
                             stream, slabs, (float*)D, (int64_t)ldd, M, N, K, plan.whole, plan.pairs);
   }
   cudaError_t e = cudaGetLastError();
