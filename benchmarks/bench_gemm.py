@@ -1,5 +1,5 @@
-"""Micro-benchmark of the tcgen05 GEMM on the layer shapes of the SmolLM-1.7B and Llama-2-7B
-configs, next to ``torch.matmul`` (cuBLAS) on the same operands.
+"""Micro-benchmark of the tcgen05 GEMM on the layer shapes of the SmolLM-1.7B, Llama-2-7B, SmolLM-360M (h960)
+and long-context configs and on ragged numbers of tokens, next to ``torch.matmul`` (cuBLAS) on the same operands.
 
 CUDA-event timing after warm-up, L2 flushed between timed iterations by writing a 256 MiB
 buffer. Prints one line per shape and layout: microseconds, TFLOP/s and the fraction of the
@@ -98,7 +98,9 @@ def main():
     if args.grouped:
         return grouped(args, peak, flush)
     shapes = [(8192, 6144, 2048), (8192, 2048, 2048), (8192, 16384, 2048), (8192, 2048, 8192),
-              (8192, 49152, 2048), (4096, 12288, 4096), (4096, 22016, 4096), (4096, 4096, 11008)]
+              (8192, 49152, 2048), (4096, 12288, 4096), (4096, 22016, 4096), (4096, 4096, 11008), (4096, 4096, 4096),
+              (16384, 11264, 2048), (8192, 5120, 960), (8192, 1600, 960), (8192, 960, 960), (2042, 16384, 2048),
+              (1999, 2560, 960)]
     if args.small:
         shapes = [(4096, 4096, 4096)]
     for (M, N, K) in shapes:

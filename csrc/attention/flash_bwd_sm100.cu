@@ -29,8 +29,9 @@
 //   S   is overwritten by S(i+1) after P(i) was published (all of S(i) is in registers then)
 //   P   is overwritten once S(i+1) has landed (the in-order pipe ran dV(i) before it)
 //   dP  is overwritten by dP(i+1) behind dK(i) / dQ(i); dS lies over the dP columns of its own thread
-// Measured (causal, B200; 546, 5740 and 701 us with P and dS through shared memory and one serial chain per
-// tile): 4 x 2048 x 32 heads x 64: 346 us; 1 x 16384 x 32/8 heads x 64: 3284 us; 1 x 4096 x 32 x 128: 437 us.
+// Measured (causal, B200, one call with its pre- and post-pass after an L2 flush; 546, 5740 and 701 us with P and dS
+// through shared memory and one serial chain per tile): 4 x 2048 x 32 heads x 64: 347 us; 1 x 16384 x 32/8 heads x
+// 64: 3131 us; 1 x 4096 x 32 x 128: 441 us.
 // What binds it now is the chain of a tile through the softmax warps (exponentials, dS, their barriers).
 //
 // delta = rowsum(dO * O) comes from a small pre-pass; the dQ accumulator is scaled and converted to

@@ -27,8 +27,8 @@
 // operand of O_t += P V_j. The accumulator is rescaled lazily: only when the running maximum grew by
 // more than 2^8, which the fp32 range of the un-normalised probabilities absorbs.
 //
-// Measured (causal, B200), before and now: 4 x 2048 x 32 heads x 64: 218 and 133 us; 1 x 16384 x 32/8 heads x
-// 64: 2111 and 1446 us; 1 x 4096 x 32 x 128: 206 and 148 us. At head_dim 64 the softmax warps never wait now
+// Measured (causal, B200, one call after an L2 flush; before this form 218, 2111 and 206 us): 4 x 2048 x 32 heads x
+// 64: 146 us; 1 x 16384 x 32/8 heads x 64: 1459 us; 1 x 4096 x 32 x 128: 154 us. At head_dim 64 the softmax warps never wait now
 // (165 of 2700 cycles per pair of tiles); two threads per row, three-input maxima or a share of the
 // exponentials on the FMA pipe changed that by less than 3 % or made it slower.
 //
