@@ -39,10 +39,10 @@ void* mptr(const c10::optional<at::Tensor>& t) {
 }
 
 // D = op(A) op(B) with explicit geometry so that views (row slices, transposes expressed
-// through the *_mn_major flags, column slices through ld) need no copies.
-void gemm(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, int64_t M, int64_t N, int64_t K,
-          int64_t lda, int64_t ldb, int64_t ldd, bool a_mn_major, bool b_mn_major, int64_t out_mode,
-          int64_t max_ctas) {
+// through the *_mn_major flags, column slices through ld) need no copies. Returns the number of kernels launched.
+int64_t gemm(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, int64_t M, int64_t N, int64_t K,
+             int64_t lda, int64_t ldb, int64_t ldd, bool a_mn_major, bool b_mn_major, int64_t out_mode,
+             int64_t max_ctas) {
   TORCH_CHECK(A.is_cuda() && B.is_cuda() && D.is_cuda(), "gemm: CUDA tensors required");
   TORCH_CHECK(A.scalar_type() == at::kBFloat16 && B.scalar_type() == at::kBFloat16,
               "gemm: bf16 operands required");
@@ -55,6 +55,7 @@ void gemm(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, int64_t M, in
                        (int)ldb, (int)ldd, a_mn_major, b_mn_major, (int)out_mode, (int)max_ctas,
                        scratch.defined() ? scratch.data_ptr<float>() : nullptr, stream_of(A)),
         "gemm");
+  return scratch.defined() ? 2 : 1;     // with scratch, a second kernel adds the pieces of the cut tiles
 }
 
 // (pairs at work or 0, tile width, 256 x 256 tiles, tiles that are not cut) of such a product on `sms` SMs (0: this

@@ -332,7 +332,9 @@ def test_cut_last_round_gives_the_same_bits_on_each_run(M, N, K):
         with torch.cuda.stream(side):
             for _ in range(run):
                 noise.mul_(1.0)
+        launched = ops.launches()
         gemm.gemm_tn(a, b, out=wide[:, 4:4 + N], accumulate=True)
+        assert ops.launches() - launched == 2            # the product and the kernel that adds the pieces
         torch.cuda.current_stream().wait_stream(side)
         first = wide.clone() if first is None else first
         assert torch.equal(wide, first)
