@@ -226,6 +226,18 @@ void ce_loss_grad(const at::Tensor& logits, int64_t ldl, const at::Tensor& targe
         "ce_loss_grad");
 }
 
+void ce_whole(const at::Tensor& logits, int64_t ldl, const at::Tensor& targets, at::Tensor& loss, at::Tensor& dlogits,
+              int64_t ldd, double grad_scale, int64_t rows, int64_t V) {
+  c10::cuda::CUDAGuard guard(logits.device());
+  TORCH_CHECK(logits.scalar_type() == at::kBFloat16 && dlogits.scalar_type() == at::kBFloat16 &&
+                  targets.scalar_type() == at::kLong && loss.scalar_type() == at::kFloat, "ce_whole: dtypes");
+  TORCH_CHECK(((reinterpret_cast<uintptr_t>(logits.data_ptr()) | reinterpret_cast<uintptr_t>(dlogits.data_ptr())) &
+               15) == 0, "ce_whole: 16-byte aligned rows");
+  check(pico_ce_whole(logits.data_ptr(), ldl, (const int64_t*)targets.data_ptr(), (float*)loss.data_ptr(),
+                      dlogits.data_ptr(), ldd, (float)grad_scale, (int)rows, (int)V, stream_of(logits)),
+        "ce_whole");
+}
+
 void adamw(const c10::optional<at::Tensor>& p, const c10::optional<at::Tensor>& master, at::Tensor& g,
            at::Tensor& m, at::Tensor& v, int64_t n, double lr, double beta1, double beta2, double eps,
            double wd, double bc1, double bc2, double grad_scale, bool zero_grad) {
@@ -879,6 +891,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("swiglu_bwd", &swiglu_bwd);
   m.def("ce_stats", &ce_stats);
   m.def("ce_loss_grad", &ce_loss_grad);
+  m.def("ce_whole", &ce_whole);
+  m.def("ce_whole_max_vocab", [] { return pico_ce_whole_max_vocab(); });
   m.def("adamw", &adamw);
   m.def("embedding_fwd", &embedding_fwd);
   m.def("embedding_bwd", &embedding_bwd);

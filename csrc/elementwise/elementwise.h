@@ -50,6 +50,12 @@ int pico_ce_loss_grad(const void* logits, int64_t ldl, const int64_t* targets, c
                       float* loss, void* dlogits, int64_t ldd, float grad_scale, int rows, int V,
                       int vocab_start, cudaStream_t stream);
 
+// Both for rows that are not sharded, V <= pico_ce_whole_max_vocab(): the logits are read once. Pointers 16-byte
+// aligned; dlogits may be the logits.
+int pico_ce_whole_max_vocab(void);
+int pico_ce_whole(const void* logits, int64_t ldl, const int64_t* targets, float* loss, void* dlogits, int64_t ldd,
+                  float grad_scale, int rows, int V, cudaStream_t stream);
+
 // Vocabulary-parallel form without a collective call: every rank writes the triples of its shard
 // into block my_rank of the [world][rows][3] fp32 table of all ranks (`dst`, symmetric memory) and
 // raises flag [slot][my_rank] = epoch; pico_ce_loss_grad_gathered waits (bounded) for all world

@@ -39,11 +39,16 @@ def install_peer_exchange(group, exchange) -> None:
 
 
 def _stats_loss_grad(l2, t, loss, dlogits, scale, vocab_start, group):
-    """The two kernel passes of the fused loss: statistics, then loss + gradient over the logits."""
+    """Loss and gradient (over the logits): one pass where a rank holds whole rows that fit shared memory, else
+    statistics, then loss and gradient."""
     rows, V = l2.shape
     ex = _PEER_EXCHANGE.get(group) if group is not None else None
     if ex is not None and ex.fits(rows):
         ex.stats_loss_grad(l2, t, loss, dlogits, scale, vocab_start)
+        return
+    if vocab_start == 0 and V <= ext().ce_whole_max_vocab() and (group is None or dist.get_world_size(group) == 1):
+        ext().ce_whole(l2, l2.stride(0), t, loss, dlogits, dlogits.stride(0), scale, rows, V)
+        count_launch()
         return
     stats = torch.empty((rows, 3), device=l2.device, dtype=torch.float32)
     ext().ce_stats(l2, l2.stride(0), t, stats, rows, V, vocab_start)

@@ -211,3 +211,31 @@ def test_rmsnorm_backward_keeps_infinities_where_they_are(rows, H):
     others = torch.arange(H, device="cuda") != 5
     assert dw[5].item() == float("inf") and torch.equal(dw[others], clean[1][others])
     assert torch.equal(dx[:-1], clean[0][:-1]) and not dx[-1].isfinite().any()
+
+
+@pytest.mark.parametrize("rows,V", [(3, 8), (5, 24), (700, 4104), (301, 49152), (2, 57344), (3, 57352)])
+def test_cross_entropy_rows_in_one_pass(rows, V):
+    """Rows shorter than the copies they arrive in, more rows than CTAs, the longest row of the one-pass kernel and the
+    first of the two-pass one; targets at both ends and outside, -inf logits. fp32 sums of exact bf16 inputs: 1e-5;
+    gradients are rounded to bf16 once: 2^-8 of the value, and 1e-5 of the largest for the fp32 part of small ones."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import cross_entropy as ce
+    torch.manual_seed(9)
+    logits = (4 * torch.randn(rows, V, device="cuda")).to(torch.bfloat16)
+    logits[0, 1::2] = -float("inf")
+    t = torch.randint(0, V, (rows,), device="cuda")
+    t[0], t[-1] = 0, V - 1
+    t[1] = -100                       # no target in this shard: log-sum-exp alone
+    ref = logits.double()
+    lse = torch.logsumexp(ref, -1)
+    inside = (t >= 0) & (t < V)
+    hit = torch.zeros_like(ref)
+    hit[inside, t[inside]] = 1
+    want = lse - torch.where(inside, ref.gather(1, t.clamp(0, V - 1)[:, None])[:, 0], torch.zeros_like(lse))
+    dwant = ((ref - lse[:, None]).exp() - hit) / rows
+    loss = torch.empty(rows, device="cuda")
+    for d in (torch.empty_like(logits), logits):          # beside the logits, then over them
+        ce._stats_loss_grad(logits, t, loss, d, 1.0 / rows, 0, None)
+        ops.check_status()
+        assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
+        assert ((d.double() - dwant).abs() <= dwant.abs() * 2 ** -8 + 1e-5 / rows).all()
