@@ -447,6 +447,12 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   return r;
 }
 
+// p[0..3] += a, b, c, d (global memory, 16-byte aligned), each sum atomic
+__device__ __forceinline__ void red_add_f32x4(float* p, float a, float b, float c, float d) {
+  asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
+               : "memory");
+}
+
 // two fp32 operations per instruction
 __device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
   uint64_t r;

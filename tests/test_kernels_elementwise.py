@@ -239,3 +239,21 @@ def test_cross_entropy_rows_in_one_pass(rows, V):
         ops.check_status()
         assert torch.allclose(loss.double(), want, rtol=1e-5, atol=1e-5)
         assert ((d.double() - dwant).abs() <= dwant.abs() * 2 ** -8 + 1e-5 / rows).all()
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("rows,H", [(1, 8), (777, 576)])
+def test_embedding_gradient_of_repeated_ids(rows, H, offset):
+    """Few ids, many rows; a gradient buffer at 16-byte alignment and one off it. fp32 sums of at most 777 bf16 values:
+    777 * 2^-24 of the sum of their magnitudes."""
+    from picotron_b200 import ops
+    torch.manual_seed(10)
+    V = 7
+    dout = torch.randn(rows, H, device="cuda").to(torch.bfloat16)
+    ids = torch.randint(0, V + 2, (rows,), device="cuda")         # two of them outside the shard
+    dw = torch.zeros(V * H + offset, device="cuda")[offset:].view(V, H)
+    ops.ext().embedding_bwd(dout, ids, dw, rows, H, V, 0)
+    keep = ids < V
+    want = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids[keep], dout[keep].double())
+    mag = torch.zeros(V, H, device="cuda", dtype=torch.float64).index_add_(0, ids[keep], dout[keep].double().abs())
+    assert ((dw.double() - want).abs() <= mag * rows * 2 ** -24).all()
