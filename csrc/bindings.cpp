@@ -124,6 +124,58 @@ std::tuple<at::Tensor, at::Tensor, int64_t> linear_fwd(const at::Tensor& x, cons
   return {y, x2, launches};
 }
 
+// Gated MLP products (gemm.h): w is [2 * I, K] with the gate rows first. (gate | up or an empty tensor, activation, the
+// number of kernels launched); how: the activation in the product's epilogue (1), by a pass of its own (0), or whichever
+// is faster (-1).
+std::tuple<at::Tensor, at::Tensor, int64_t> gemm_swiglu(const at::Tensor& x, const at::Tensor& w, bool keep,
+                                                        int64_t how) {
+  TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                  x.dim() == 2 && w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1) &&
+                  x.size(1) % 8 == 0 && w.size(0) % 16 == 0,
+              "gemm_swiglu: bf16 rows and weights with unit inner stride, widths in whole 16-byte units");
+  const int64_t M = x.size(0), I = w.size(0) / 2, K = x.size(1);
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor act = at::empty({M, I}, x.options());
+  if (how < 0) how = pico_gemm_swiglu_pays((int)M, (int)I, (int)K, keep, 0);
+  if (!how) {
+    auto [gate_up, launches] = gemm_new(x, w, false);
+    check(pico_swiglu_fwd(gate_up.data_ptr(), 2 * I, act.data_ptr(), (int)M, (int)I, nullptr, stream_of(x)),
+          "swiglu_fwd");
+    return {gate_up, act, launches + 1};
+  }
+  at::Tensor gate_up = at::empty({keep ? M : 0, 2 * I}, x.options());
+  check(pico_gemm_swiglu(x.data_ptr(), w.data_ptr(), keep ? gate_up.data_ptr() : nullptr, act.data_ptr(), (int)M,
+                         (int)I, (int)K, (int)x.stride(0), (int)w.stride(0), stream_of(x)),
+        "gemm_swiglu");
+  return {gate_up, act, 1};
+}
+
+// Gradient of gate | up from that of the rows y = act w^T, w [K, I], and the number of kernels launched; how as above.
+std::tuple<at::Tensor, int64_t> gemm_swiglu_bwd(const at::Tensor& dy, const at::Tensor& w, const at::Tensor& gate_up,
+                                                int64_t how) {
+  TORCH_CHECK(dy.is_cuda() && w.is_cuda() && gate_up.is_cuda() && dy.scalar_type() == at::kBFloat16 &&
+                  w.scalar_type() == at::kBFloat16 && gate_up.scalar_type() == at::kBFloat16 && dy.dim() == 2 &&
+                  w.dim() == 2 && dy.stride(1) == 1 && w.stride(1) == 1 && dy.size(1) == w.size(0) &&
+                  dy.size(1) % 8 == 0 && w.size(1) % 8 == 0 && gate_up.is_contiguous() && gate_up.dim() == 2 &&
+                  gate_up.size(0) == dy.size(0) && gate_up.size(1) == 2 * w.size(1),
+              "gemm_swiglu_bwd: bf16 matrices with unit inner stride, gate | up [rows, 2 * I] contiguous");
+  const int64_t M = dy.size(0), I = w.size(1), K = dy.size(1);
+  c10::cuda::CUDAGuard guard(dy.device());
+  at::Tensor out = at::empty_like(gate_up);
+  if (how < 0) how = pico_gemm_swiglu_pays((int)M, (int)I, (int)K, 1, 1);
+  if (!how) {
+    auto [d_act, launches] = gemm_new(dy, w, true);
+    check(pico_swiglu_bwd(d_act.data_ptr(), gate_up.data_ptr(), 2 * I, out.data_ptr(), 2 * I, (int)M, (int)I, nullptr,
+                          stream_of(dy)),
+          "swiglu_bwd");
+    return {out, launches + 1};
+  }
+  check(pico_gemm_swiglu_bwd(dy.data_ptr(), w.data_ptr(), gate_up.data_ptr(), out.data_ptr(), (int)M, (int)I, (int)K,
+                             (int)dy.stride(0), (int)w.stride(0), stream_of(dy)),
+        "gemm_swiglu_bwd");
+  return {out, 1};
+}
+
 // (norm(x + residual), x + residual or x, 1 / rms) of [rows, H] rows
 std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_new(const at::Tensor& x,
                                                            const c10::optional<at::Tensor>& residual,
@@ -880,6 +932,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_plan", &gemm_plan);
   m.def("gemm_new", &gemm_new);
   m.def("linear_fwd", &linear_fwd);
+  m.def("gemm_swiglu", &gemm_swiglu, py::arg("x"), py::arg("w"), py::arg("keep"), py::arg("how") = -1);
+  m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd, py::arg("dy"), py::arg("w"), py::arg("gate_up"), py::arg("how") = -1);
+  m.def("gemm_swiglu_pays", [](int64_t M, int64_t I, int64_t K, bool keep, bool backward) {
+    return pico_gemm_swiglu_pays((int)M, (int)I, (int)K, keep, backward) != 0;
+  });
   m.def("rmsnorm_new", &rmsnorm_new);
   m.def("attention_fwd_new", &attention_fwd_new);
   m.def("attention_bwd_new", &attention_bwd_new);

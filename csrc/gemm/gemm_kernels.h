@@ -4,7 +4,13 @@
 
 namespace pico {
 
-enum GemmOutMode : int { GEMM_OUT_BF16 = 0, GEMM_OUT_F32 = 1, GEMM_OUT_F32_ACC = 2 };
+enum GemmOutMode : int {
+  GEMM_OUT_BF16 = 0,
+  GEMM_OUT_F32 = 1,
+  GEMM_OUT_F32_ACC = 2,
+  GEMM_OUT_SWIGLU = 3,        // pico_gemm_swiglu and its backward, pair kernel only
+  GEMM_OUT_SWIGLU_BWD = 4,
+};
 
 constexpr int kGemmPairUnsupported = -10;
 

@@ -16,6 +16,22 @@
 //   warp 1    : MMA issuer    - first CTA only; its commits release the stage in both CTAs
 //   warps 2-5 : epilogue      - this CTA's 128 rows: tcgen05.ld, convert, swizzled staging, TMA store
 //                               (or TMA reduce-add for D +=); accumulators are double buffered
+// SwiGLU tiles have eight epilogue warps, 2-9, two for each quarter of the accumulator's lanes, and
+//   warps 10, 11: movers      - bring what the epilogue reads into the staging buffers ahead of it (it works in place)
+//                               and send its results away
+//
+// SwiGLU epilogues, for the gated MLP y = (silu(x Wg^T) * (x Wu^T)) Wd^T:
+//   forward : a tile has 128 gate columns and the same 128 up columns (the first CTA loads the rows of Wg, the second
+//             those of Wu); gate | up and the activation leave from the same registers
+//   backward: the gradient of the activation, dy Wd, meets gate and up in the epilogue and leaves as their gradients;
+//             it is never stored
+// What a pass of its own over gate | up took (402 MB forward, 671 MB backward for 8192 rows of 2 x 8192) then runs under
+// the main loop, 16 thousand cycles per tile at K = 2048. Values are rounded to bf16 before the activation, as that pass
+// reads them.
+// Product and pass / fused, us: 8192 rows, 2048 -> 8192: forward 420 / 363, backward 306 / 226; 16384, 2048 -> 5632:
+// 566 / 496, 414 / 338; 8192, 960 -> 2560: 77 / 65, 71 / 55. The movers' four buffers cost a stage of operands; six
+// buffers and four stages measured 393 and 284 us in the first line, and with four epilogue warps the short ones 1 us
+// more.
 //
 // Work split: output tiles are dealt to the pairs in whole rounds; where D is accumulated (weight
 // gradients) the tiles of the last, partial round are cut along K into equal shares for all pairs, so that
@@ -41,19 +57,22 @@ namespace pair {
 constexpr int BM = 128;                   // rows of one CTA; a pair works on 2 * BM
 constexpr int BK = 64;
 constexpr int UMMA_K = 16;
-constexpr int kEpilogueThreads = 128;
-constexpr int kThreads = 64 + kEpilogueThreads;
 constexpr int kStagingBytes = 128 * 128;
-constexpr int kNumStaging = 2;
 
-template <int BN>
+template <int BN, int OUT>
 struct Cfg {
+  static constexpr bool kGate = OUT == GEMM_OUT_SWIGLU, kGateBwd = OUT == GEMM_OUT_SWIGLU_BWD;
+  static constexpr bool kMovers = kGate || kGateBwd;
+  static constexpr int kEpilogueThreads = kMovers ? 256 : 128;
+  static constexpr int kFirstMover = 2 + kEpilogueThreads / 32;
+  static constexpr int kThreads = 64 + kEpilogueThreads + (kMovers ? 64 : 0);
   static constexpr int kABytes = BM * BK * 2;
   static constexpr int kBBytes = (BN / 2) * BK * 2;
   static constexpr int kStageBytes = kABytes + kBBytes;
-  static constexpr int kStages = 6;
+  static constexpr int kStages = kMovers ? 5 : 6;
+  static constexpr int kNumStaging = kMovers ? 4 : 2;
   static constexpr int kTiles = kStages * kStageBytes + kNumStaging * kStagingBytes;
-  static constexpr int kSmemBytes = kTiles + (2 * kStages + 4) * 8 + 16;
+  static constexpr int kSmemBytes = kTiles + (2 * kStages + 4 + 3 * kNumStaging) * 8 + 16;
   static constexpr int kTmemCols = 2 * BN;
 };
 
@@ -116,19 +135,52 @@ struct Schedule : Tiles {
   }
 };
 
+// What an epilogue reads and writes.
+struct OutMaps {
+  CUtensorMap d;                // D; SwiGLU forward: the activation
+  CUtensorMap slabs;            // of the cut tiles
+  CUtensorMap gate, up;         // SwiGLU: written forward, read backward
+  CUtensorMap d_gate, d_up;     // their gradients
+};
+
+// The buffers of the staging ring in their order of use, and the parity of the rounds it has made.
+template <int kCount>
+struct Ring {
+  int b = 0;
+  uint32_t phase = 0;
+  __device__ __forceinline__ void next() {
+    if (++b == kCount) {
+      b = 0;
+      phase ^= 1;
+    }
+  }
+};
+
+__device__ __forceinline__ float bf16_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ float swiglu(float g, float u) { return g / (1.f + __expf(-g)) * u; }
+// gradients of gate (returned) and up
+__device__ __forceinline__ float swiglu_grad(float g, float u, float d, float& du) {
+  const float sg = 1.f / (1.f + __expf(-g));
+  du = d * (g * sg);
+  return d * u * sg * (1.f + g * (1.f - sg));
+}
+
 template <int BN, int A_MN, int B_MN, int OUT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, OUT>::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ CUtensorMap tmap_d, const __grid_constant__ CUtensorMap tmap_slabs, int M,
-                 int N, int K, int whole, int* status) {
-  using C = Cfg<BN>;
+                 const __grid_constant__ OutMaps out, int M, int N, int K, int whole, int keep_gate, int* status) {
+  using C = Cfg<BN, OUT>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* staging = smem + C::kStages * C::kStageBytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kTiles);
   uint64_t* empty_bar = full_bar + C::kStages;
   uint64_t* tmem_full = empty_bar + C::kStages;
   uint64_t* tmem_empty = tmem_full + 2;
-  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(tmem_empty + 2);
+  uint64_t* in_full = tmem_empty + 2;             // movers only, per staging buffer: the epilogue may work on it,
+  uint64_t* out_full = in_full + C::kNumStaging;  // is done,
+  uint64_t* out_sent = out_full + C::kNumStaging; // and the result has been read from it
+  uint32_t* tmem_ptr_smem = reinterpret_cast<uint32_t*>(out_sent + C::kNumStaging);
   volatile int* abort_word = reinterpret_cast<volatile int*>(tmem_ptr_smem + 1);
   if ((smem_u32(smem) & 1023u) != 0) {   // swizzled tiles need 1024-byte alignment; the same in both CTAs
     if (threadIdx.x == 0) report_error(status, PICO_ERR_BOUNDS, 998, (int)(smem_u32(smem) & 1023u));
@@ -147,13 +199,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tmem_full[a], 1);
-      mbar_init(&tmem_empty[a], 2);               // one arrival from each CTA's epilogue
+      mbar_init(&tmem_empty[a], C::kMovers ? 16 : 2);  // from each CTA's epilogue: one arrival, or one of each warp
+    }
+    for (int b = 0; b < C::kNumStaging; ++b) {
+      mbar_init(&in_full[b], 1);
+      mbar_init(&out_full[b], C::kEpilogueThreads);
+      mbar_init(&out_sent[b], 1);
     }
     *abort_word = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_a);
     tma_prefetch_desc(&tmap_b);
-    tma_prefetch_desc(&tmap_d);
+    tma_prefetch_desc(C::kGateBwd ? &out.gate : &out.d);
   }
   if (warp == 1) {
     tmem_alloc_pair(tmem_ptr_smem, C::kTmemCols);
@@ -177,7 +234,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       bool ok = true;
       while (ok && sched.get(w)) {
         const int m0 = w.m * 2 * BM + (int)rank * BM;
-        const int n0 = w.n * BN + (int)rank * (BN / 2);
+        // SwiGLU forward: gate columns in the first CTA, the up columns of the same numbers in the second
+        const int n0 = C::kGate ? w.n * (BN / 2) + (int)rank * (N / 2) : w.n * BN + (int)rank * (BN / 2);
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
           if (!mbar_wait(&empty_bar[s], phase ^ 1, abort_word, status, 100 + s)) {
             ok = false;
@@ -264,8 +322,169 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         }
       }
     }
+  } else if (warp >= C::kFirstMover) {
+    // ------------------------------------------------------------------ loads (first) and stores (second) of staging
+    if (lane == 0) {
+      Ring<C::kNumStaging> r;
+      bool ok = true;
+      // one buffer: fetched from `src` (NULL: nothing to fetch), sent to the same place of `dst`
+      auto move = [&](const CUtensorMap* src, const CUtensorMap* dst, int x, int y) {
+        uint8_t* sbuf = staging + r.b * kStagingBytes;
+        if (warp == C::kFirstMover) {
+          ok = ok && mbar_wait(&out_sent[r.b], r.phase ^ 1, abort_word, status, 500 + r.b);
+          if (!ok) return;
+          if (src == nullptr) {
+            mbar_arrive(&in_full[r.b]);
+          } else {
+            mbar_arrive_expect_tx(&in_full[r.b], kStagingBytes);
+            tma_load_2d(sbuf, src, &in_full[r.b], x, y);
+          }
+        } else {
+          ok = ok && mbar_wait(&out_full[r.b], r.phase, abort_word, status, 550 + r.b);
+          if (!ok) return;
+          tma_store_2d(dst, sbuf, x, y);
+          tma_store_commit();
+          tma_store_wait_read<0>();
+          mbar_arrive(&out_sent[r.b]);
+        }
+        r.next();
+      };
+      while (ok && sched.get(w)) {
+        const int m0 = w.m * 2 * BM + (int)rank * BM;
+        if (m0 >= M) continue;
+        if (C::kGate) {
+          const int n0 = w.n * (BN / 2);
+          for (int c = 0; ok && c < BN / 128 && n0 + c * 64 < N / 2; ++c) {
+            if (keep_gate) {
+              move(nullptr, &out.gate, n0 + c * 64, m0);
+              move(nullptr, &out.up, n0 + c * 64, m0);
+            }
+            move(nullptr, &out.d, n0 + c * 64, m0);
+          }
+        } else {
+          const int n0 = w.n * BN;
+          for (int c = 0; ok && c < BN / 64 && n0 + c * 64 < N; ++c) {
+            move(&out.gate, &out.d_gate, n0 + c * 64, m0);
+            move(&out.up, &out.d_up, n0 + c * 64, m0);
+          }
+        }
+      }
+      if (warp != C::kFirstMover) tma_store_wait<0>();
+    }
+  } else if (C::kMovers) {
+    // ------------------------------------------------------------------ epilogue in the movers' buffers
+    const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
+    const int h = (warp - 2) >> 2;                // and the 32 of a chunk's 64 columns it works on
+    const int row = quarter * 32 + lane;          // row of this CTA's half tile owned by this thread
+    Ring<C::kNumStaging> r;
+    int acc = 0;
+    uint32_t acc_phase = 0;
+    bool ok = true;
+    // this thread's row of the buffer whose turn it is, once it may be worked on
+    auto take = [&]() {
+      ok = ok && mbar_wait_warp(&in_full[r.b], r.phase, abort_word, status, 600 + r.b);
+      return staging + r.b * kStagingBytes + row * 128;
+    };
+    while (ok && sched.get(w)) {
+      const int m0 = w.m * 2 * BM + (int)rank * BM;
+      if (!mbar_wait_warp(&tmem_full[acc], acc_phase, abort_word, status, 400 + acc)) break;
+      tc_fence_after();
+      const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
+      if (m0 >= M) {
+        // nothing of this CTA's half lies in D
+      } else if (C::kGate) {
+        const int n0 = w.n * (BN / 2);
+#pragma unroll 1
+        for (int c = 0; c < BN / 128 && n0 + c * 64 < N / 2; ++c) {
+          int bufs[3] = {0, 0, 0};
+          uint8_t* rows[3] = {staging, staging, staging};
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            if (i < 2 && !keep_gate) continue;
+            rows[i] = take();
+            bufs[i] = r.b;
+            r.next();
+          }
+          if (!ok) break;
+          uint32_t g[32], u[32];
+          tmem_ld_32x32b_x32(t_row + c * 64 + h * 32, g);
+          tmem_ld_32x32b_x32(t_row + BN / 2 + c * 64 + h * 32, u);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            uint32_t gw[4], uw[4], aw[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int e = 8 * j + 2 * i;
+              gw[i] = pack_bf16x2(__uint_as_float(g[e]), __uint_as_float(g[e + 1]));
+              uw[i] = pack_bf16x2(__uint_as_float(u[e]), __uint_as_float(u[e + 1]));
+              aw[i] = pack_bf16x2(swiglu(bf16_lo(gw[i]), bf16_lo(uw[i])), swiglu(bf16_hi(gw[i]), bf16_hi(uw[i])));
+            }
+            const int at = ((h * 4 + j) ^ (row & 7)) << 4;
+            if (keep_gate) {
+              *reinterpret_cast<uint4*>(rows[0] + at) = make_uint4(gw[0], gw[1], gw[2], gw[3]);
+              *reinterpret_cast<uint4*>(rows[1] + at) = make_uint4(uw[0], uw[1], uw[2], uw[3]);
+            }
+            *reinterpret_cast<uint4*>(rows[2] + at) = make_uint4(aw[0], aw[1], aw[2], aw[3]);
+          }
+          fence_proxy_async_smem();
+          if (keep_gate) {
+            mbar_arrive(&out_full[bufs[0]]);
+            mbar_arrive(&out_full[bufs[1]]);
+          }
+          mbar_arrive(&out_full[bufs[2]]);
+        }
+      } else {
+        const int n0 = w.n * BN;
+#pragma unroll 1
+        for (int c = 0; c < BN / 64 && n0 + c * 64 < N; ++c) {
+          uint32_t v[32];
+          tmem_ld_32x32b_x32(t_row + c * 64 + h * 32, v);
+          uint8_t* grow = take();
+          const int gb = r.b;
+          r.next();
+          uint8_t* urow = take();
+          const int ub = r.b;
+          r.next();
+          tmem_ld_wait();
+          if (!ok) break;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int at = ((h * 4 + j) ^ (row & 7)) << 4;
+            uint4* gp = reinterpret_cast<uint4*>(grow + at);
+            uint4* up = reinterpret_cast<uint4*>(urow + at);
+            const uint4 gq = *gp, uq = *up;
+            const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w}, uw[4] = {uq.x, uq.y, uq.z, uq.w};
+            uint32_t dg[4], du[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t* d = &v[8 * j + 2 * i];
+              float u0, u1;
+              const float g0 = swiglu_grad(bf16_lo(gw[i]), bf16_lo(uw[i]), __uint_as_float(d[0]), u0);
+              const float g1 = swiglu_grad(bf16_hi(gw[i]), bf16_hi(uw[i]), __uint_as_float(d[1]), u1);
+              dg[i] = pack_bf16x2(g0, g1);
+              du[i] = pack_bf16x2(u0, u1);
+            }
+            *gp = make_uint4(dg[0], dg[1], dg[2], dg[3]);
+            *up = make_uint4(du[0], du[1], du[2], du[3]);
+          }
+          fence_proxy_async_smem();
+          mbar_arrive(&out_full[gb]);
+          mbar_arrive(&out_full[ub]);
+        }
+      }
+      // accumulator drained by this warp: hand it back to the issuing CTA's MMA warp
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_map(&tmem_empty[acc], 0));
+      if (++acc == 2) {
+        acc = 0;
+        acc_phase ^= 1;
+      }
+    }
   } else {
     // ------------------------------------------------------------------ epilogue
+    constexpr int kNumStaging = C::kNumStaging, kEpilogueThreads = C::kEpilogueThreads;
     const int et = threadIdx.x - 64;             // 0..127
     const int quarter = warp & 3;                 // TMEM lane quarter this warp may access
     const int row = quarter * 32 + lane;          // row of this CTA's half tile owned by this thread
@@ -329,11 +548,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         named_barrier_sync(1, kEpilogueThreads);
         if (et == 0) {
           if (OUT == GEMM_OUT_F32_ACC && w.kb0 != 0)       // not the first piece of its tile: this pair's slab
-            tma_store_2d(&tmap_slabs, sbuf, c * kColsPerChunk, (2 * pair_id + (int)rank) * BM);
+            tma_store_2d(&out.slabs, sbuf, c * kColsPerChunk, (2 * pair_id + (int)rank) * BM);
           else if (OUT == GEMM_OUT_F32_ACC)
-            tma_reduce_add_2d(&tmap_d, sbuf, n0 + c * kColsPerChunk, m0);
+            tma_reduce_add_2d(&out.d, sbuf, n0 + c * kColsPerChunk, m0);
           else
-            tma_store_2d(&tmap_d, sbuf, n0 + c * kColsPerChunk, m0);
+            tma_store_2d(&out.d, sbuf, n0 + c * kColsPerChunk, m0);
           tma_store_commit();
         }
         buf ^= 1;
@@ -426,24 +645,19 @@ add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_
   }
 }
 
+// Maps of the operands, the kernel's attributes and its launch.
 template <int BN, int A_MN, int B_MN, int OUT>
-static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
-                  int ldd, float* slabs, cudaStream_t stream) {
-  using C = Cfg<BN>;
+static int start(const GemmPlan& plan, const void* A, const void* B, const OutMaps& out, int M, int N, int K, int lda,
+                 int ldb, int keep_gate, cudaStream_t stream) {
+  using C = Cfg<BN, OUT>;
   using pico_host::Swizzle;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  CUtensorMap ta, tb, td;
+  CUtensorMap ta, tb;
   int rc = A_MN == 0 ? pico_host::make_tmap_2d(&ta, A, bf, 2, K, M, (uint64_t)lda * 2, 64, BM, Swizzle::B128)
                      : pico_host::make_tmap_2d(&ta, A, bf, 2, M, K, (uint64_t)lda * 2, 64, 64, Swizzle::B128);
   if (rc) return rc;
   rc = B_MN == 0 ? pico_host::make_tmap_2d(&tb, B, bf, 2, K, N, (uint64_t)ldb * 2, 64, BN / 2, Swizzle::B128)
                  : pico_host::make_tmap_2d(&tb, B, bf, 2, N, K, (uint64_t)ldb * 2, 64, 64, Swizzle::B128);
-  if (rc) return rc;
-  if (OUT == GEMM_OUT_BF16)
-    rc = pico_host::make_tmap_2d(&td, D, bf, 2, N, M, (uint64_t)ldd * 2, 64, BM, Swizzle::B128);
-  else
-    rc = pico_host::make_tmap_2d(&td, D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, N, M, (uint64_t)ldd * 4, 32, BM,
-                                 Swizzle::B128);
   if (rc) return rc;
   auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT>;
   static int attr_dev = -1;  // per template instantiation
@@ -457,20 +671,44 @@ static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, i
     }
     attr_dev = dev;
   }
-  CUtensorMap ts = td;
+  const int pairs = plan.whole == plan.tiles && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
+  pico_host::launch_ahead(kern, 2 * pairs, C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K, plan.whole,
+                          keep_gate, pico_status_buffer());
+  return 0;
+}
+
+static int launched() {
+  cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) {
+    pico_host::set_error("gemm launch: %s", cudaGetErrorString(e));
+    return (int)e;
+  }
+  return 0;
+}
+
+template <int BN, int A_MN, int B_MN, int OUT>
+static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
+                  int ldd, float* slabs, cudaStream_t stream) {
+  using pico_host::Swizzle;
+  OutMaps out = {};
+  int rc = OUT == GEMM_OUT_BF16
+               ? pico_host::make_tmap_2d(&out.d, D, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, M, (uint64_t)ldd * 2, 64,
+                                         BM, Swizzle::B128)
+               : pico_host::make_tmap_2d(&out.d, D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, N, M, (uint64_t)ldd * 4, 32,
+                                         BM, Swizzle::B128);
+  if (rc) return rc;
   const bool cut = plan.whole < plan.tiles;
   if (cut) {
     if (OUT != GEMM_OUT_F32_ACC || slabs == nullptr) {
       pico_host::set_error("pair gemm: tiles cut along K need an accumulated result and scratch");
       return -2;
     }
-    rc = pico_host::make_tmap_2d(&ts, slabs, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 256, (uint64_t)plan.pairs * 256,
-                                 256 * 4, 32, BM, Swizzle::B128);
+    rc = pico_host::make_tmap_2d(&out.slabs, slabs, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, 256,
+                                 (uint64_t)plan.pairs * 256, 256 * 4, 32, BM, Swizzle::B128);
     if (rc) return rc;
   }
-  const int pairs = !cut && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
-  pico_host::launch_ahead(kern, 2 * pairs, kThreads, C::kSmemBytes, stream, ta, tb, td, ts, M, N, K, plan.whole,
-                          pico_status_buffer());
+  rc = start<BN, A_MN, B_MN, OUT>(plan, A, B, out, M, N, K, lda, ldb, 0, stream);
+  if (rc) return rc;
   if (cut) {
     // few tiles have many pieces each (up to 18): short threads with many loads in flight, latency binds; else two or
     // three, and fewer and longer threads
@@ -479,12 +717,7 @@ static int launch(const GemmPlan& plan, const void* A, const void* B, void* D, i
     pico_host::launch_ahead(few ? add_pieces_kernel<1, 8> : add_pieces_kernel<4, 1>, dim3(few ? 64 : 16, rest), 256, 0,
                             stream, slabs, (float*)D, (int64_t)ldd, M, N, K, plan.whole, plan.pairs);
   }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) {
-    pico_host::set_error("gemm launch: %s", cudaGetErrorString(e));
-    return (int)e;
-  }
-  return 0;
+  return launched();
 }
 
 template <int BN>
@@ -513,4 +746,73 @@ int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M
   return pair::dispatch<256>(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, slabs, stream);
 }
 
+// All tiles of an [M, N] product whole.
+static int whole_plan(int M, int N, GemmPlan& plan) {
+  const int64_t tiles = (int64_t)((M + 255) / 256) * ((N + 255) / 256);
+  const int sms = pico_host::num_sms();
+  if (tiles > INT32_MAX || sms < 2) {
+    pico_host::set_error("swiglu gemm: too many tiles, or fewer than two SMs");
+    return -2;
+  }
+  plan = GemmPlan{true, 256, sms / 2, (int)tiles, (int)tiles};
+  return 0;
+}
+
+// The two halves of a [rows, 2 * I] buffer as matrices of their own, so that a tile past I is clipped in each.
+static int half_maps(CUtensorMap* gate, CUtensorMap* up, const void* gu, int rows, int I) {
+  const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const uint64_t pitch = (uint64_t)I * 4;
+  const int rc = pico_host::make_tmap_2d(gate, gu, bf, 2, I, rows, pitch, 64, pair::BM, pico_host::Swizzle::B128);
+  return rc ? rc : pico_host::make_tmap_2d(up, (const char*)gu + (int64_t)I * 2, bf, 2, I, rows, pitch, 64, pair::BM,
+                                           pico_host::Swizzle::B128);
+}
+
 }  // namespace pico
+
+// The fused form ends on an epilogue that nothing overlaps, 3 to 5 us longer than that of the plain product; the pass it
+// saves takes its launch and its bytes. So it pays from some number of activations on, where the plain product runs on
+// pairs too (elsewhere its narrower tiles waste less). Measured, product and pass / fused, us:
+//   forward           512 x 960 x 2560 12.3 / 13.1, 256 x 2048 x 8192 18.9 / 19.2, 4096 x 576 x 1536 21.4 / 21.1
+//   .. without gate|up 512 x 576 x 1536 8.3 / 8.6, 512 x 960 x 2560 12.3 / 10.9, 256 x 2048 x 8192 18.9 / 16.9
+//   backward          1024 x 960 x 2560 13.8 / 14.3, 4096 x 576 x 1536 20.0 / 18.7
+// and off pairs, 300 x 4096 x 11008: 77 / 89 forward, 47 / 58 backward.
+extern "C" int pico_gemm_swiglu_pays(int M, int I, int K, int keep_gate, int backward) {
+  if (M <= 0 || I <= 0 || K <= 0 || I > INT32_MAX / 2) return 0;
+  const pico::GemmPlan plan = pico::plan_gemm(pico_host::num_sms(), M, backward ? I : 2 * I, K, 0, backward,
+                                              pico::GEMM_OUT_BF16, 0, false);
+  return plan.pair && (int64_t)M * I >= (backward ? 4000000 : keep_gate ? 2500000 : 1250000);
+}
+
+extern "C" int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, void* act, int M, int I, int K, int ldx,
+                                int ldw, cudaStream_t stream) {
+  if (M <= 0 || I <= 0 || K <= 0) return 0;
+  if (I > INT32_MAX / 2) {
+    pico_host::set_error("swiglu gemm: width %d", I);
+    return -2;
+  }
+  pico::GemmPlan plan;
+  int rc = pico::whole_plan(M, 2 * I, plan);
+  if (rc) return rc;
+  pico::pair::OutMaps out = {};
+  rc = pico_host::make_tmap_2d(&out.d, act, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, I, M, (uint64_t)I * 2, 64,
+                               pico::pair::BM, pico_host::Swizzle::B128);
+  if (!rc && gate_up != nullptr) rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
+  if (!rc)
+    rc = pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU>(plan, x, w, out, M, 2 * I, K, ldx, ldw,
+                                                             gate_up != nullptr, stream);
+  return rc ? rc : pico::pair::launched();
+}
+
+extern "C" int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* gate_up, void* d_gate_up, int M, int I,
+                                    int K, int lddy, int ldw, cudaStream_t stream) {
+  if (M <= 0 || I <= 0 || K <= 0) return 0;
+  pico::GemmPlan plan;
+  int rc = pico::whole_plan(M, I, plan);
+  if (rc) return rc;
+  pico::pair::OutMaps out = {};
+  rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
+  if (!rc) rc = pico::half_maps(&out.d_gate, &out.d_up, d_gate_up, M, I);
+  if (!rc)
+    rc = pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD>(plan, dy, w, out, M, I, K, lddy, ldw, 1, stream);
+  return rc ? rc : pico::pair::launched();
+}

@@ -25,6 +25,8 @@ import torch.nn as nn
 
 from ..ops import attention as attn_ops
 from ..ops import embedding as emb_ops
+from ..ops import gated_mlp as gated_mlp_ops
+from ..ops import gemm as gemm_ops
 from ..ops import norm as norm_ops
 from ..ops import rope as rope_ops
 from ..ops import swiglu as swiglu_ops
@@ -187,6 +189,12 @@ class Attention(nn.Module):
         return self.out_proj(out)
 
 
+def hooked(mod: nn.Module) -> bool:
+    """Whether a call of ``mod`` does more than its forward pass (hooks on it or on all modules, a patched forward)."""
+    return bool(mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks
+                or "forward" in mod.__dict__ or torch.nn.modules.module._has_any_global_hook())
+
+
 class MLP(nn.Module):
     """SwiGLU feed-forward: down(silu(gate(x)) * up(x)) (picotron/model.py:236-258)."""
 
@@ -207,11 +215,21 @@ class MLP(nn.Module):
     def hidden(self, x):
         return swiglu_ops.swiglu(multi_linear([self.gate_proj, self.up_proj], x, cat=True))
 
+    def _one_op(self, x):
+        """The weights of ``ops.gated_mlp`` when the whole MLP can run as that op: unsharded linears (no collective
+        between them) and nobody watching the calls of the down projection, which it does not make."""
+        down = self.down_proj
+        if not (type(self.gate_proj) is type(self.up_proj) is type(down) is Linear) or hooked(down):
+            return None
+        ws = gemm_ops.WeightSet.of([self.gate_proj, self.up_proj])
+        return ws if gated_mlp_ops.fits(x, ws, down.weight) else None
+
     def forward(self, x, residual=None):
         if getattr(self.down_proj, "fused", None) is not None and residual is not None:
             # fused sequence parallelism: the reduce-scatter epilogue of the down projection adds the residual
             return self.down_proj(self.hidden(x), residual=residual)
-        y = self.down_proj(self.hidden(x))
+        ws = self._one_op(x)
+        y = self.down_proj(self.hidden(x)) if ws is None else gated_mlp_ops.gated_mlp(x, ws, self.down_proj.weight)
         return y if residual is None else y + residual
 
 
