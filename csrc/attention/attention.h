@@ -29,6 +29,11 @@ typedef struct {
   // optional: device buffer of 1024 uint64; CTA (0,0,0) of the forward kernel records globaltimer
   // stamps of its pipeline phases there (performance debugging). NULL = off.
   unsigned long long* trace;
+  // backward, optional (NULL = off): q and k were rotated (rotary embedding) with these tables, fp32 [positions,
+  // head_dim / 2], the first token of each sequence at position rope_pos0; dq and dk are rotated back
+  const float* rope_cos;
+  const float* rope_sin;
+  int rope_pos0;
 } PicoAttnParams;
 
 // out[b, sq, H, d] (bf16) and lse[b, H, sq] (fp32, natural log; -inf for rows without keys).

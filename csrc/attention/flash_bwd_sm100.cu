@@ -35,7 +35,8 @@
 // What binds it now is the chain of a tile through the softmax warps (exponentials, dS, their barriers).
 //
 // delta = rowsum(dO * O) comes from a small pre-pass; the dQ accumulator is scaled and converted to
-// bf16 by a post-pass. Every wait is bounded.
+// bf16 by a post-pass. Where q and k carry a rotary embedding, the post-pass also rotates dQ and dK back (dK in the
+// main kernel's epilogue measured 8 us more per call: 32 rows of the tables per load). Every wait is bounded.
 #include <cuda_bf16.h>
 #include <math_constants.h>
 
@@ -125,6 +126,75 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
     }
     for (int off = gsz >> 1; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
     if (item < total && li == 0) delta[((int64_t)b * p.heads + h) * p.seq_q + row] = acc;
+  }
+}
+
+// As attn_dq_convert_kernel, rotated back before the rounding, and then dk in place. An item is 8 columns of the first
+// half of a head and the 8 of the second half that they were rotated with. Bytes bind it; a rotation of its own read
+// and wrote dq once more. Whole backward, post-pass and rotation / this, us: 4 x 2048 x 32 x 64: 350 / 340; 8 x 1024 x 15/5
+// x 64: 92 / 86; 1 x 128 x 9/3 x 64: 15.2 / 13.9.
+__global__ void attn_unrotate_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
+                                     __nv_bfloat16* __restrict__ dk, PicoAttnParams p, int64_t dq_batch_stride,
+                                     int64_t dq_row_stride, int64_t dk_batch_stride, int64_t dk_row_stride) {
+  ahead_wait();
+  ahead_next();
+  const int half = p.head_dim / 2, per_head = half / 8;
+  const int64_t q_items = (int64_t)p.batch * p.seq_q * p.heads * per_head;
+  const int64_t items = q_items + (int64_t)p.batch * p.seq_k * p.kv_heads * per_head;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < items;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const bool is_q = i < q_items;
+    const int64_t n = is_q ? i : i - q_items;
+    const int heads = is_q ? p.heads : p.kv_heads, seq = is_q ? p.seq_q : p.seq_k;
+    const int v = (int)(n % per_head) * 8;
+    const int64_t u = n / per_head;
+    const int head = (int)(u % heads);
+    const int64_t t = u / heads;
+    const int row = (int)(t % seq);
+    const int64_t b = t / seq;
+    __nv_bfloat16* dst = (is_q ? dq + b * dq_batch_stride + row * dq_row_stride
+                               : dk + b * dk_batch_stride + row * dk_row_stride) + head * p.head_dim + v;
+    const int64_t at = (int64_t)(p.rope_pos0 + row) * half + v;
+    float lo[8], hi[8], c[8], s[8];
+#pragma unroll
+    for (int j = 0; j < 8; j += 4) {
+      *reinterpret_cast<float4*>(c + j) = *reinterpret_cast<const float4*>(p.rope_cos + at + j);
+      *reinterpret_cast<float4*>(s + j) = *reinterpret_cast<const float4*>(p.rope_sin + at + j);
+    }
+    if (is_q) {
+      const float* src = acc + u * p.head_dim + v;
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        *reinterpret_cast<float4*>(lo + j) = *reinterpret_cast<const float4*>(src + j);
+        *reinterpret_cast<float4*>(hi + j) = *reinterpret_cast<const float4*>(src + half + j);
+      }
+    } else {
+      const uint4 l = *reinterpret_cast<const uint4*>(dst), h = *reinterpret_cast<const uint4*>(dst + half);
+      const uint32_t lw[4] = {l.x, l.y, l.z, l.w}, hw[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        lo[2 * j] = __uint_as_float(lw[j] << 16);
+        lo[2 * j + 1] = __uint_as_float(lw[j] & 0xffff0000u);
+        hi[2 * j] = __uint_as_float(hw[j] << 16);
+        hi[2 * j + 1] = __uint_as_float(hw[j] & 0xffff0000u);
+      }
+    }
+    const float sc = is_q ? p.sm_scale : 1.f;      // dS is kept unscaled by the main kernel, dk has its scale
+    uint32_t ol[4], oh[4];
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      float x[4];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const float a = lo[j + k] * sc, g = hi[j + k] * sc;
+        x[k] = a * c[j + k] + g * s[j + k];
+        x[2 + k] = g * c[j + k] - a * s[j + k];
+      }
+      ol[j / 2] = pack_bf16x2(x[0], x[1]);
+      oh[j / 2] = pack_bf16x2(x[2], x[3]);
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(ol[0], ol[1], ol[2], ol[3]);
+    *reinterpret_cast<uint4*>(dst + half) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
   }
 }
 
@@ -692,7 +762,13 @@ extern "C" int pico_attention_bwd(const void* q, const void* k, const void* v, c
     rc = launch_bwd<128>(q, k, v, dout, lse, dk, dv, delta, dq_accum, p, do_batch_stride, do_row_stride,
                          dk_batch_stride, dk_row_stride, dv_batch_stride, dv_row_stride, stream);
   if (rc) return rc;
-  {
+  if (p->rope_cos != nullptr) {
+    const int64_t items = (rows + (int64_t)p->batch * p->seq_k * p->kv_heads) * (p->head_dim / 16);
+    int64_t blocks = (items + 255) / 256;
+    if (blocks > sms * 16) blocks = sms * 16;
+    pico_host::launch_ahead(attn_unrotate_kernel, (int)blocks, 256, 0, stream, dq_accum, (__nv_bfloat16*)dq,
+                            (__nv_bfloat16*)dk, *p, dq_batch_stride, dq_row_stride, dk_batch_stride, dk_row_stride);
+  } else {
     int64_t nvec = rows * p->head_dim / 8;
     int64_t blocks = (nvec + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;

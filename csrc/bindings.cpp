@@ -847,9 +847,24 @@ void attention_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
 void attention_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out,
                    const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq, at::Tensor& dk, at::Tensor& dv,
                    at::Tensor& delta, at::Tensor& dq_accum, double sm_scale, bool causal, int64_t q_pos0,
-                   int64_t k_pos0) {
+                   int64_t k_pos0, const c10::optional<at::Tensor>& cos, const c10::optional<at::Tensor>& sin,
+                   int64_t rope_pos0) {
   c10::cuda::CUDAGuard guard(q.device());
   PicoAttnParams p = attn_params(q, k, v, out, sm_scale, causal, q_pos0, k_pos0);
+  if (cos.has_value() && cos->defined()) {
+    TORCH_CHECK(sin.has_value() && sin->defined() && cos->is_cuda() && sin->is_cuda() &&
+                    cos->scalar_type() == at::kFloat && sin->scalar_type() == at::kFloat && cos->is_contiguous() &&
+                    sin->is_contiguous() && cos->dim() == 2 && cos->sizes() == sin->sizes() &&
+                    cos->size(1) == q.size(3) / 2,
+                "attention_bwd: rotary tables are fp32 [positions, head_dim / 2]");
+    TORCH_CHECK(rope_pos0 >= 0 && rope_pos0 + std::max(q.size(1), k.size(1)) <= cos->size(0),
+                "attention_bwd: rotary tables too short");
+    TORCH_CHECK(((reinterpret_cast<uintptr_t>(cos->data_ptr()) | reinterpret_cast<uintptr_t>(sin->data_ptr())) & 15) ==
+                    0, "attention_bwd: 16-byte aligned rotary tables");
+    p.rope_cos = cos->data_ptr<float>();
+    p.rope_sin = sin->data_ptr<float>();
+    p.rope_pos0 = (int)rope_pos0;
+  }
   for (const at::Tensor* t : std::initializer_list<const at::Tensor*>{&dout, &dq, &dk, &dv}) {
     TORCH_CHECK(t->scalar_type() == at::kBFloat16 && t->dim() == 4 && t->stride(3) == 1 &&
                     t->stride(2) == t->size(3), "attention_bwd: [b, s, h, d] bf16 tensors with packed heads");
@@ -890,7 +905,10 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
                                                                  const at::Tensor& k_, const at::Tensor& v_,
                                                                  const at::Tensor& out_, const at::Tensor& lse,
                                                                  double sm_scale, bool causal, int64_t q_pos0,
-                                                                 int64_t k_pos0) {
+                                                                 int64_t k_pos0,
+                                                                 const c10::optional<at::Tensor>& cos,
+                                                                 const c10::optional<at::Tensor>& sin,
+                                                                 int64_t rope_pos0) {
   at::Tensor q = pack_heads(q_), k = pack_heads(k_), v = pack_heads(v_);
   at::Tensor out = pack_heads(out_), dout = pack_heads(dout_);
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && dout.sizes() == q.sizes() &&
@@ -911,7 +929,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
   }
   const auto f32 = q.options().dtype(at::kFloat);
   at::Tensor delta = at::empty({b, H, sq}, f32), dq_accum = at::empty({b, sq, H, d}, f32);
-  attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, delta, dq_accum, sm_scale, causal, q_pos0, k_pos0);
+  attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, delta, dq_accum, sm_scale, causal, q_pos0, k_pos0, cos, sin,
+                rope_pos0);
   return {dq, dk, dv};
 }
 
@@ -939,7 +958,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("rmsnorm_new", &rmsnorm_new);
   m.def("attention_fwd_new", &attention_fwd_new);
-  m.def("attention_bwd_new", &attention_bwd_new);
+  m.def("attention_bwd_new", &attention_bwd_new, py::arg("dout"), py::arg("q"), py::arg("k"), py::arg("v"),
+        py::arg("out"), py::arg("lse"), py::arg("sm_scale"), py::arg("causal"), py::arg("q_pos0"), py::arg("k_pos0"),
+        py::arg("cos") = c10::optional<at::Tensor>(), py::arg("sin") = c10::optional<at::Tensor>(),
+        py::arg("rope_pos0") = 0);
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("rmsnorm_bwd_num_partials", &rmsnorm_bwd_num_partials);
@@ -968,7 +990,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_scatter_sum", &moe_scatter_sum);
   m.def("status_fetch", &status_fetch);
   m.def("attention_fwd", &attention_fwd);
-  m.def("attention_bwd", &attention_bwd);
+  m.def("attention_bwd", &attention_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("dout"),
+        py::arg("lse"), py::arg("dq"), py::arg("dk"), py::arg("dv"), py::arg("delta"), py::arg("dq_accum"),
+        py::arg("sm_scale"), py::arg("causal"), py::arg("q_pos0"), py::arg("k_pos0"),
+        py::arg("cos") = c10::optional<at::Tensor>(), py::arg("sin") = c10::optional<at::Tensor>(),
+        py::arg("rope_pos0") = 0);
   m.def("symm_alloc", &symm_alloc);
   m.def("symm_open", &symm_open);
   m.def("symm_close", &symm_close);

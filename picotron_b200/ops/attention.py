@@ -95,12 +95,14 @@ def flash_attention_forward(q, k, v, causal, sm_scale=None, q_pos0: int = 0, k_p
     return out, lse
 
 
-def flash_attention_backward(dout, q, k, v, out, lse, causal, sm_scale=None, q_pos0: int = 0, k_pos0: int = 0):
+def flash_attention_backward(dout, q, k, v, out, lse, causal, sm_scale=None, q_pos0: int = 0, k_pos0: int = 0,
+                             rope=None):
     """tcgen05 kernel: returns (dq, dk, dv) as column slices of one ``[b, s, (H + 2*Hkv)*d]`` buffer when
-    the sequence lengths match (so a fused QKV projection can consume them without a copy)."""
+    the sequence lengths match (so a fused QKV projection can consume them without a copy). ``rope``: (cos, sin, position
+    of the first token) of the rotary embedding that q and k carry; dq and dk are then those of the unrotated ones."""
     from . import count_launch, ext
     scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(q.shape[-1])
-    grads = ext().attention_bwd_new(dout, q, k, v, out, lse, scale, causal, q_pos0, k_pos0)
+    grads = ext().attention_bwd_new(dout, q, k, v, out, lse, scale, causal, q_pos0, k_pos0, *(rope or ()))
     count_launch(3)
     return grads
 
@@ -125,8 +127,8 @@ class _RopeAttentionFn(torch.autograd.Function):
 
     ``qkv``: [b, s, (H + 2*Hkv)*d] as the fused GEMM wrote it. q and k are rotated in place (the
     projection output is not needed by any other backward), attention runs on strided views, and
-    the backward writes dq/dk/dv straight into one ``[b, s, (H + 2*Hkv)*d]`` buffer, un-rotates
-    dq/dk in place and hands that buffer to the projection's backward: no split / cat / clone copies.
+    the backward writes dv and the un-rotated dq/dk straight into one ``[b, s, (H + 2*Hkv)*d]`` buffer and hands that
+    to the projection's backward: no split / cat / clone copies.
     """
 
     @staticmethod
@@ -149,21 +151,17 @@ class _RopeAttentionFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
-        from .rope import rope_inplace_
         raw, out, lse, cos_half, sin_half = ctx.saved_tensors
         H, Hkv, d, pos_offset, causal, sm_scale = ctx.dims
         b, s, _ = raw.shape
         q = raw[..., :H * d].view(b, s, H, d)
         k = raw[..., H * d:(H + Hkv) * d].view(b, s, Hkv, d)
         v = raw[..., (H + Hkv) * d:].view(b, s, Hkv, d)
-        dq, dk, dv = flash_attention_backward(dout.reshape(b, s, H, d), q, k, v, out, lse, causal, sm_scale)
+        dq, dk, dv = flash_attention_backward(dout.reshape(b, s, H, d), q, k, v, out, lse, causal, sm_scale,
+                                              rope=(cos_half, sin_half, pos_offset))
         fused = dq._base
         if fused is not None and fused.shape == raw.shape and fused.is_contiguous():
-            # dq | dk | dv of one buffer: un-rotate dq and dk in one launch
-            rope_inplace_(fused[..., :(H + Hkv) * d].view(b, s, H + Hkv, d), cos_half, sin_half, pos_offset, -1)
-            return fused, None, None, None, None, None, None, None, None
-        rope_inplace_(dq, cos_half, sin_half, pos_offset, -1)
-        rope_inplace_(dk, cos_half, sin_half, pos_offset, -1)
+            return fused, None, None, None, None, None, None, None, None      # dq | dk | dv of one buffer
         dqkv = torch.cat([dq.reshape(b, s, -1), dk.reshape(b, s, -1), dv.reshape(b, s, -1)], dim=-1)
         return dqkv, None, None, None, None, None, None, None, None
 

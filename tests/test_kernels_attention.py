@@ -238,3 +238,36 @@ def test_attention_tile_edges_against_64_bits(sq, sk, H, Hkv, d, causal, q_pos0)
     assert torch.allclose(lse.double(), torch.logsumexp(s6, -1).detach(), atol=1e-4, rtol=1e-5)
     for got, exp in zip(grads, want):
         assert off(got, exp) < 6.6e-3
+
+
+@pytest.mark.parametrize("b,s,H,Hkv,d,offset", [(1, 1, 1, 1, 64, 0), (2, 129, 4, 2, 64, 5), (1, 300, 3, 1, 128, 0),
+                                                (3, 97, 2, 2, 128, 31)])
+def test_rotary_attention_gradients_against_64_bits(b, s, H, Hkv, d, offset):
+    """dq and dk leave the attention backward rotated back (both halves of a head, ragged lengths, a position offset).
+    Values are bf16 roundings of rotated q and k forward (2^-9 each) and of the gradients: 2-norm within 1.5 %."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import attention as A
+    from picotron_b200.ops import rope as R
+    torch.manual_seed(s + d)
+    qkv = torch.randn(b, s, (H + 2 * Hkv) * d, device="cuda").to(torch.bfloat16)
+    cos, sin = R.get_cos_sin(s + offset + 3, d, 10000.0, device="cuda")
+    ch, sh = R.rope_tables_for_kernel(cos, sin)
+    x = qkv.clone().requires_grad_()
+    go = torch.randn(b, s, H * d, device="cuda").to(torch.bfloat16)
+    (g,) = torch.autograd.grad(A.rope_attention_fused(x * 1, H, Hkv, d, ch, sh, offset), x, go)
+    ops.check_status()
+    xr = qkv.double().requires_grad_()
+    heads = xr.view(b, s, H + 2 * Hkv, d)
+    c, n = (t[offset:offset + s].double()[None, :, None] for t in (ch, sh))
+    lo, hi = heads.chunk(2, -1)
+    turned = torch.cat([lo * c - hi * n, hi * c + lo * n], -1)
+    q, k, v = turned[:, :, :H], turned[:, :, H:H + Hkv], heads[:, :, H + Hkv:]
+    k, v = (t.repeat_interleave(H // Hkv, dim=2) for t in (k, v))
+    score = torch.einsum("bqhd,bkhd->bhqk", q, k) / d ** 0.5
+    score = score.masked_fill(torch.ones(s, s, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    out = torch.einsum("bhqk,bkhd->bqhd", score.softmax(-1), v).reshape(b, s, H * d)
+    (want,) = torch.autograd.grad(out, xr, go.double())
+    for lo_, hi_ in ((0, H), (H, H + Hkv), (H + Hkv, H + 2 * Hkv)):
+        a, w = g[..., lo_ * d:hi_ * d].double(), want[..., lo_ * d:hi_ * d]
+        if s > 1 or lo_ > H:                       # one token: its probability is 1 and dq, dk are rounding noise
+            assert (a - w).norm() <= 0.015 * w.norm()
