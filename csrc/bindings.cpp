@@ -18,8 +18,9 @@
 #include "fused/tp_comm.h"
 #include "gemm/gemm.h"
 #include "runtime/symm.h"
+#include "torch_ops.h"
 
-namespace {
+namespace pico_torch {
 
 void check(int rc, const char* what) {
   if (rc != 0) {
@@ -941,9 +942,11 @@ std::vector<int64_t> status_fetch() {
   return std::vector<int64_t>(out, out + 8);
 }
 
-}  // namespace
+}  // namespace pico_torch
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  using namespace pico_torch;
+  def_native_calls(m);
   m.def("gemm", &gemm);
   m.def("gemm_parts", &gemm_parts);
   m.def("gemm_parts_of_k",

@@ -24,6 +24,7 @@ import torch
 import torch.nn as nn
 
 from ..ops import attention as attn_ops
+from ..ops import ext, untracked, use_kernels
 from ..ops import embedding as emb_ops
 from ..ops import gated_mlp as gated_mlp_ops
 from ..ops import gemm as gemm_ops
@@ -315,6 +316,31 @@ class DecoderLayer(nn.Module):
         self.fused_ptb = fused_ptb
         self.ptb_overlap = fused_ptb and overlap
 
+    def native_weights(self, hidden: int):
+        """((weights and eps of this layer), (heads, kv heads, head_dim)) for ``dense_forward``, or None (see
+        ``Llama._native_layers``)."""
+        attn, mlp, n1 = self.attention, self.mlp, self.input_layernorm
+        if self.parallel_block or type(attn) is not Attention or type(mlp) is not MLP or attn.core is not _local_attention \
+                or attn.head_dim not in (64, 128) or "forward" in self.__dict__:
+            return None
+        n2, mods = self.post_attention_layernorm, (attn.q_proj, attn.k_proj, attn.v_proj, attn.out_proj, mlp.gate_proj,
+                                                   mlp.up_proj, mlp.down_proj)
+        if not (type(n1) is type(n2) is RMSNorm and all(type(m) is Linear for m in mods)) \
+                or any(hooked(m) for m in (self, n1, attn, attn.out_proj, n2, mlp, mlp.down_proj)):
+            return None
+        qkv, gate_up = gemm_ops.WeightSet.of(mods[:3]), gemm_ops.WeightSet.of(mods[4:6])
+        heads, kv_heads = attn.num_local_heads, attn.num_local_kv_heads
+        out, down = attn.out_proj.weight, mlp.down_proj.weight
+        inter, width = mlp.gate_proj.weight.shape[0], heads * attn.head_dim
+        if qkv.fused_weight is None or gate_up.fused_weight is None or not use_kernels(qkv.fused_weight) \
+                or any(w.dtype != torch.bfloat16 for w in (out, down, n1.weight, n2.weight)) \
+                or heads % kv_heads or qkv.fused_weight.shape != (width + 2 * kv_heads * attn.head_dim, hidden) \
+                or gate_up.fused_weight.shape != (2 * inter, hidden) or out.shape != (hidden, width) \
+                or down.shape != (hidden, inter) or not gemm_ops._gemm_ok(hidden, width, inter):
+            return None
+        return ((n1.weight, qkv.fused_weight, out, n2.weight, gate_up.fused_weight, down, n1.eps, n2.eps),
+                (heads, kv_heads, attn.head_dim))
+
     def forward(self, x, rope):
         if self.parallel_block:
             return self._forward_parallel(x, rope)
@@ -408,7 +434,37 @@ class Llama(nn.Module):
         self.final_norm.reset_parameters()
         self.final_proj.reset_parameters()
 
+    def _native_layers(self, input_ids):
+        """What ``dense_forward`` (``csrc/native_calls.cpp``) needs of the layers, or None where the pass has to go
+        through the modules: sharded, expert or parallel-block layers, weights that are not stored side by side, types
+        and sizes off the kernels, or anyone watching a module's call."""
+        emb, head = self.embedding, self.final_proj
+        if not (type(emb) is Embedding and type(head) is FinalProjection and type(self.final_norm) is RMSNorm
+                and input_ids.is_cuda and input_ids.dim() == 2 and input_ids.dtype == torch.int64
+                and input_ids.numel() > 0 and use_kernels(emb.weight, head.weight)
+                and not any(hooked(m) for m in (emb, self.final_norm, head))):
+            return None
+        hidden = emb.weight.shape[1]
+        if not gemm_ops._gemm_ok(hidden, head.weight.shape[0]) or head.weight.shape[1] != hidden:
+            return None
+        layers, shape = [], None
+        for layer in self.decoder_layers_iter():
+            one = layer.native_weights(hidden) if type(layer) is DecoderLayer else None
+            if one is None or (shape is not None and one[1] != shape):
+                return None
+            layers.append(one[0])
+            shape = one[1]
+        return (layers, shape) if layers else None
+
     def forward(self, input_ids, position_ids=None, hidden_states=None):
+        native = self._native_layers(input_ids) if untracked() else None
+        if native is not None:
+            layers, (heads, kv_heads, head_dim) = native
+            w = self.embedding.weight
+            _, _, (cos, sin) = self.rope.tables(w.device, w.dtype)
+            return ext().dense_forward(input_ids, w, layers, self.final_norm.weight, self.final_norm.eps,
+                                       self.final_proj.weight, heads, kv_heads, head_dim, cos, sin,
+                                       self.rope.pos_offset)
         x = self.embedding(input_ids)
         for layer in self.decoder_layers_iter():
             x = layer(x, self.rope)

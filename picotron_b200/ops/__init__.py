@@ -19,7 +19,8 @@ _EXT = None
 _EXT_LOCK = threading.Lock()
 _SO_PATH = Path(__file__).resolve().parent.parent / "_C.so"
 
-#: number of kernels of this library launched so far in this process (see ``count_launch``)
+#: number of kernels of this library launched so far in this process (see ``count_launch``); those that native code
+#: launches (``csrc/native_calls.cpp``) are counted there
 LAUNCHES = 0
 
 
@@ -29,7 +30,7 @@ def count_launch(n: int = 1) -> None:
 
 
 def launches() -> int:
-    return LAUNCHES
+    return LAUNCHES + (_EXT.native_launches() if _EXT is not None else 0)
 
 
 def ext():
@@ -76,8 +77,15 @@ def untracked() -> bool:
     """True when an op may run its kernel without an autograd function around it: gradients are off and nothing else
     looks at the call (function transforms, forward-mode differentiation and tracing do so also under
     ``no_grad``). An autograd function costs the host ~8 us, several times a small kernel."""
-    return not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() \
-        and forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
+    return not torch.is_grad_enabled() and unwatched()
+
+
+def unwatched() -> bool:
+    """True when nothing but reverse-mode autograd looks at an op: no function transform, no forward-mode level, no
+    tracing. Only then may an op be a native autograd node (``csrc/native_calls.cpp``); under the others the Python
+    function serves, or refuses, as ever."""
+    return not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0 \
+        and torch._C._get_tracing_state() is None
 
 
 def check_status(what: str = "") -> None:

@@ -108,6 +108,9 @@ def flash_attention_backward(dout, q, k, v, out, lse, causal, sm_scale=None, q_p
 
 
 class _FlashAttnFn(torch.autograd.Function):
+    """The Python form of ``AttentionNode`` (``csrc/native_calls.cpp``), for calls that something besides autograd
+    watches."""
+
     @staticmethod
     def forward(ctx, q, k, v, causal, sm_scale):
         out, lse = flash_attention_forward(q, k, v, causal, sm_scale)
@@ -187,10 +190,13 @@ def attention(q, k, v, causal: bool = True, sm_scale: float | None = None) -> to
     """Whole-sequence attention. q: [b, s, H, d]; k, v: [b, s, Hkv, d] -> [b, s, H, d]. bf16 CUDA
     tensors with head_dim 64 or 128 run on the tcgen05 flash-attention kernels of this library;
     everything else uses the torch restatement."""
-    from . import reference_ops_forced, untracked
+    from . import ext, reference_ops_forced, untracked, unwatched
     if kernel_supports(q, k) and not reference_ops_forced():
         if untracked():
             return flash_attention_forward(q, k, v, causal, sm_scale)[0]
+        if unwatched():
+            return ext().attention_node(q, k, v, bool(causal),
+                                        sm_scale if sm_scale is not None else 1.0 / math.sqrt(q.shape[-1]))
         return _FlashAttnFn.apply(q, k, v, causal, sm_scale)
     if q.is_cuda and q.dtype in (torch.bfloat16, torch.float16):
         H, kvh = q.shape[2], k.shape[2]

@@ -14,7 +14,7 @@ from __future__ import annotations
 import torch
 import torch.nn.functional as F
 
-from . import count_launch, ext, untracked, use_kernels
+from . import count_launch, ext, untracked, unwatched, use_kernels
 
 
 def linear_ref(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
@@ -119,6 +119,8 @@ def wgrad_into(weight: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
 
 
 class _LinearFn(torch.autograd.Function):
+    """The Python form of ``LinearNode`` (``csrc/native_calls.cpp``), for calls that something besides autograd watches."""
+
     @staticmethod
     def forward(ctx, x, w):
         y, x2, n = ext().linear_fwd(x, w)
@@ -145,6 +147,8 @@ def linear(x: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
             y, _, n = ext().linear_fwd(x, w)
             count_launch(n)
             return y
+        if unwatched():
+            return ext().linear_node(x, w)
         return _LinearFn.apply(x, w)
     if _ZB_MODE and torch.is_grad_enabled():
         return _LinearRefFn.apply(x, w)

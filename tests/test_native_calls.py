@@ -1,0 +1,160 @@
+"""Native autograd nodes and the native forward pass give what the Python operators and modules give, bit for bit, and
+leave to those what something else watches."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bf16(*shape):
+    return torch.randn(*shape, device="cuda").to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("kind", ["2d", "3d", "transposed", "sliced", "one row"])
+@pytest.mark.parametrize("needs", [(True, True), (True, False), (False, True)])
+def test_linear_node_matches_the_python_function(kind, needs):
+    from picotron_b200 import ops
+    from picotron_b200.ops import gemm
+    torch.manual_seed(0)
+    x = {"2d": lambda: _bf16(70, 64), "3d": lambda: _bf16(3, 35, 64), "transposed": lambda: _bf16(64, 72).t(),
+         "sliced": lambda: _bf16(5, 40, 76)[:, 1:38, 4:68], "one row": lambda: _bf16(1, 64)}[kind]().requires_grad_(needs[0])
+    w = _bf16(136, 64).requires_grad_(needs[1])
+    dy = _bf16(136, *x.shape[:-1]).movedim(0, -1) if kind != "one row" else _bf16(1, 136)     # not contiguous
+    wanted = [t for t in (x, w) if t.requires_grad]
+    before = ops.launches()
+    y = gemm.linear(x, w)
+    assert "LinearNode" in y.grad_fn.name()
+    got = torch.autograd.grad(y, wanted, dy)
+    assert ops.launches() - before == 1 + len(wanted)
+    ref = gemm._LinearFn.apply(x, w)
+    for a, b in zip(got, torch.autograd.grad(ref, wanted, dy)):
+        assert a.shape == b.shape and torch.equal(a, b)
+    assert torch.equal(y, ref)
+    ops.check_status()
+
+
+def test_linear_node_leaves_main_grad_and_postponed_gradients_to_python():
+    from picotron_b200.ops import gemm
+    torch.manual_seed(1)
+    x, w, dy = _bf16(40, 64).requires_grad_(), torch.nn.Parameter(_bf16(72, 64)), _bf16(40, 72)
+    with gemm.defer_wgrad() as queue:
+        gemm.linear(x, w).backward(dy)
+    assert w.grad is None and len(queue) == 1
+    gemm.run_deferred(queue)
+    late = w.grad.clone()
+    w.grad = None
+    y = gemm.linear(x, w)
+    w.main_grad = torch.zeros(72, 64, device="cuda")             # looked up when the gradient is there, not before
+    ready = []
+    w.grad_ready_hook = lambda: ready.append(1)
+    y.backward(dy)
+    assert w.grad is None and ready == [1]
+    want = dy.double().t() @ x.detach().double()
+    assert (w.main_grad.double() - want).norm() <= 1e-5 * want.norm()
+    assert (late.double() - want).norm() <= 2 ** -8 * want.norm()
+
+
+@pytest.mark.parametrize("b,s,H,Hkv,d,causal", [(1, 33, 3, 1, 64, False), (2, 130, 4, 4, 128, True)])
+def test_attention_node_matches_the_python_function(b, s, H, Hkv, d, causal):
+    """One to two key blocks per query: dQ has at most two addends and repeats bit for bit. Slices of a fused buffer."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import attention as A
+    torch.manual_seed(2)
+    heads = _bf16(b, s, H + 2 * Hkv, d).requires_grad_()
+    q, k, v = heads[:, :, :H], heads[:, :, H:H + Hkv], heads[:, :, H + Hkv:]
+    go = _bf16(b, H, s, d).transpose(1, 2)
+    before = ops.launches()
+    out = A.attention(q, k, v, causal, 0.2)
+    assert "AttentionNode" in out.grad_fn.name()
+    got = torch.autograd.grad(out, (q, k, v), go)
+    assert ops.launches() - before == 4
+    ref = A._FlashAttnFn.apply(q, k, v, causal, 0.2)
+    for a, r in zip(got, torch.autograd.grad(ref, (q, k, v), go)):
+        assert torch.equal(a, r)
+    assert torch.equal(out, ref)
+    ops.check_status()
+
+
+def test_nodes_keep_saved_tensor_hooks_and_refuse_a_second_pass():
+    from picotron_b200.ops import attention as A
+    from picotron_b200.ops import gemm
+    x, w = _bf16(24, 64).requires_grad_(), _bf16(64, 64).requires_grad_()
+    seen = []
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: seen.append(t.shape) or t.cpu(), lambda t: t.cuda()):
+        y = gemm.linear(x, w)
+        o = A.attention(*(t.view(1, 24, 1, 64) for t in (y, y, y)), True)
+    assert len(seen) == 2 + 5
+    o.sum().backward()
+    assert x.grad is not None and w.grad is not None
+    with pytest.raises(RuntimeError):
+        o.sum().backward()
+
+
+def test_watched_calls_take_the_python_functions():
+    """Transforms are refused as before; under a forward-mode level the Python function answers."""
+    from picotron_b200.ops import gemm
+    x, w = _bf16(24, 64), _bf16(64, 64)
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: gemm.linear(t, w).float().sum())(x)
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(lambda t: gemm.linear(t, w))(x.view(2, 12, 64))
+    with torch.autograd.forward_ad.dual_level():
+        y = gemm.linear(x.requires_grad_(), w)
+        assert "_LinearFn" in y.grad_fn.name()
+
+
+def _model(name, layers, seq):
+    from picotron_b200.config import MODEL_SHAPES
+    from picotron_b200.models.llama import Llama
+    from picotron_b200.param_store import ParamStore
+    from types import SimpleNamespace
+    shape = dict(MODEL_SHAPES["HuggingFaceTB/SmolLM-135M"], num_hidden_layers=layers, max_position_embeddings=seq,
+                 init_std=0.05, **name)
+    torch.manual_seed(3)
+    with torch.device("cuda"):
+        model = Llama(SimpleNamespace(**shape))
+    model.reset_parameters()
+    model = model.to(torch.bfloat16)
+    return model, ParamStore(model)
+
+
+@pytest.mark.parametrize("b,s", [(1, 1), (1, 33), (3, 130)])
+def test_native_forward_matches_the_modules(b, s):
+    from picotron_b200 import ops
+    model, _ = _model({}, 2, 130)
+    ids = torch.randint(0, 49152, (b, s), device="cuda")
+    with torch.no_grad():
+        assert model._native_layers(ids) is not None
+        native = model(ids)
+        seen = []
+        for mod in (model.decoder_layers[1], model.decoder_layers[0].mlp.down_proj, model.final_norm):
+            handle = mod.register_forward_hook(lambda *a: seen.append(1))
+            assert model._native_layers(ids) is None
+            assert torch.equal(model(ids), native)
+            handle.remove()
+        assert len(seen) == 3
+    ops.check_status()
+    assert native.shape == (b, s, 49152) and native.grad_fn is None
+    assert model(ids).grad_fn is not None                       # with gradients the modules run
+
+
+def test_native_forward_is_left_where_it_does_not_apply():
+    ids = torch.randint(0, 49152, (1, 20), device="cuda")
+    model, _ = _model({}, 2, 32)
+    model.rope.pos_offset = 4
+    with torch.no_grad():
+        native = model(ids)
+        handle = model.final_norm.register_forward_hook(lambda *a: None)
+        assert torch.equal(model(ids), native)
+        handle.remove()
+        with pytest.raises(RuntimeError, match="position table too short"):
+            model(torch.randint(0, 49152, (1, 29), device="cuda"))
+        model.decoder_layers[1].attention.core = lambda q, k, v, causal: q       # as context parallelism installs one
+        assert model._native_layers(ids) is None
+    parallel, _ = _model(dict(parallel_block=True), 2, 32)
+    loose, _ = _model({}, 1, 32)
+    for m in loose.modules():                                    # weights that are not stored side by side
+        m.__dict__.pop("_fused_group", None)
+    with torch.no_grad():
+        assert parallel._native_layers(ids) is None and loose._native_layers(ids) is None
+        assert parallel(ids).shape == loose(ids).shape == (1, 20, 49152)
