@@ -11,11 +11,6 @@ int64_t gemm(const at::Tensor& A, const at::Tensor& B, at::Tensor& D, int64_t M,
              int64_t ldb, int64_t ldd, bool a_mn_major, bool b_mn_major, int64_t out_mode, int64_t max_ctas);
 std::tuple<at::Tensor, int64_t> gemm_new(const at::Tensor& a, const at::Tensor& b, bool b_mn_major);
 std::tuple<at::Tensor, at::Tensor, int64_t> linear_fwd(const at::Tensor& x, const at::Tensor& w);
-std::tuple<at::Tensor, at::Tensor, int64_t> gemm_swiglu(const at::Tensor& x, const at::Tensor& w, bool keep,
-                                                        int64_t how);
-std::tuple<at::Tensor, at::Tensor, at::Tensor> rmsnorm_new(const at::Tensor& x,
-                                                           const c10::optional<at::Tensor>& residual,
-                                                           const at::Tensor& w, double eps);
 std::tuple<at::Tensor, at::Tensor> attention_fwd_new(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                                                      double sm_scale, bool causal, int64_t q_pos0, int64_t k_pos0);
 std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tensor& dout, const at::Tensor& q,
@@ -25,10 +20,6 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
                                                                  int64_t k_pos0, const c10::optional<at::Tensor>& cos,
                                                                  const c10::optional<at::Tensor>& sin,
                                                                  int64_t rope_pos0);
-void rope_inplace(at::Tensor& x, int64_t row_stride, int64_t rows, int64_t seq, int64_t pos_offset, int64_t nheads,
-                  int64_t d, const at::Tensor& cos, const at::Tensor& sin, int64_t sign);
-void embedding_fwd(const at::Tensor& W, const at::Tensor& ids, at::Tensor& out, int64_t rows, int64_t H,
-                   int64_t Vlocal, int64_t vocab_start);
 
 void def_native_calls(pybind11::module_& m);
 

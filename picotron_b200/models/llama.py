@@ -190,10 +190,15 @@ class Attention(nn.Module):
         return self.out_proj(out)
 
 
-def hooked(mod: nn.Module) -> bool:
-    """Whether a call of ``mod`` does more than its forward pass (hooks on it or on all modules, a patched forward)."""
+def own_hooks(mod: nn.Module) -> bool:
+    """Whether a call of ``mod`` does more than its class's forward pass: hooks on it, a patched forward."""
     return bool(mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks
-                or "forward" in mod.__dict__ or torch.nn.modules.module._has_any_global_hook())
+                or "forward" in mod.__dict__)
+
+
+def hooked(mod: nn.Module) -> bool:
+    """``own_hooks``, or hooks on all modules."""
+    return own_hooks(mod) or torch.nn.modules.module._has_any_global_hook()
 
 
 class MLP(nn.Module):
@@ -319,27 +324,36 @@ class DecoderLayer(nn.Module):
     def native_weights(self, hidden: int):
         """((weights and eps of this layer), (heads, kv heads, head_dim)) for ``dense_forward``, or None (see
         ``Llama._native_layers``)."""
-        attn, mlp, n1 = self.attention, self.mlp, self.input_layernorm
-        if self.parallel_block or type(attn) is not Attention or type(mlp) is not MLP or attn.core is not _local_attention \
-                or attn.head_dim not in (64, 128) or "forward" in self.__dict__:
+        if self.parallel_block:
             return None
-        n2, mods = self.post_attention_layernorm, (attn.q_proj, attn.k_proj, attn.v_proj, attn.out_proj, mlp.gate_proj,
-                                                   mlp.up_proj, mlp.down_proj)
-        if not (type(n1) is type(n2) is RMSNorm and all(type(m) is Linear for m in mods)) \
-                or any(hooked(m) for m in (self, n1, attn, attn.out_proj, n2, mlp, mlp.down_proj)):
+        # straight from the dicts: attribute access by name costs the host more than the rest of this
+        mods = self._modules
+        n1, attn, n2, mlp = (mods[k] for k in ("input_layernorm", "attention", "post_attention_layernorm", "mlp"))
+        if not (type(attn) is Attention and type(mlp) is MLP and type(n1) is type(n2) is RMSNorm) \
+                or attn.core is not _local_attention or attn.head_dim not in (64, 128):
             return None
-        qkv, gate_up = gemm_ops.WeightSet.of(mods[:3]), gemm_ops.WeightSet.of(mods[4:6])
+        am, mm = attn._modules, mlp._modules
+        q, k, v, out, gate, up, down = (am["q_proj"], am["k_proj"], am["v_proj"], am["out_proj"], mm["gate_proj"],
+                                        mm["up_proj"], mm["down_proj"])
+        for m in (q, k, v, out, gate, up, down):
+            if type(m) is not Linear:
+                return None
+        for m in (self, n1, attn, out, n2, mlp, down):
+            if own_hooks(m):
+                return None
+        qkv, gate_up = getattr(q, "_fused_group", None), getattr(gate, "_fused_group", None)
+        if qkv is None or gate_up is None or qkv.mods != [q, k, v] or gate_up.mods != [gate, up]:
+            return None
         heads, kv_heads = attn.num_local_heads, attn.num_local_kv_heads
-        out, down = attn.out_proj.weight, mlp.down_proj.weight
-        inter, width = mlp.gate_proj.weight.shape[0], heads * attn.head_dim
-        if qkv.fused_weight is None or gate_up.fused_weight is None or not use_kernels(qkv.fused_weight) \
-                or any(w.dtype != torch.bfloat16 for w in (out, down, n1.weight, n2.weight)) \
-                or heads % kv_heads or qkv.fused_weight.shape != (width + 2 * kv_heads * attn.head_dim, hidden) \
-                or gate_up.fused_weight.shape != (2 * inter, hidden) or out.shape != (hidden, width) \
-                or down.shape != (hidden, inter) or not gemm_ops._gemm_ok(hidden, width, inter):
+        w1, w2, w_out, w_down = (m._parameters["weight"] for m in (n1, n2, out, down))
+        inter, width = gate_up.splits[0], heads * attn.head_dim
+        if any(w.dtype != torch.bfloat16 for w in (qkv.weight, gate_up.weight, w_out, w_down, w1, w2)) \
+                or heads % kv_heads or qkv.weight.shape != (width + 2 * kv_heads * attn.head_dim, hidden) \
+                or gate_up.weight.shape != (2 * inter, hidden) or w_out.shape != (hidden, width) \
+                or w_down.shape != (hidden, inter) or not w_out.is_contiguous() or not w_down.is_contiguous() \
+                or not gemm_ops._gemm_ok(hidden, width, inter):
             return None
-        return ((n1.weight, qkv.fused_weight, out, n2.weight, gate_up.fused_weight, down, n1.eps, n2.eps),
-                (heads, kv_heads, attn.head_dim))
+        return ((w1, qkv.weight, w_out, w2, gate_up.weight, w_down, n1.eps, n2.eps), (heads, kv_heads, attn.head_dim))
 
     def forward(self, x, rope):
         if self.parallel_block:
@@ -442,10 +456,12 @@ class Llama(nn.Module):
         if not (type(emb) is Embedding and type(head) is FinalProjection and type(self.final_norm) is RMSNorm
                 and input_ids.is_cuda and input_ids.dim() == 2 and input_ids.dtype == torch.int64
                 and input_ids.numel() > 0 and use_kernels(emb.weight, head.weight)
-                and not any(hooked(m) for m in (emb, self.final_norm, head))):
+                and not torch.nn.modules.module._has_any_global_hook()
+                and not any(own_hooks(m) for m in (emb, self.final_norm, head))):
             return None
         hidden = emb.weight.shape[1]
-        if not gemm_ops._gemm_ok(hidden, head.weight.shape[0]) or head.weight.shape[1] != hidden:
+        if not gemm_ops._gemm_ok(hidden, head.weight.shape[0]) or head.weight.shape[1] != hidden \
+                or not (emb.weight.is_contiguous() and head.weight.is_contiguous()):
             return None
         layers, shape = [], None
         for layer in self.decoder_layers_iter():
