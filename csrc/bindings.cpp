@@ -146,7 +146,7 @@ std::tuple<at::Tensor, at::Tensor, int64_t> gemm_swiglu(const at::Tensor& x, con
   }
   at::Tensor gate_up = at::empty({keep ? M : 0, 2 * I}, x.options());
   check(pico_gemm_swiglu(x.data_ptr(), w.data_ptr(), keep ? gate_up.data_ptr() : nullptr, act.data_ptr(), (int)M,
-                         (int)I, (int)K, (int)x.stride(0), (int)w.stride(0), stream_of(x)),
+                         (int)I, (int)K, (int)x.stride(0), (int)w.stride(0), nullptr, 1, stream_of(x)),
         "gemm_swiglu");
   return {gate_up, act, 1};
 }
@@ -172,9 +172,47 @@ std::tuple<at::Tensor, int64_t> gemm_swiglu_bwd(const at::Tensor& dy, const at::
     return {out, launches + 1};
   }
   check(pico_gemm_swiglu_bwd(dy.data_ptr(), w.data_ptr(), gate_up.data_ptr(), out.data_ptr(), (int)M, (int)I, (int)K,
-                             (int)dy.stride(0), (int)w.stride(0), stream_of(dy)),
+                             (int)dy.stride(0), (int)w.stride(0), nullptr, 1, stream_of(dy)),
         "gemm_swiglu_bwd");
   return {out, 1};
+}
+
+// The same with row groups: w holds a [2 * I, K] (backward [K, I]) matrix for each, tile_group int32 the group of every
+// 128-row tile. (gate | up, activation) and the gradient of gate | up; rows of tiles of no group are not written.
+std::tuple<at::Tensor, at::Tensor> grouped_swiglu(const at::Tensor& x, const at::Tensor& w,
+                                                  const at::Tensor& tile_group, int64_t groups) {
+  TORCH_CHECK(x.is_cuda() && w.is_cuda() && tile_group.is_cuda() && x.scalar_type() == at::kBFloat16 &&
+                  w.scalar_type() == at::kBFloat16 && tile_group.scalar_type() == at::kInt && x.dim() == 2 &&
+                  w.dim() == 2 && x.stride(1) == 1 && w.stride(1) == 1 && x.size(1) == w.size(1) && groups > 0 &&
+                  x.size(1) % 8 == 0 && w.size(0) % (16 * groups) == 0 && tile_group.is_contiguous() &&
+                  tile_group.numel() >= (x.size(0) + 127) / 128,
+              "grouped_swiglu: bf16 rows, a [2 * I, K] weight per group, the group of every row tile");
+  const int64_t M = x.size(0), I = w.size(0) / groups / 2;
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor gate_up = at::empty({M, 2 * I}, x.options()), act = at::empty({M, I}, x.options());
+  check(pico_gemm_swiglu(x.data_ptr(), w.data_ptr(), gate_up.data_ptr(), act.data_ptr(), (int)M, (int)I,
+                         (int)x.size(1), (int)x.stride(0), (int)w.stride(0), tile_group.data_ptr<int>(), (int)groups,
+                         stream_of(x)),
+        "grouped_swiglu");
+  return {gate_up, act};
+}
+at::Tensor grouped_swiglu_bwd(const at::Tensor& dy, const at::Tensor& w, const at::Tensor& gate_up,
+                              const at::Tensor& tile_group, int64_t groups) {
+  TORCH_CHECK(dy.is_cuda() && w.is_cuda() && gate_up.is_cuda() && tile_group.is_cuda() &&
+                  dy.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
+                  gate_up.scalar_type() == at::kBFloat16 && tile_group.scalar_type() == at::kInt && dy.dim() == 2 &&
+                  w.dim() == 2 && gate_up.dim() == 2 && dy.stride(1) == 1 && w.stride(1) == 1 && groups > 0 &&
+                  w.size(0) == dy.size(1) * groups && w.size(1) % 8 == 0 && gate_up.is_contiguous() &&
+                  gate_up.size(0) == dy.size(0) && gate_up.size(1) == 2 * w.size(1) && tile_group.is_contiguous() &&
+                  tile_group.numel() >= (dy.size(0) + 127) / 128,
+              "grouped_swiglu_bwd: bf16 rows, a [K, I] weight per group, the group of every row tile");
+  c10::cuda::CUDAGuard guard(dy.device());
+  at::Tensor out = at::empty_like(gate_up);
+  check(pico_gemm_swiglu_bwd(dy.data_ptr(), w.data_ptr(), gate_up.data_ptr(), out.data_ptr(), (int)dy.size(0),
+                             (int)w.size(1), (int)dy.size(1), (int)dy.stride(0), (int)w.stride(0),
+                             tile_group.data_ptr<int>(), (int)groups, stream_of(dy)),
+        "grouped_swiglu_bwd");
+  return out;
 }
 
 // (norm(x + residual), x + residual or x, 1 / rms) of [rows, H] rows
@@ -956,6 +994,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("linear_fwd", &linear_fwd);
   m.def("gemm_swiglu", &gemm_swiglu, py::arg("x"), py::arg("w"), py::arg("keep"), py::arg("how") = -1);
   m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd, py::arg("dy"), py::arg("w"), py::arg("gate_up"), py::arg("how") = -1);
+  m.def("grouped_swiglu", &grouped_swiglu);
+  m.def("grouped_swiglu_bwd", &grouped_swiglu_bwd);
+  m.def("gemm_rows_on_pairs", [](int64_t M, int64_t groups) { return pico_gemm_rows_on_pairs((int)M, (int)groups) != 0; });
   m.def("gemm_swiglu_pays", [](int64_t M, int64_t I, int64_t K, bool keep, bool backward) {
     return pico_gemm_swiglu_pays((int)M, (int)I, (int)K, keep, backward) != 0;
   });

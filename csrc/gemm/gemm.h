@@ -39,13 +39,17 @@ int pico_gemm_bf16_parts(const void* A, const void* B, void* D, float* slabs, in
 //   pico_gemm_swiglu    : gate | up = x[M,K] * w[2*I,K]^T (gate rows first) into gate_up [M, 2*I], unless that is NULL,
 //                         and act[M,I] = silu(gate) * up
 //   pico_gemm_swiglu_bwd: d_gate_up [M, 2*I] from d_act = dy[M,K] * w[K,I] (which is not stored) and gate_up
-// bf16, 16-byte aligned, I and K multiples of 8; gate_up, act and d_gate_up contiguous.
+// bf16, 16-byte aligned, I and K multiples of 8; gate_up, act and d_gate_up contiguous. tile_group, groups: NULL and 1,
+// or row groups as in PicoGemmComm with a w for each of them, stacked, where pico_gemm_rows_on_pairs; rows of tiles of
+// no group are not written. Backward K is then a multiple of 64.
 int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, void* act, int M, int I, int K, int ldx, int ldw,
-                     cudaStream_t stream);
+                     const int* tile_group, int groups, cudaStream_t stream);
 // pico_gemm_swiglu_pays: whether they are faster than the plain product and a pass over its result.
 int pico_gemm_swiglu_pays(int M, int I, int K, int keep_gate, int backward);
 int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* gate_up, void* d_gate_up, int M, int I, int K,
-                         int lddy, int ldw, cudaStream_t stream);
+                         int lddy, int ldw, const int* tile_group, int groups, cudaStream_t stream);
+// Whether M rows in `groups` row groups run on CTA pairs.
+int pico_gemm_rows_on_pairs(int M, int groups);
 
 // Collective fusion (see csrc/runtime/symm.h for the symmetric-memory model).
 //   Row geometry: the M rows are pieces of blk_rows rows (a multiple of 128); piece p belongs to

@@ -42,6 +42,13 @@
 // sums depend on which pair is done first.) Measured, dW += dY^T X of 8192 tokens, uncut, cut, cut without an order:
 // 6144 x 2048 165, 158, 149 us; 960 x 960 (16 tiles) 52, 29, 24 us; 2048 x 2048 (64 tiles) 67, 77, 66 us.
 //
+// Row groups (the experts' products: rows of A and D in segments of whole 128-row tiles, one matrix B each): a pair takes
+// two neighbouring row tiles of one group, so each CTA's half of B serves both. The last tile of an odd segment goes
+// alone, its second CTA's rows are computed and dropped. Which tiles lead a pair is found at the start of the kernel
+// from the group of every row tile: no host read, no layout beside the one-CTA kernel's. One CTA / pairs, us: 49152 rows of
+// 64 experts, 2048 -> 2 x 1024 with the activation 427 / 373, its backward 286 / 231, 2048 x 1024 200 / 189; 8192 rows of
+// 8 experts 70 / 60, 48 / 39, 34 / 31.
+//
 // Operand layouts and raggedness as in gemm_bf16_sm100.cu.
 #include <cuda_bf16.h>
 
@@ -59,7 +66,9 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int kStagingBytes = 128 * 128;
 
-template <int BN, int OUT>
+constexpr int kMaxRowTiles = 640;         // of a product with row groups; their list takes the rest of shared memory
+
+template <int BN, int OUT, bool kGroups = false>
 struct Cfg {
   static constexpr bool kGate = OUT == GEMM_OUT_SWIGLU, kGateBwd = OUT == GEMM_OUT_SWIGLU_BWD;
   static constexpr bool kMovers = kGate || kGateBwd;
@@ -72,13 +81,18 @@ struct Cfg {
   static constexpr int kStages = kMovers ? 5 : 6;
   static constexpr int kNumStaging = kMovers ? 4 : 2;
   static constexpr int kTiles = kStages * kStageBytes + kNumStaging * kStagingBytes;
-  static constexpr int kSmemBytes = kTiles + (2 * kStages + 4 + 3 * kNumStaging) * 8 + 16;
+  static constexpr int kSmemBytes = kTiles + (2 * kStages + 4 + 3 * kNumStaging) * 8 + 16 +
+                                    (kGroups ? kMaxRowTiles * 4 : 0);
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
   static constexpr int kTmemCols = 2 * BN;
 };
 
 // One stretch of work of a pair: K blocks [kb0, kb1) of output tile (m, n), in units of pair tiles.
+// With row groups: the rows begin at `row`, the second CTA has none where the tile is alone, B is that of group grp.
 struct Work {
   int m, n, kb0, kb1;
+  int row, grp;
+  bool alone;
 };
 
 // The output tiles and the order in which they are worked on.
@@ -102,13 +116,20 @@ struct Tiles {
 };
 
 // Walks a pair's work: whole tiles first, then its share of the tiles that are cut along K.
+template <bool kGroups>
 struct Schedule : Tiles {
+  const uint32_t* lead;                     // row groups: the row tiles that lead a pair, see list_pairs
   int whole, pairs;                         // `whole` tiles are not cut
   int next;                                 // next whole tile of this pair
   int64_t unit, unit_end;                   // this pair's K blocks of the cut tiles
 
-  __device__ __forceinline__ Schedule(int M, int N, int K, int BN, int whole_, int pair_id, int pairs_)
-      : Tiles(M, N, K, BN), whole(whole_), pairs(pairs_), next(pair_id) {
+  __device__ __forceinline__ Schedule(int M, int N, int K, int BN, int whole_, int pair_id, int pairs_,
+                                      const uint32_t* lead_, int num_lead)
+      : Tiles(M, N, K, BN), lead(lead_), whole(whole_), pairs(pairs_), next(pair_id) {
+    if (kGroups) {
+      num_m = num_lead;
+      whole = num_m * num_n;
+    }
     const int64_t units = (int64_t)(num_m * num_n - whole) * num_kb;
     unit = units * pair_id / pairs;
     unit_end = units * (pair_id + 1) / pairs;
@@ -131,9 +152,41 @@ struct Schedule : Tiles {
       return false;
     }
     place(tile, w);
+    w.row = w.m * 2 * BM;
+    w.alone = false;
+    if (kGroups) {
+      const uint32_t e = lead[w.m];
+      w.row = (int)(e & 0x7fffu) * BM;
+      w.alone = (e & 0x8000u) == 0;
+      w.grp = (int)(e >> 16);
+    }
     return true;
   }
 };
+
+// The row tiles that lead a pair: those at an even place in their segment. Entry: the tile | 0x8000 where the next tile
+// is of the same group | group << 16. Called by one warp; returns their number.
+__device__ __forceinline__ int list_pairs(const int* __restrict__ tile_group, int num_tiles, uint32_t* list, int lane) {
+  int count = 0, begin = 0, prev = -2;               // begin: of the segment that the tiles before this stretch end in
+  for (int base = 0; base < num_tiles; base += 32) {
+    const int t = base + lane;
+    const int g = t < num_tiles ? __ldg(tile_group + t) : -1;
+    const int after = t + 1 < num_tiles ? __ldg(tile_group + t + 1) : -1;
+    int before = __shfl_up_sync(0xffffffffu, g, 1);
+    if (lane == 0) before = prev;
+    const uint32_t begins = __ballot_sync(0xffffffffu, g != before);
+    const uint32_t upto = begins & (0xffffffffu >> (31 - lane));
+    const int seg = upto != 0 ? base + 31 - __clz(upto) : begin;
+    const bool leads = g >= 0 && ((t - seg) & 1) == 0;
+    const uint32_t all = __ballot_sync(0xffffffffu, leads);
+    if (leads) list[count + __popc(all & ((1u << lane) - 1u))] =
+        (uint32_t)t | (after == g ? 0x8000u : 0u) | ((uint32_t)g << 16);
+    count += __popc(all);
+    if (begins != 0) begin = base + 31 - __clz(begins);
+    prev = __shfl_sync(0xffffffffu, g, 31);
+  }
+  return count;
+}
 
 // What an epilogue reads and writes.
 struct OutMaps {
@@ -166,11 +219,12 @@ __device__ __forceinline__ float swiglu_grad(float g, float u, float d, float& d
   return d * u * sg * (1.f + g * (1.f - sg));
 }
 
-template <int BN, int A_MN, int B_MN, int OUT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, OUT>::kThreads, 1)
+template <int BN, int A_MN, int B_MN, int OUT, bool kGroups>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, OUT, kGroups>::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                 const __grid_constant__ OutMaps out, int M, int N, int K, int whole, int keep_gate, int* status) {
-  using C = Cfg<BN, OUT>;
+                 const __grid_constant__ OutMaps out, int M, int N, int K, int whole, int keep_gate,
+                 const int* tile_group, int* status) {
+  using C = Cfg<BN, OUT, kGroups>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* staging = smem + C::kStages * C::kStageBytes;
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + C::kTiles);
@@ -223,7 +277,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr_smem, 0);
   ahead_wait();
   ahead_next();
-  Schedule sched(M, N, K, BN, whole, pair_id, pairs);
+  uint32_t* lead = reinterpret_cast<uint32_t*>(const_cast<int*>(abort_word) + 2);
+  int num_lead = 0;
+  if (kGroups) {
+    if (warp == 0) {
+      const int n = list_pairs(tile_group, (M + BM - 1) / BM, lead, lane);
+      if (lane == 0) abort_word[1] = n;
+    }
+    __syncthreads();
+    num_lead = abort_word[1];
+  }
+  Schedule<kGroups> sched(M, N, K, BN, whole, pair_id, pairs, lead, num_lead);
   Work w;
 
   if (warp == 0) {
@@ -233,7 +297,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       uint32_t phase = 0;
       bool ok = true;
       while (ok && sched.get(w)) {
-        const int m0 = w.m * 2 * BM + (int)rank * BM;
+        const int m0 = w.row + (int)rank * BM;
+        const int b0 = !kGroups ? 0 : w.grp * (B_MN == 0 ? N : K);       // this group's B in the stack of all
         // SwiGLU forward: gate columns in the first CTA, the up columns of the same numbers in the second
         const int n0 = C::kGate ? w.n * (BN / 2) + (int)rank * (N / 2) : w.n * BN + (int)rank * (BN / 2);
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
@@ -255,11 +320,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
               tma_load_2d_pair(sa + j * (64 * BK * 2), &tmap_a, bar, m0 + j * 64, k0);
           }
           if (B_MN == 0) {
-            tma_load_2d_pair(sb, &tmap_b, bar, k0, n0);  // box 64(K) x BN/2
+            tma_load_2d_pair(sb, &tmap_b, bar, k0, b0 + n0);  // box 64(K) x BN/2
           } else {
 #pragma unroll
             for (int j = 0; j < BN / 128; ++j)           // boxes 64(N) x 64(K)
-              tma_load_2d_pair(sb + j * (64 * BK * 2), &tmap_b, bar, n0 + j * 64, k0);
+              tma_load_2d_pair(sb + j * (64 * BK * 2), &tmap_b, bar, n0 + j * 64, b0 + k0);
           }
           if (++s == C::kStages) {
             s = 0;
@@ -350,8 +415,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         r.next();
       };
       while (ok && sched.get(w)) {
-        const int m0 = w.m * 2 * BM + (int)rank * BM;
-        if (m0 >= M) continue;
+        const int m0 = w.row + (int)rank * BM;
+        if (m0 >= M || (kGroups && rank != 0 && w.alone)) continue;
         if (C::kGate) {
           const int n0 = w.n * (BN / 2);
           for (int c = 0; ok && c < BN / 128 && n0 + c * 64 < N / 2; ++c) {
@@ -386,11 +451,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       return staging + r.b * kStagingBytes + row * 128;
     };
     while (ok && sched.get(w)) {
-      const int m0 = w.m * 2 * BM + (int)rank * BM;
+      const int m0 = w.row + (int)rank * BM;
       if (!mbar_wait_warp(&tmem_full[acc], acc_phase, abort_word, status, 400 + acc)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-      if (m0 >= M) {
+      if (m0 >= M || (kGroups && rank != 0 && w.alone)) {
         // nothing of this CTA's half lies in D
       } else if (C::kGate) {
         const int n0 = w.n * (BN / 2);
@@ -494,7 +559,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     uint32_t acc_phase = 0;
     int buf = 0;
     while (sched.get(w)) {
-      const int m0 = w.m * 2 * BM + (int)rank * BM;
+      const int m0 = w.row + (int)rank * BM;
       const int n0 = w.n * BN;
       const bool ok = mbar_wait(&tmem_full[acc], acc_phase, abort_word, status, 400 + acc);
       // uniform decision for the four epilogue warps (they share named barriers below)
@@ -515,7 +580,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll 1
       for (int c = 0; c < kChunks; ++c) {
         // skip what lies entirely outside D (uniform across threads)
-        if (n0 + c * kColsPerChunk >= N || m0 >= M) break;
+        if (n0 + c * kColsPerChunk >= N || m0 >= M || (kGroups && rank != 0 && w.alone)) break;
         uint8_t* sbuf = staging + buf * kStagingBytes;
         if (et == 0) tma_store_wait_read<kNumStaging - 1>();
         named_barrier_sync(1, kEpilogueThreads);
@@ -646,20 +711,23 @@ add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_
 }
 
 // Maps of the operands, the kernel's attributes and its launch.
-template <int BN, int A_MN, int B_MN, int OUT>
+// groups, tile_group: row groups, B has one matrix for each (1 and NULL: none).
+template <int BN, int A_MN, int B_MN, int OUT, bool kGroups = false>
 static int start(const GemmPlan& plan, const void* A, const void* B, const OutMaps& out, int M, int N, int K, int lda,
-                 int ldb, int keep_gate, cudaStream_t stream) {
-  using C = Cfg<BN, OUT>;
+                 int ldb, int keep_gate, cudaStream_t stream, int groups = 1, const int* tile_group = nullptr) {
+  using C = Cfg<BN, OUT, kGroups>;
   using pico_host::Swizzle;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap ta, tb;
   int rc = A_MN == 0 ? pico_host::make_tmap_2d(&ta, A, bf, 2, K, M, (uint64_t)lda * 2, 64, BM, Swizzle::B128)
                      : pico_host::make_tmap_2d(&ta, A, bf, 2, M, K, (uint64_t)lda * 2, 64, 64, Swizzle::B128);
   if (rc) return rc;
-  rc = B_MN == 0 ? pico_host::make_tmap_2d(&tb, B, bf, 2, K, N, (uint64_t)ldb * 2, 64, BN / 2, Swizzle::B128)
-                 : pico_host::make_tmap_2d(&tb, B, bf, 2, N, K, (uint64_t)ldb * 2, 64, 64, Swizzle::B128);
+  rc = B_MN == 0 ? pico_host::make_tmap_2d(&tb, B, bf, 2, K, (uint64_t)N * groups, (uint64_t)ldb * 2, 64, BN / 2,
+                                           Swizzle::B128)
+                 : pico_host::make_tmap_2d(&tb, B, bf, 2, N, (uint64_t)K * groups, (uint64_t)ldb * 2, 64, 64,
+                                           Swizzle::B128);
   if (rc) return rc;
-  auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT>;
+  auto kern = gemm_pair_kernel<BN, A_MN, B_MN, OUT, kGroups>;
   static int attr_dev = -1;  // per template instantiation
   int dev = 0;
   cudaGetDevice(&dev);
@@ -673,7 +741,7 @@ static int start(const GemmPlan& plan, const void* A, const void* B, const OutMa
   }
   const int pairs = plan.whole == plan.tiles && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
   pico_host::launch_ahead(kern, 2 * pairs, C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K, plan.whole,
-                          keep_gate, pico_status_buffer());
+                          keep_gate, tile_group, pico_status_buffer());
   return 0;
 }
 
@@ -746,6 +814,30 @@ int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M
   return pair::dispatch<256>(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, slabs, stream);
 }
 
+// `tiles` has room for one short tile per group, so from twice the groups on a group has about two. One CTA / pairs, us,
+// up, activation, down and their input gradients in all: 64 groups, 128 tiles (8192 rows) 389 / 391 to 160 tiles 478 /
+// 423, 208 tiles 668 / 672, 256 tiles 690 / 660 (rounds of whole tiles differ); 8 groups, 24 tiles 103 / 95. Below that
+// there are fewer pair tiles than pairs and their epilogues show: 8 groups, 16 tiles 64 / 68, 20 tiles 52 / 55.
+bool gemm_pair_takes_rows(int M, int groups) {
+  const int tiles = (M + pair::BM - 1) / pair::BM;
+  return tiles <= pair::kMaxRowTiles && tiles >= 2 * (int64_t)groups && tiles >= 24 &&
+         groups < 32768 && pico_host::num_sms() >= 2;
+}
+
+int gemm_pair_rows(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int b_mn,
+                   const int* tile_group, int groups, cudaStream_t stream) {
+  const GemmPlan plan{true, 256, pico_host::num_sms() / 2, INT32_MAX, INT32_MAX};     // counted in the kernel
+  pair::OutMaps out = {};
+  int rc = pico_host::make_tmap_2d(&out.d, D, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, M, (uint64_t)ldd * 2, 64,
+                                   pair::BM, pico_host::Swizzle::B128);
+  if (rc) return rc;
+  rc = b_mn ? pair::start<256, 0, 1, GEMM_OUT_BF16, true>(plan, A, B, out, M, N, K, lda, ldb, 0, stream, groups,
+                                                          tile_group)
+            : pair::start<256, 0, 0, GEMM_OUT_BF16, true>(plan, A, B, out, M, N, K, lda, ldb, 0, stream, groups,
+                                                          tile_group);
+  return rc ? rc : pair::launched();
+}
+
 // All tiles of an [M, N] product whole.
 static int whole_plan(int M, int N, GemmPlan& plan) {
   const int64_t tiles = (int64_t)((M + 255) / 256) * ((N + 255) / 256);
@@ -783,9 +875,19 @@ extern "C" int pico_gemm_swiglu_pays(int M, int I, int K, int keep_gate, int bac
   return plan.pair && (int64_t)M * I >= (backward ? 4000000 : keep_gate ? 2500000 : 1250000);
 }
 
+static bool row_groups_ok(int M, int K, int groups, bool whole_k) {
+  if (pico::gemm_pair_takes_rows(M, groups) && (!whole_k || K % pico::pair::BK == 0)) return true;
+  pico_host::set_error("swiglu gemm: row groups of two tiles and more on average, 24 to %d tiles, K (%d) a multiple of "
+                       "%d backward", pico::pair::kMaxRowTiles, K, pico::pair::BK);
+  return false;
+}
+
+extern "C" int pico_gemm_rows_on_pairs(int M, int groups) { return pico::gemm_pair_takes_rows(M, groups); }
+
 extern "C" int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, void* act, int M, int I, int K, int ldx,
-                                int ldw, cudaStream_t stream) {
+                                int ldw, const int* tile_group, int groups, cudaStream_t stream) {
   if (M <= 0 || I <= 0 || K <= 0) return 0;
+  if (tile_group != nullptr && !row_groups_ok(M, K, groups, false)) return -2;
   if (I > INT32_MAX / 2) {
     pico_host::set_error("swiglu gemm: width %d", I);
     return -2;
@@ -798,14 +900,19 @@ extern "C" int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, voi
                                pico::pair::BM, pico_host::Swizzle::B128);
   if (!rc && gate_up != nullptr) rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
   if (!rc)
-    rc = pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU>(plan, x, w, out, M, 2 * I, K, ldx, ldw,
-                                                             gate_up != nullptr, stream);
+    rc = tile_group != nullptr
+             ? pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU, true>(plan, x, w, out, M, 2 * I, K, ldx, ldw,
+                                                                         gate_up != nullptr, stream, groups, tile_group)
+             : pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU>(plan, x, w, out, M, 2 * I, K, ldx, ldw,
+                                                                   gate_up != nullptr, stream);
   return rc ? rc : pico::pair::launched();
 }
 
 extern "C" int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* gate_up, void* d_gate_up, int M, int I,
-                                    int K, int lddy, int ldw, cudaStream_t stream) {
+                                    int K, int lddy, int ldw, const int* tile_group, int groups,
+                                    cudaStream_t stream) {
   if (M <= 0 || I <= 0 || K <= 0) return 0;
+  if (tile_group != nullptr && !row_groups_ok(M, K, groups, true)) return -2;
   pico::GemmPlan plan;
   int rc = pico::whole_plan(M, I, plan);
   if (rc) return rc;
@@ -813,6 +920,9 @@ extern "C" int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* g
   rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
   if (!rc) rc = pico::half_maps(&out.d_gate, &out.d_up, d_gate_up, M, I);
   if (!rc)
-    rc = pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD>(plan, dy, w, out, M, I, K, lddy, ldw, 1, stream);
+    rc = tile_group != nullptr
+             ? pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD, true>(plan, dy, w, out, M, I, K, lddy, ldw, 1,
+                                                                             stream, groups, tile_group)
+             : pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD>(plan, dy, w, out, M, I, K, lddy, ldw, 1, stream);
   return rc ? rc : pico::pair::launched();
 }

@@ -209,7 +209,7 @@ static at::Tensor dense_forward(const at::Tensor& ids_, const at::Tensor& embedd
     norm(norm2, eps2);
     if (in_epilogue) {
       ok(pico_gemm_swiglu(normed, gate_up.data_ptr(), nullptr, act, (int)T, (int)inter, (int)hidden, (int)hidden,
-                          (int)hidden, stream), "gemm_swiglu");
+                          (int)hidden, nullptr, 1, stream), "gemm_swiglu");
     } else {
       product(normed, gate_up, gate_up_rows);
       ok(pico_swiglu_fwd(gate_up_rows, 2 * inter, act, (int)T, (int)inter, nullptr, stream), "swiglu_fwd");

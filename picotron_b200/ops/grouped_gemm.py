@@ -160,6 +160,49 @@ def grouped_linear(x: torch.Tensor, mods, layout: GroupLayout, out_rows: int) ->
     return _GroupedLinearFn.apply(x, w, layout, out_rows, None)
 
 
+class _GroupedMLPFn(torch.autograd.Function):
+    """``down(silu(gate(x)) * up(x))`` of every expert with the activation inside the grouped products (see
+    ``gated_mlp``). ``w_gu`` and ``w_down`` are fused views of parameters that carry ``main_grad`` buffers."""
+
+    @staticmethod
+    def forward(ctx, x, w_gu, w_down, layout, grad_gu, grad_down, *params):
+        gate_up, act = ext().grouped_swiglu(x, w_gu, layout.tile_group, layout.num_groups)
+        count_launch()
+        ctx.save_for_backward(x, w_gu, w_down, gate_up, act)
+        ctx.layout, ctx.grads, ctx.params = layout, (grad_gu, grad_down), params
+        return grouped_gemm_nt(act, w_down, layout, w_down.shape[0] // layout.num_groups)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x, w_gu, w_down, gate_up, act = ctx.saved_tensors
+        layout, (grad_gu, grad_down) = ctx.layout, ctx.grads
+        dy = dy.contiguous()
+        d_gate_up = ext().grouped_swiglu_bwd(dy, w_down, gate_up, layout.tile_group, layout.num_groups)
+        count_launch()
+        grouped_gemm_tn(dy, act, layout, grad_down, accumulate=True)
+        dx = grouped_gemm_nn(d_gate_up, w_gu, layout, gate_up.shape[1]) if ctx.needs_input_grad[0] else None
+        grouped_gemm_tn(d_gate_up, x, layout, grad_gu, accumulate=True)
+        for p in ctx.params:
+            hook = getattr(p, "grad_ready_hook", None)
+            if hook is not None:
+                hook()
+        return (dx, None, None, None, None, None) + (None,) * len(ctx.params)
+
+
+def grouped_mlp(x: torch.Tensor, gate_ups, downs, layout: GroupLayout):
+    """The gated MLPs of all experts over the padded expert-major ``x`` in one op, or None where its kernels do not apply:
+    ``gate_ups`` are gate and up of each expert in turn, ``downs`` the down projections. Rows past the last segment of the
+    layout are not written."""
+    from .gemm import WeightSet
+    gu, down = WeightSet.of(gate_ups), WeightSet.of(downs)
+    if gu.fused_main_grad is None or down.fused_main_grad is None or x.shape[0] == 0 or x.stride(-1) != 1 \
+            or (x.stride(0) * 2) % 16 or gu.fused_weight.dtype != x.dtype or not kernel_ok(x, x.shape[1], gu.splits[0]) \
+            or not ext().gemm_rows_on_pairs(x.shape[0], layout.num_groups):
+        return None
+    return _GroupedMLPFn.apply(x, gu.fused_weight, down.fused_weight, layout, gu.fused_main_grad, down.fused_main_grad,
+                               *gu.params, *down.params)
+
+
 def grouped_linear_ref(x, weights: List[torch.Tensor], layout: GroupLayout):
     """Plain PyTorch restatement (test oracle): per-expert ``F.linear`` on the padded layout."""
     seg = layout.seg_start.tolist()

@@ -265,13 +265,18 @@ class MoELayer(nn.Module):
 
     def _experts_on_layout(self, xp: torch.Tensor, layout, rows_in_use=None) -> torch.Tensor:
         """SwiGLU feed-forward of every local expert over the padded expert-major rows ``xp``: two
-        grouped GEMM launches around one SwiGLU kernel (the reference's fused-MoE composition,
+        grouped GEMM launches with the SwiGLU in the first (or, where few rows or separate weights rule that out,
+        around one SwiGLU kernel: the reference's fused-MoE composition,
         picotron/expert_parallel/megakernel.py:294-357)."""
         experts = list(self.local_experts)
         inter = experts[0].gate_proj.weight.shape[0]
-        gu = grouped_gemm.grouped_linear(xp, [m for e in experts for m in (e.gate_proj, e.up_proj)], layout, 2 * inter)
+        gate_ups, downs = [m for e in experts for m in (e.gate_proj, e.up_proj)], [e.down_proj for e in experts]
+        y = grouped_gemm.grouped_mlp(xp, gate_ups, downs, layout)
+        if y is not None:
+            return y
+        gu = grouped_gemm.grouped_linear(xp, gate_ups, layout, 2 * inter)
         # rows_in_use: device-side fill level of a buffer sized for the worst case (dropless exchange)
-        return grouped_gemm.grouped_linear(swiglu_ops.swiglu(gu, rows_in_use), [e.down_proj for e in experts], layout,
+        return grouped_gemm.grouped_linear(swiglu_ops.swiglu(gu, rows_in_use), downs, layout,
                                            experts[0].down_proj.weight.shape[0])
 
     def _dispatch(self, rows_sorted, plan: RoutePlan):

@@ -84,3 +84,89 @@ def test_mlp_module_takes_the_one_op_and_matches_the_separate_ones(keep_grad_of_
         if a is not None:
             assert (a.float() - b.float()).norm() <= 2 ** -8 * b.float().norm()
     assert all(p.grad is None for p in mlp.parameters())
+
+
+def _tiles(counts, spare):
+    """Group of every 128-row tile for groups of these many tiles, and `spare` tiles of no group behind them."""
+    return torch.tensor([g for g, c in enumerate(counts) for _ in range(c)] + [-1] * spare, dtype=torch.int32).cuda()
+
+
+@pytest.mark.parametrize("counts,spare,inter,hidden", [([1, 7, 16], 0, 64, 64), ([3, 0, 8, 1, 4], 9, 136, 128),
+                                                       ([33, 31, 1], 2, 320, 192), ([0, 0, 12], 13, 264, 64),
+                                                       ([2] * 40 + [9] * 40, 0, 192, 128)])
+def test_row_groups_on_pairs(counts, spare, inter, hidden):
+    """Odd and even segments, empty groups, tiles of no group, segments across the stretches of 32 tiles in which pairs
+    are listed, more pairs than the chip has: plain products and those with the activation, each row against its group's
+    matrix in 64 bits. Rows of no group keep what was there."""
+    from picotron_b200 import ops
+    torch.manual_seed(sum(counts))
+    G, tg = len(counts), _tiles(counts, spare)
+    P = tg.numel() * 128
+    assert ops.ext().gemm_rows_on_pairs(P, G)
+    group = tg.long().repeat_interleave(128)
+    x = torch.randn(P, hidden, device="cuda").to(torch.bfloat16)
+    dy = torch.randn(P, hidden, device="cuda").to(torch.bfloat16)
+    wg = (torch.randn(G, 2 * inter, hidden, device="cuda") / hidden ** 0.5).to(torch.bfloat16)
+    wd = (torch.randn(G, hidden, inter, device="cuda") / inter ** 0.5).to(torch.bfloat16)
+    gu, act = ops.ext().grouped_swiglu(x, wg.view(-1, hidden), tg, G)
+    dgu = ops.ext().grouped_swiglu_bwd(dy, wd.view(-1, inter), gu, tg, G)
+    plain = torch.full((P, 2 * inter), 7.0, device="cuda", dtype=torch.bfloat16)
+    back = torch.full((P, inter), 7.0, device="cuda", dtype=torch.bfloat16)
+    ops.ext().gemm_grouped(x, wg.view(-1, hidden), plain, P, 2 * inter, hidden, hidden, hidden, 2 * inter, False, False, 0,
+                           0, tg, G, 2 * inter)
+    ops.ext().gemm_grouped(dy, wd.view(-1, inter), back, P, inter, hidden, hidden, inter, inter, False, True, 0, 0, tg, G,
+                           hidden)
+    ops.check_status()
+    assert (plain[group < 0] == 7).all() and (back[group < 0] == 7).all()
+    for g, c in enumerate(counts):
+        if c == 0:
+            continue
+        r = group == g
+        xs, w, ds, v = x[r].double(), wg[g].double(), dy[r].double(), wd[g].double()
+        _close(plain[r], xs @ w.t(), xs.abs() @ w.abs().t(), hidden)
+        _close(back[r], ds @ v, ds.abs() @ v.abs(), hidden)
+        assert torch.equal(gu[r], plain[r])
+        ga, up = gu[r].double().chunk(2, -1)
+        _close(act[r], torch.nn.functional.silu(ga) * up, torch.zeros_like(ga), 0)
+        d, mag, sg = ds @ v, ds.abs() @ v.abs(), torch.sigmoid(ga)
+        dga, dup = dgu[r].chunk(2, -1)
+        _close(dup, d * ga * sg, mag * (ga * sg).abs(), hidden)
+        of = up * sg * (1 + ga * (1 - sg))
+        slack = 16 * 2.0 ** -24 * d.abs() * up.abs() * sg * (1 + ga.abs())
+        bound = (d * of).abs() * 2 ** -8 + mag * of.abs() * (hidden + 2) * 2.0 ** -24 + slack + 1e-30
+        assert ((dga.double() - d * of).abs() <= bound).all()
+
+
+def test_expert_layer_with_the_activation_inside_matches_the_separate_ops(monkeypatch):
+    from types import SimpleNamespace
+    from picotron_b200 import ops
+    from picotron_b200 import process_group_manager as pgm
+    from picotron_b200.ops import grouped_gemm
+    from picotron_b200.param_store import ParamStore
+    from picotron_b200.parallel.expert_parallel import MoELayer
+    if pgm.process_group_manager is None:
+        pgm.setup_process_group_manager(1, 1, 1, 1, 1)
+    torch.manual_seed(5)
+    cfg = SimpleNamespace(hidden_size=256, intermediate_size=192, num_experts=4, num_experts_per_tok=2, init_std=0.05)
+    with torch.device("cuda"):
+        layer = MoELayer(cfg).to(torch.bfloat16)
+    layer.train()
+    store = ParamStore(layer)
+    x = torch.randn(1, 1500, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+    dy = torch.randn_like(x)
+    got = []
+    for separate in (False, True):
+        if separate:
+            monkeypatch.setattr(grouped_gemm, "grouped_mlp", lambda *a: None)
+        store.zero_grads()
+        x.grad = None
+        before = ops.launches()
+        y = layer(x)
+        y.backward(dy)
+        got.append((y.detach().clone(), x.grad.clone(), store.flat_grads.clone(), ops.launches() - before))
+    ops.check_status()
+    assert torch.equal(got[0][0], got[1][0]) and got[0][3] == got[1][3] - 2
+    # the separate path rounds the activation's gradient; then the roundings of gate | up's gradient, of the routed rows'
+    # and of their sum fall differently on the two sides: 2^-9 of the value each, three of them on either side
+    for a, b in zip(got[0][1:3], got[1][1:3]):
+        assert (a.float() - b.float()).norm() <= (1 + 2 * 3) * 2 ** -9 * b.float().norm()
