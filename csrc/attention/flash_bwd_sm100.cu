@@ -1,6 +1,7 @@
 // Flash attention backward for sm_100a on tcgen05 tensor cores.
 //
-// One CTA owns a block of 128 keys of one (batch, kv head); K_j and V_j stay resident in shared
+// One CTA owns a block of 128 keys of one (batch, kv head), or where there are too few of those for the chip a share of
+// its steps (pico_attention_bwd_splits); K_j and V_j stay resident in shared
 // memory and the dK_j / dV_j accumulators stay in tensor memory while the CTA walks every query
 // block (and every query head of the group, for grouped-query attention) that can see those keys.
 // All score tiles are computed transposed (keys = tensor-memory lanes, queries = columns):
@@ -129,22 +130,27 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
   }
 }
 
-// As attn_dq_convert_kernel, rotated back before the rounding, and then dk in place. An item is 8 columns of the first
-// half of a head and the 8 of the second half that they were rotated with. Bytes bind it; a rotation of its own read
-// and wrote dq once more. Whole backward, post-pass and rotation / this, us: 4 x 2048 x 32 x 64: 350 / 340; 8 x 1024 x 15/5
-// x 64: 92 / 86; 1 x 128 x 9/3 x 64: 15.2 / 13.9.
-__global__ void attn_unrotate_kernel(const float* __restrict__ acc, __nv_bfloat16* __restrict__ dq,
-                                     __nv_bfloat16* __restrict__ dk, PicoAttnParams p, int64_t dq_batch_stride,
-                                     int64_t dq_row_stride, int64_t dk_batch_stride, int64_t dk_row_stride) {
+// The post-pass where there is more to do than attn_dq_convert_kernel does: dq from its accumulator, rotated back before
+// the rounding (kRope), dk rotated back in place (kRope) or, where the steps of a key block were split, dk and dv as the
+// sums of their splits' slabs, in order. An item is 8 columns of the first half of a head and the 8 of the second half
+// that they were rotated with. Bytes bind it; a rotation of its own read and wrote dq once more. Whole backward, post-pass
+// and rotation / this, us: 4 x 2048 x 32 x 64: 350 / 340; 8 x 1024 x 15/5 x 64: 92 / 86; 1 x 128 x 9/3 x 64: 15.2 / 13.9.
+template <bool kRope>
+__global__ void attn_finish_kernel(const float* __restrict__ acc, const float* __restrict__ slabs, int splits,
+                                   __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk,
+                                   __nv_bfloat16* __restrict__ dv, PicoAttnParams p, int64_t dq_batch_stride,
+                                   int64_t dq_row_stride, int64_t dk_batch_stride, int64_t dk_row_stride,
+                                   int64_t dv_batch_stride, int64_t dv_row_stride) {
   ahead_wait();
   ahead_next();
   const int half = p.head_dim / 2, per_head = half / 8;
   const int64_t q_items = (int64_t)p.batch * p.seq_q * p.heads * per_head;
-  const int64_t items = q_items + (int64_t)p.batch * p.seq_k * p.kv_heads * per_head;
+  const int64_t kv_items = (int64_t)p.batch * p.seq_k * p.kv_heads * per_head;
+  const int64_t items = q_items + (splits > 1 ? 2 : kRope ? 1 : 0) * kv_items;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < items;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const bool is_q = i < q_items;
-    const int64_t n = is_q ? i : i - q_items;
+    const bool is_q = i < q_items, is_v = i >= q_items + kv_items;
+    const int64_t n = is_q ? i : is_v ? i - q_items - kv_items : i - q_items;
     const int heads = is_q ? p.heads : p.kv_heads, seq = is_q ? p.seq_q : p.seq_k;
     const int v = (int)(n % per_head) * 8;
     const int64_t u = n / per_head;
@@ -153,20 +159,29 @@ __global__ void attn_unrotate_kernel(const float* __restrict__ acc, __nv_bfloat1
     const int row = (int)(t % seq);
     const int64_t b = t / seq;
     __nv_bfloat16* dst = (is_q ? dq + b * dq_batch_stride + row * dq_row_stride
-                               : dk + b * dk_batch_stride + row * dk_row_stride) + head * p.head_dim + v;
-    const int64_t at = (int64_t)(p.rope_pos0 + row) * half + v;
-    float lo[8], hi[8], c[8], s[8];
-#pragma unroll
-    for (int j = 0; j < 8; j += 4) {
-      *reinterpret_cast<float4*>(c + j) = *reinterpret_cast<const float4*>(p.rope_cos + at + j);
-      *reinterpret_cast<float4*>(s + j) = *reinterpret_cast<const float4*>(p.rope_sin + at + j);
-    }
-    if (is_q) {
-      const float* src = acc + u * p.head_dim + v;
+                          : is_v ? dv + b * dv_batch_stride + row * dv_row_stride
+                                 : dk + b * dk_batch_stride + row * dk_row_stride) + head * p.head_dim + v;
+    float lo[8], hi[8];
+    if (is_q || splits > 1) {
+      const int64_t slab = (int64_t)p.batch * p.seq_k * p.kv_heads * p.head_dim;
+      const float* src = (is_q ? acc : slabs + (is_v ? slab : 0)) + u * p.head_dim + v;
 #pragma unroll
       for (int j = 0; j < 8; j += 4) {
         *reinterpret_cast<float4*>(lo + j) = *reinterpret_cast<const float4*>(src + j);
         *reinterpret_cast<float4*>(hi + j) = *reinterpret_cast<const float4*>(src + half + j);
+      }
+      if (!is_q) {
+#pragma unroll 2
+        for (int sp = 1; sp < splits; ++sp) {
+          src += 2 * slab;
+#pragma unroll
+          for (int j = 0; j < 8; j += 4) {
+            const float4 l = *reinterpret_cast<const float4*>(src + j);
+            const float4 h = *reinterpret_cast<const float4*>(src + half + j);
+            lo[j] += l.x; lo[j + 1] += l.y; lo[j + 2] += l.z; lo[j + 3] += l.w;
+            hi[j] += h.x; hi[j + 1] += h.y; hi[j + 2] += h.z; hi[j + 3] += h.w;
+          }
+        }
       }
     } else {
       const uint4 l = *reinterpret_cast<const uint4*>(dst), h = *reinterpret_cast<const uint4*>(dst + half);
@@ -179,22 +194,32 @@ __global__ void attn_unrotate_kernel(const float* __restrict__ acc, __nv_bfloat1
         hi[2 * j + 1] = __uint_as_float(hw[j] & 0xffff0000u);
       }
     }
-    const float sc = is_q ? p.sm_scale : 1.f;      // dS is kept unscaled by the main kernel, dk has its scale
-    uint32_t ol[4], oh[4];
+    // dS is kept unscaled by the main kernel, and so are the slabs; a dk that is read back has its scale
+    const float sc = is_v || (!is_q && splits == 1) ? 1.f : p.sm_scale;
 #pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      float x[4];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const float a = lo[j + k] * sc, g = hi[j + k] * sc;
-        x[k] = a * c[j + k] + g * s[j + k];
-        x[2 + k] = g * c[j + k] - a * s[j + k];
-      }
-      ol[j / 2] = pack_bf16x2(x[0], x[1]);
-      oh[j / 2] = pack_bf16x2(x[2], x[3]);
+    for (int j = 0; j < 8; ++j) {
+      lo[j] *= sc;
+      hi[j] *= sc;
     }
-    *reinterpret_cast<uint4*>(dst) = make_uint4(ol[0], ol[1], ol[2], ol[3]);
-    *reinterpret_cast<uint4*>(dst + half) = make_uint4(oh[0], oh[1], oh[2], oh[3]);
+    if (kRope && !is_v) {
+      const int64_t at = (int64_t)(p.rope_pos0 + row) * half + v;
+#pragma unroll
+      for (int j = 0; j < 8; j += 4) {
+        float c[4], s[4];
+        *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(p.rope_cos + at + j);
+        *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(p.rope_sin + at + j);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float a = lo[j + k], g = hi[j + k];
+          lo[j + k] = a * c[k] + g * s[k];
+          hi[j + k] = g * c[k] - a * s[k];
+        }
+      }
+    }
+    *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf16x2(lo[0], lo[1]), pack_bf16x2(lo[2], lo[3]),
+                                                pack_bf16x2(lo[4], lo[5]), pack_bf16x2(lo[6], lo[7]));
+    *reinterpret_cast<uint4*>(dst + half) = make_uint4(pack_bf16x2(hi[0], hi[1]), pack_bf16x2(hi[2], hi[3]),
+                                                       pack_bf16x2(hi[4], hi[5]), pack_bf16x2(hi[6], hi[7]));
   }
 }
 
@@ -240,12 +265,13 @@ __device__ __forceinline__ int all_agree(bool ok) {
   return all_ok;
 }
 
-template <int D>
+template <int D, bool kSplit>
 __global__ void __launch_bounds__(BwdCfg<D>::kThreads, 1)
 flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__ lse,
                  const float* __restrict__ delta, __nv_bfloat16* __restrict__ dk, __nv_bfloat16* __restrict__ dv,
                  const PicoAttnParams p, int64_t dk_batch_stride, int64_t dk_row_stride,
-                 int64_t dv_batch_stride, int64_t dv_row_stride, int* status) {
+                 int64_t dv_batch_stride, int64_t dv_row_stride, float* __restrict__ slabs, int splits,
+                 int* status) {
   using Cfg = BwdCfg<D>;
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0) {   // swizzled tiles need 1024-byte alignment
@@ -280,7 +306,7 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
   const int lane = threadIdx.x & 31;
   // blocks are dispatched x-fastest: under a causal mask key block 0 has the most query blocks to
   // walk, so every (head, batch) of the heavy key blocks starts before any light one
-  const int kv_block = blockIdx.z;
+  const int kv_block = kSplit ? blockIdx.z / splits : blockIdx.z, split = kSplit ? blockIdx.z % splits : 0;
   const int kv_head = blockIdx.x;
   const int batch = blockIdx.y;
   const int group = p.heads / p.kv_heads;
@@ -294,7 +320,10 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
     i_min = need <= 0 ? 0 : (need + kBM - 1) / kBM;
   }
   const int nqb = max(0, num_q_blocks - i_min);
-  const int total = nqb * group;
+  // this split's stretch of the steps (query blocks of the first head of the group, then of the next, ...)
+  const int first = kSplit ? (int)((int64_t)nqb * group * split / splits) : 0;
+  const int total = kSplit ? (int)((int64_t)nqb * group * (split + 1) / splits) - first : nqb * group;
+  const int g0 = kSplit && nqb > 0 ? first / nqb : 0, i0 = i_min + (kSplit && nqb > 0 ? first % nqb : 0);
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -340,7 +369,7 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
 #pragma unroll
       for (int pn = 0; pn < Cfg::kPanels; ++pn)
         tma_load_4d(sK + pn * 16384, &maps.k, kv_full, pn * 64, kv_head, k0, batch);
-      int g = 0, i = i_min;
+      int g = g0, i = i0;
       for (int it = 0; it < total; ++it) {
         const int head = kv_head * group + g;
         const int qs = it % Cfg::kQStages, ds = it % Cfg::kDoStages;
@@ -468,7 +497,7 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
       stats[slot * 256 + 128 + dt] = -dl;
       mbar_arrive(&stat_full[slot]);
     };
-    int sg = 0, si = i_min;                                // step whose statistics are loaded next
+    int sg = g0, si = i0;                                // step whose statistics are loaded next
     auto stat_next = [&]() {
       if (++si == num_q_blocks) {
         si = i_min;
@@ -481,7 +510,7 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
       put_stat(it, l, dl);
       stat_next();
     }
-    int g = 0, i = i_min;
+    int g = g0, i = i0;
     for (int it = 0; it < total; ++it) {
       float l = 0.f, dl = 0.f;
       if (it + 2 < total) {
@@ -548,7 +577,7 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
     const bool key_valid = k0 + row < p.seq_k;
     const int key_pos = p.k_pos0 + k0 + row - p.q_pos0;     // in query indices
     bool alive = true;
-    int i = i_min;
+    int i = i0;
     for (int it = 0; it < total; ++it) {
       const int q0 = i * kBM;
       const float* st = stats + (it & 1) * 256 + part * kCols;
@@ -652,7 +681,13 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = 0u;
         }
-        if (key_valid) {
+        if (kSplit && key_valid) {
+          float* part = slabs + ((((int64_t)(2 * split + (is_dk ? 0 : 1)) * p.batch + batch) * p.seq_k + kidx) *
+                                     p.kv_heads + kv_head) * D + c * 32;
+#pragma unroll
+          for (int q4 = 0; q4 < 8; ++q4)
+            *reinterpret_cast<uint4*>(part + 4 * q4) = make_uint4(v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+        } else if (key_valid) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
             uint4 o;
@@ -679,12 +714,12 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
   }
 }
 
-template <int D>
+template <int D, bool kSplit>
 static int launch_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse,
                       void* dk, void* dv, const float* delta, float* dq_accum, const PicoAttnParams* p,
                       int64_t do_batch_stride, int64_t do_row_stride, int64_t dk_batch_stride,
-                      int64_t dk_row_stride, int64_t dv_batch_stride, int64_t dv_row_stride,
-                      cudaStream_t stream) {
+                      int64_t dk_row_stride, int64_t dv_batch_stride, int64_t dv_row_stride, float* slabs,
+                      int splits, cudaStream_t stream) {
   using Cfg = BwdCfg<D>;
   BwdMaps maps;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -704,7 +739,7 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
   rc = pico_host::make_tmap_bshd(&maps.dq_accum, dq_accum, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, D, p->heads,
                                  p->seq_q, p->batch, acc_row, acc_row * p->seq_q, 32, kBM);
   if (rc) return rc;
-  auto kern = flash_bwd_kernel<D>;
+  auto kern = flash_bwd_kernel<D, kSplit>;
   static int attr_dev = -1;
   int dev = 0;
   cudaGetDevice(&dev);
@@ -716,10 +751,10 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
     }
     attr_dev = dev;
   }
-  dim3 grid(p->kv_heads, p->batch, (p->seq_k + kBN - 1) / kBN);
+  dim3 grid(p->kv_heads, p->batch, (p->seq_k + kBN - 1) / kBN * splits);
   pico_host::launch_ahead(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, maps, lse, delta, (__nv_bfloat16*)dk,
                           (__nv_bfloat16*)dv, *p, dk_batch_stride, dk_row_stride, dv_batch_stride, dv_row_stride,
-                          pico_status_buffer());
+                          slabs, splits, pico_status_buffer());
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
     pico_host::set_error("attention bwd launch: %s", cudaGetErrorString(e));
@@ -730,13 +765,58 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
 
 }  // namespace pico
 
+// How many CTAs share the steps of a key block: the smallest modelled time, in steps (1.7 us at head_dim 64, 2.9 at 128).
+// CTAs are dealt heavy ones first, so the longest (under a causal mask that of the first keys, all query blocks of all
+// heads of the group) or the mean sets the time, each with ~3 steps around its own; a split costs its slabs, written and
+// read once, and ~2 steps for the longer post-pass. Measured, whole backward, us, unsplit / split: 1 x 8192 x 4/1 heads x
+// 128 (64 CTAs) 691 / 206; 4 x 2048 x 4/1 x 64 (64) 110 / 49; 1 x 4096 x 1 x 64 (32) 54 / 28; 1 x 256 x 9/3 x 64 (6)
+// 17.9 / 15.8; where the model says no, 2 x 2048 x 8 x 128 (256): 70 / 111 in two.
+extern "C" int pico_attention_bwd_splits(const PicoAttnParams* p) {
+  const int64_t key_blocks = (p->seq_k + pico::kBN - 1) / pico::kBN, q_blocks = (p->seq_q + pico::kBM - 1) / pico::kBM;
+  if (p->kv_heads <= 0 || p->batch <= 0 || key_blocks <= 0 || p->heads < p->kv_heads) return 1;
+  const double sms = pico_host::num_sms(), ctas = (double)key_blocks * p->kv_heads * p->batch;
+  if (ctas >= 4 * sms) return 1;
+  const int64_t group = p->heads / p->kv_heads;
+  int64_t longest = 0, sum = 0;
+  for (int64_t j = 0; j < key_blocks; ++j) {
+    int64_t seen = q_blocks;                           // query blocks that see a key of block j
+    if (p->causal) {
+      const int64_t need = (int64_t)p->k_pos0 + j * pico::kBN - p->q_pos0 - (pico::kBM - 1);
+      seen -= need <= 0 ? 0 : (need + pico::kBM - 1) / pico::kBM;
+    }
+    if (seen <= 0) continue;
+    longest = seen * group > longest ? seen * group : longest;
+    sum += seen * group;
+  }
+  const double work = (double)sum * p->kv_heads * p->batch;
+  // slab bytes per split at 5 TB/s, in steps
+  const double slab = 16.0 * p->batch * p->seq_k * p->kv_heads * p->head_dim / 5e6 / (p->head_dim == 64 ? 1.7 : 2.9);
+  int best = 1;
+  double best_time = 0;      // a split that gains less than a tenth (as 3 x 1333 x 15/5 x 64, 69.0 / 69.9) is left
+  for (int n = 1; n <= 16 && n <= longest && key_blocks * n <= 65535; ++n) {
+    const double own = (double)((longest + n - 1) / n) + 3, mean = (work + 3 * ctas * n) / sms;
+    const double time = (own > mean ? own : mean) + (n > 1 ? 2 + n * slab : 0);
+    if (n == 1) {
+      best_time = time * 0.85;
+    } else if (time < best_time) {
+      best = n;
+      best_time = time;
+    }
+  }
+  return best;
+}
+
 extern "C" int pico_attention_bwd(const void* q, const void* k, const void* v, const void* out, const void* dout,
                                   const float* lse, void* dq, void* dk, void* dv, float* delta, float* dq_accum,
                                   const PicoAttnParams* p, int64_t do_batch_stride, int64_t do_row_stride,
                                   int64_t dq_batch_stride, int64_t dq_row_stride, int64_t dk_batch_stride,
                                   int64_t dk_row_stride, int64_t dv_batch_stride, int64_t dv_row_stride,
-                                  cudaStream_t stream) {
+                                  float* slabs, int splits, cudaStream_t stream) {
   using namespace pico;
+  if (splits < 1 || (splits > 1 && slabs == nullptr)) {
+    pico_host::set_error("attention bwd: %d splits need slabs", splits);
+    return -2;
+  }
   if (p->batch <= 0 || p->seq_q <= 0 || p->seq_k <= 0 || p->heads <= 0) return 0;
   if (p->head_dim != 64 && p->head_dim != 128) {
     pico_host::set_error("attention: head_dim %d not supported (64 or 128)", p->head_dim);
@@ -754,20 +834,20 @@ extern "C" int pico_attention_bwd(const void* q, const void* k, const void* v, c
     pico_host::launch_ahead(attn_delta_kernel, (int)blocks, 256, 0, stream, (const __nv_bfloat16*)out,
                             (const __nv_bfloat16*)dout, delta, dq_accum, *p, do_batch_stride, do_row_stride);
   }
-  int rc;
-  if (p->head_dim == 64)
-    rc = launch_bwd<64>(q, k, v, dout, lse, dk, dv, delta, dq_accum, p, do_batch_stride, do_row_stride,
-                        dk_batch_stride, dk_row_stride, dv_batch_stride, dv_row_stride, stream);
-  else
-    rc = launch_bwd<128>(q, k, v, dout, lse, dk, dv, delta, dq_accum, p, do_batch_stride, do_row_stride,
-                         dk_batch_stride, dk_row_stride, dv_batch_stride, dv_row_stride, stream);
+  auto launch = p->head_dim == 64 ? (splits > 1 ? launch_bwd<64, true> : launch_bwd<64, false>)
+                                  : (splits > 1 ? launch_bwd<128, true> : launch_bwd<128, false>);
+  const int rc = launch(q, k, v, dout, lse, dk, dv, delta, dq_accum, p, do_batch_stride, do_row_stride, dk_batch_stride,
+                        dk_row_stride, dv_batch_stride, dv_row_stride, slabs, splits, stream);
   if (rc) return rc;
-  if (p->rope_cos != nullptr) {
-    const int64_t items = (rows + (int64_t)p->batch * p->seq_k * p->kv_heads) * (p->head_dim / 16);
+  if (p->rope_cos != nullptr || splits > 1) {
+    const int64_t items = (rows + (splits > 1 ? 2 : 1) * (int64_t)p->batch * p->seq_k * p->kv_heads) *
+                          (p->head_dim / 16);
     int64_t blocks = (items + 255) / 256;
     if (blocks > sms * 16) blocks = sms * 16;
-    pico_host::launch_ahead(attn_unrotate_kernel, (int)blocks, 256, 0, stream, dq_accum, (__nv_bfloat16*)dq,
-                            (__nv_bfloat16*)dk, *p, dq_batch_stride, dq_row_stride, dk_batch_stride, dk_row_stride);
+    pico_host::launch_ahead(p->rope_cos != nullptr ? attn_finish_kernel<true> : attn_finish_kernel<false>, (int)blocks,
+                            256, 0, stream, dq_accum, slabs, splits, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk,
+                            (__nv_bfloat16*)dv, *p, dq_batch_stride, dq_row_stride, dk_batch_stride, dk_row_stride,
+                            dv_batch_stride, dv_row_stride);
   } else {
     int64_t nvec = rows * p->head_dim / 8;
     int64_t blocks = (nvec + 255) / 256;

@@ -883,13 +883,12 @@ void attention_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
         "attention_fwd");
 }
 
-void attention_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out,
-                   const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq, at::Tensor& dk, at::Tensor& dv,
-                   at::Tensor& delta, at::Tensor& dq_accum, double sm_scale, bool causal, int64_t q_pos0,
-                   int64_t k_pos0, const c10::optional<at::Tensor>& cos, const c10::optional<at::Tensor>& sin,
-                   int64_t rope_pos0) {
-  c10::cuda::CUDAGuard guard(q.device());
-  PicoAttnParams p = attn_params(q, k, v, out, sm_scale, causal, q_pos0, k_pos0);
+// The scratch is fp32: delta of lse's size, dq_accum of q's, slabs for `splits` partial dk and dv (NULL where that is 1).
+static void run_attention_bwd(PicoAttnParams& p, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
+                              const at::Tensor& out, const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq,
+                              at::Tensor& dk, at::Tensor& dv, float* delta, float* dq_accum, float* slabs, int splits,
+                              const c10::optional<at::Tensor>& cos, const c10::optional<at::Tensor>& sin,
+                              int64_t rope_pos0) {
   if (cos.has_value() && cos->defined()) {
     TORCH_CHECK(sin.has_value() && sin->defined() && cos->is_cuda() && sin->is_cuda() &&
                     cos->scalar_type() == at::kFloat && sin->scalar_type() == at::kFloat && cos->is_contiguous() &&
@@ -908,15 +907,28 @@ void attention_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
     TORCH_CHECK(t->scalar_type() == at::kBFloat16 && t->dim() == 4 && t->stride(3) == 1 &&
                     t->stride(2) == t->size(3), "attention_bwd: [b, s, h, d] bf16 tensors with packed heads");
   }
+  check(pico_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+                           (const float*)lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta, dq_accum,
+                           &p, dout.stride(0), dout.stride(1), dq.stride(0), dq.stride(1), dk.stride(0), dk.stride(1),
+                           dv.stride(0), dv.stride(1), slabs, splits, stream_of(q)),
+        "attention_bwd");
+}
+
+void attention_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out,
+                   const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq, at::Tensor& dk, at::Tensor& dv,
+                   at::Tensor& delta, at::Tensor& dq_accum, double sm_scale, bool causal, int64_t q_pos0,
+                   int64_t k_pos0, const c10::optional<at::Tensor>& cos, const c10::optional<at::Tensor>& sin,
+                   int64_t rope_pos0) {
+  c10::cuda::CUDAGuard guard(q.device());
+  PicoAttnParams p = attn_params(q, k, v, out, sm_scale, causal, q_pos0, k_pos0);
   TORCH_CHECK(delta.scalar_type() == at::kFloat && dq_accum.scalar_type() == at::kFloat &&
                   dq_accum.is_contiguous() && delta.numel() >= lse.numel() && dq_accum.numel() >= q.numel(),
               "attention_bwd: fp32 scratch too small");
-  check(pico_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
-                           (const float*)lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
-                           (float*)delta.data_ptr(), (float*)dq_accum.data_ptr(), &p, dout.stride(0),
-                           dout.stride(1), dq.stride(0), dq.stride(1), dk.stride(0), dk.stride(1), dv.stride(0),
-                           dv.stride(1), stream_of(q)),
-        "attention_bwd");
+  const int splits = pico_attention_bwd_splits(&p);
+  at::Tensor slabs;
+  if (splits > 1) slabs = at::empty({2 * splits * k.numel()}, lse.options());
+  run_attention_bwd(p, q, k, v, out, dout, lse, dq, dk, dv, (float*)delta.data_ptr(), (float*)dq_accum.data_ptr(),
+                    splits > 1 ? slabs.data_ptr<float>() : nullptr, splits, cos, sin, rope_pos0);
 }
 
 bool packed_heads(const at::Tensor& t) {
@@ -966,10 +978,14 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
     dk = at::empty({b, sk, kvh, d}, q.options());
     dv = at::empty({b, sk, kvh, d}, q.options());
   }
-  const auto f32 = q.options().dtype(at::kFloat);
-  at::Tensor delta = at::empty({b, H, sq}, f32), dq_accum = at::empty({b, sq, H, d}, f32);
-  attention_bwd(q, k, v, out, dout, lse, dq, dk, dv, delta, dq_accum, sm_scale, causal, q_pos0, k_pos0, cos, sin,
-                rope_pos0);
+  // one allocation for the scratch, its parts on 256-byte boundaries
+  PicoAttnParams p = attn_params(q, k, v, out, sm_scale, causal, q_pos0, k_pos0);
+  const int splits = pico_attention_bwd_splits(&p);
+  const int64_t accum = b * sq * H * d, slabs = splits > 1 ? 2 * splits * b * sk * kvh * d : 0;
+  at::Tensor scratch = at::empty({accum + slabs + b * H * sq}, q.options().dtype(at::kFloat));
+  float* f = scratch.data_ptr<float>();
+  run_attention_bwd(p, q, k, v, out, dout, lse, dq, dk, dv, f + accum + slabs, f, splits > 1 ? f + accum : nullptr,
+                    splits, cos, sin, rope_pos0);
   return {dq, dk, dv};
 }
 

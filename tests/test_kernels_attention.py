@@ -271,3 +271,29 @@ def test_rotary_attention_gradients_against_64_bits(b, s, H, Hkv, d, offset):
         a, w = g[..., lo_ * d:hi_ * d].double(), want[..., lo_ * d:hi_ * d]
         if s > 1 or lo_ > H:                       # one token: its probability is 1 and dq, dk are rounding noise
             assert (a - w).norm() <= 0.015 * w.norm()
+
+
+@pytest.mark.parametrize("b,s,H,Hkv,d,causal", [(1, 300, 1, 1, 64, True), (1, 1100, 8, 1, 64, True),
+                                                (2, 513, 3, 1, 128, False), (1, 129, 2, 2, 128, True)])
+def test_key_blocks_shared_by_several_ctas(b, s, H, Hkv, d, causal):
+    """Few key blocks: the steps of each are split, unevenly and, where a block has fewer than shares, with empty ones.
+    dK and dV are sums of the shares in order, the same bits on each run; 2-norm of bf16 roundings of P and dS (2^-9 each)
+    and of the results against 64 bits."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import attention as A
+    torch.manual_seed(s)
+    q, go = (torch.randn(b, s, H, d, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(b, s, Hkv, d, device="cuda").to(torch.bfloat16) for _ in range(2))
+    out, lse = A.flash_attention_forward(q, k, v, causal)
+    first = [t.clone() for t in A.flash_attention_backward(go, q, k, v, out, lse, causal)]
+    for _ in range(3):
+        dq, dk, dv = A.flash_attention_backward(go, q, k, v, out, lse, causal)
+        assert torch.equal(dk, first[1]) and torch.equal(dv, first[2])
+    ops.check_status()
+    qr, kr, vr = (t.double().requires_grad_() for t in (q, k, v))
+    score = torch.einsum("bqhd,bkhd->bhqk", qr, kr.repeat_interleave(H // Hkv, 2)) / d ** 0.5
+    if causal:
+        score = score.masked_fill(torch.ones(s, s, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    ref = torch.einsum("bhqk,bkhd->bqhd", score.softmax(-1), vr.repeat_interleave(H // Hkv, 2))
+    for got, want in zip(first, torch.autograd.grad(ref, (qr, kr, vr), go.double())):
+        assert (got.double() - want).norm() <= 3 * 2 ** -9 * want.norm()
