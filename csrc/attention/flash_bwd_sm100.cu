@@ -130,11 +130,12 @@ __global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ out, const _
   }
 }
 
-// The post-pass where there is more to do than attn_dq_convert_kernel does: dq from its accumulator, rotated back before
-// the rounding (kRope), dk rotated back in place (kRope) or, where the steps of a key block were split, dk and dv as the
-// sums of their splits' slabs, in order. An item is 8 columns of the first half of a head and the 8 of the second half
-// that they were rotated with. Bytes bind it; a rotation of its own read and wrote dq once more. Whole backward, post-pass
-// and rotation / this, us: 4 x 2048 x 32 x 64: 350 / 340; 8 x 1024 x 15/5 x 64: 92 / 86; 1 x 128 x 9/3 x 64: 15.2 / 13.9.
+// The post-pass where there is more to do than attn_dq_convert_kernel does: dq from its accumulator, rotated back
+// before the rounding (kRope), dk rotated back in place (kRope) or, where the steps of a key block were split, dk and
+// dv as the sums of their splits' slabs, in order. An item is 8 columns of the first half of a head and the 8 of the
+// second half that they were rotated with. Bytes bind it; a rotation of its own read and wrote dq once more. Whole
+// backward, post-pass and rotation / this, us: 4 x 2048 x 32 x 64: 350 / 340; 8 x 1024 x 15/5 x 64: 92 / 86; 1 x 128 x
+// 9/3 x 64: 15.2 / 13.9.
 template <bool kRope>
 __global__ void attn_finish_kernel(const float* __restrict__ acc, const float* __restrict__ slabs, int splits,
                                    __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk,
@@ -686,7 +687,8 @@ flash_bwd_kernel(const __grid_constant__ BwdMaps maps, const float* __restrict__
                                      p.kv_heads + kv_head) * D + c * 32;
 #pragma unroll
           for (int q4 = 0; q4 < 8; ++q4)
-            *reinterpret_cast<uint4*>(part + 4 * q4) = make_uint4(v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
+            *reinterpret_cast<uint4*>(part + 4 * q4) =
+                make_uint4(v[4 * q4], v[4 * q4 + 1], v[4 * q4 + 2], v[4 * q4 + 3]);
         } else if (key_valid) {
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -765,12 +767,12 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
 
 }  // namespace pico
 
-// How many CTAs share the steps of a key block: the smallest modelled time, in steps (1.7 us at head_dim 64, 2.9 at 128).
-// CTAs are dealt heavy ones first, so the longest (under a causal mask that of the first keys, all query blocks of all
-// heads of the group) or the mean sets the time, each with ~3 steps around its own; a split costs its slabs, written and
-// read once, and ~2 steps for the longer post-pass. Measured, whole backward, us, unsplit / split: 1 x 8192 x 4/1 heads x
-// 128 (64 CTAs) 691 / 206; 4 x 2048 x 4/1 x 64 (64) 110 / 49; 1 x 4096 x 1 x 64 (32) 54 / 28; 1 x 256 x 9/3 x 64 (6)
-// 17.9 / 15.8; where the model says no, 2 x 2048 x 8 x 128 (256): 70 / 111 in two.
+// How many CTAs share the steps of a key block: the smallest modelled time, in steps (1.7 us at head_dim 64, 2.9 at
+// 128). CTAs are dealt heavy ones first, so the longest (under a causal mask that of the first keys, all query blocks
+// of all heads of the group) or the mean sets the time, each with ~3 steps around its own; a split costs its slabs,
+// written and read once, and ~2 steps for the longer post-pass. Measured, whole backward, us, unsplit / split: 1 x 8192
+// x 4/1 heads x 128 (64 CTAs) 691 / 206; 4 x 2048 x 4/1 x 64 (64) 110 / 49; 1 x 4096 x 1 x 64 (32) 54 / 28; 1 x 256 x
+// 9/3 x 64 (6) 17.9 / 15.8; where the model says no, 2 x 2048 x 8 x 128 (256): 70 / 111 in two.
 extern "C" int pico_attention_bwd_splits(const PicoAttnParams* p) {
   const int64_t key_blocks = (p->seq_k + pico::kBN - 1) / pico::kBN, q_blocks = (p->seq_q + pico::kBM - 1) / pico::kBM;
   if (p->kv_heads <= 0 || p->batch <= 0 || key_blocks <= 0 || p->heads < p->kv_heads) return 1;

@@ -126,8 +126,8 @@ std::tuple<at::Tensor, at::Tensor, int64_t> linear_fwd(const at::Tensor& x, cons
 }
 
 // Gated MLP products (gemm.h): w is [2 * I, K] with the gate rows first. (gate | up or an empty tensor, activation, the
-// number of kernels launched); how: the activation in the product's epilogue (1), by a pass of its own (0), or whichever
-// is faster (-1).
+// number of kernels launched); how: the activation in the product's epilogue (1), by a pass of its own (0), or
+// whichever is faster (-1).
 std::tuple<at::Tensor, at::Tensor, int64_t> gemm_swiglu(const at::Tensor& x, const at::Tensor& w, bool keep,
                                                         int64_t how) {
   TORCH_CHECK(x.is_cuda() && w.is_cuda() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16 &&
@@ -883,7 +883,8 @@ void attention_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
         "attention_fwd");
 }
 
-// The scratch is fp32: delta of lse's size, dq_accum of q's, slabs for `splits` partial dk and dv (NULL where that is 1).
+// The scratch is fp32: delta of lse's size, dq_accum of q's, slabs for `splits` partial dk and dv (NULL where that is
+// 1).
 static void run_attention_bwd(PicoAttnParams& p, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
                               const at::Tensor& out, const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq,
                               at::Tensor& dk, at::Tensor& dv, float* delta, float* dq_accum, float* slabs, int splits,
@@ -1012,7 +1013,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_swiglu_bwd", &gemm_swiglu_bwd, py::arg("dy"), py::arg("w"), py::arg("gate_up"), py::arg("how") = -1);
   m.def("grouped_swiglu", &grouped_swiglu);
   m.def("grouped_swiglu_bwd", &grouped_swiglu_bwd);
-  m.def("gemm_rows_on_pairs", [](int64_t M, int64_t groups) { return pico_gemm_rows_on_pairs((int)M, (int)groups) != 0; });
+  m.def("gemm_rows_on_pairs",
+        [](int64_t M, int64_t groups) { return pico_gemm_rows_on_pairs((int)M, (int)groups) != 0; });
   m.def("gemm_swiglu_pays", [](int64_t M, int64_t I, int64_t K, bool keep, bool backward) {
     return pico_gemm_swiglu_pays((int)M, (int)I, (int)K, keep, backward) != 0;
   });

@@ -179,12 +179,12 @@ ce_loss_grad_kernel(const __nv_bfloat16* __restrict__ logits, int64_t ldl,
   }
 }
 
-// Loss and gradient of whole (unsharded) rows in one pass over memory: a row is copied into shared memory, so the logits
-// are read once and not twice (1.6 instead of 2.4 GB at 8192 x 49152). Two rows fit an SM, one CTA each, and one is on
-// its way while the other is worked on. The row arrives in kPieces copies and its maximum is taken as they come; the
-// exponentials are evaluated twice, for the sum and for the gradient (6100 cycles of their unit per row of 49152 and
-// SM, its bytes take ~8000). In registers (12 vectors of 8 per thread) a row left 16 for everything else and spilled.
-// Measured at 8192 x 49152: 421 us in two passes, 294 here (1024 x 49152: 64, 49).
+// Loss and gradient of whole (unsharded) rows in one pass over memory: a row is copied into shared memory, so the
+// logits are read once and not twice (1.6 instead of 2.4 GB at 8192 x 49152). Two rows fit an SM, one CTA each, and one
+// is on its way while the other is worked on. The row arrives in kPieces copies and its maximum is taken as they come;
+// the exponentials are evaluated twice, for the sum and for the gradient (6100 cycles of their unit per row of 49152
+// and SM, its bytes take ~8000). In registers (12 vectors of 8 per thread) a row left 16 for everything else and
+// spilled. Measured at 8192 x 49152: 421 us in two passes, 294 here (1024 x 49152: 64, 49).
 constexpr int kPieces = 4;
 
 __global__ void __launch_bounds__(kCeThreads, 2)

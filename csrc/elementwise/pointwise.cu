@@ -424,8 +424,9 @@ extern "C" int pico_embedding_bwd(const void* dout, const int64_t* ids, float* d
     return -2;
   }
   const bool aligned = (reinterpret_cast<uintptr_t>(dW) & 15) == 0;   // the vector reductions need it
-  pico_host::launch_ahead(aligned ? embedding_bwd_kernel<true> : embedding_bwd_kernel<false>, grid_for((int64_t)rows * (H / 8), 256), 256, 0, stream,
-                          (const __nv_bfloat16*)dout, ids, dW, rows, H, Vlocal, vocab_start);
+  pico_host::launch_ahead(aligned ? embedding_bwd_kernel<true> : embedding_bwd_kernel<false>,
+                          grid_for((int64_t)rows * (H / 8), 256), 256, 0, stream, (const __nv_bfloat16*)dout, ids, dW,
+                          rows, H, Vlocal, vocab_start);
   return finish("embedding_bwd");
 }
 

@@ -711,7 +711,13 @@ static int run_gemm(const void* A, const void* B, void* D, int M, int N, int K, 
       comm->a_flags == nullptr && comm->num_groups > 0 && out_mode == pico::OUT_BF16 && max_ctas <= 0 &&
       a_mn_major == 0 && N > 128 && comm->b_group_rows == (b_mn_major ? K : N) &&
       (b_mn_major == 0 || K % pico::BK == 0) && pico::gemm_pair_takes_rows(M, comm->num_groups))
-    return pico::gemm_pair_rows(A, B, D, M, N, K, lda, ldb, ldd, b_mn_major, comm->tile_group, comm->num_groups, stream);
+    return pico::gemm_pair_rows(A, B, D, M, N, K, lda, ldb, ldd, b_mn_major, comm->tile_group, comm->num_groups,
+                                stream);
+  if (comm != nullptr && comm->seg_start != nullptr && comm->tile_group == nullptr && comm->d_num_dest == 0 &&
+      comm->a_flags == nullptr && comm->num_groups > 0 && out_mode == pico::OUT_F32_ACC && max_ctas <= 0 &&
+      a_mn_major == 1 && b_mn_major == 1 && M % pico::BM == 0 && N > 128 &&
+      pico::gemm_pair_takes_sums(M, N, comm->num_groups))
+    return pico::gemm_pair_sums(A, B, (float*)D, M, N, K, lda, ldb, ldd, comm->seg_start, comm->num_groups, stream);
   if (plan.pair)
     return pico::gemm_pair(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn_major, b_mn_major, out_mode, scratch, stream);
   auto one_cta = plan.bn == 64    ? pico::dispatch_bn<64>

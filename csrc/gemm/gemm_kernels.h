@@ -36,7 +36,12 @@ int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M
 // bf16 D with row groups (PicoGemmComm::tile_group, K-major A, B stacked) on the same kernel, and whether their number
 // and size suit it.
 bool gemm_pair_takes_rows(int M, int groups);
-int gemm_pair_rows(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int b_mn_major,
-                   const int* tile_group, int groups, cudaStream_t stream);
+int gemm_pair_rows(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
+                   int b_mn_major, const int* tile_group, int groups, cudaStream_t stream);
+
+// D += with reduction groups (PicoGemmComm::seg_start; MN-major operands, M a multiple of 128) on the same kernel.
+bool gemm_pair_takes_sums(int M, int N, int groups);
+int gemm_pair_sums(const void* A, const void* B, float* D, int M, int N, int K, int lda, int ldb, int ldd,
+                   const int* seg_start, int groups, cudaStream_t stream);
 
 }  // namespace pico

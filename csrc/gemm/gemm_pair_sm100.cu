@@ -25,13 +25,12 @@
 //             those of Wu); gate | up and the activation leave from the same registers
 //   backward: the gradient of the activation, dy Wd, meets gate and up in the epilogue and leaves as their gradients;
 //             it is never stored
-// What a pass of its own over gate | up took (402 MB forward, 671 MB backward for 8192 rows of 2 x 8192) then runs under
-// the main loop, 16 thousand cycles per tile at K = 2048. Values are rounded to bf16 before the activation, as that pass
-// reads them.
-// Product and pass / fused, us: 8192 rows, 2048 -> 8192: forward 420 / 363, backward 306 / 226; 16384, 2048 -> 5632:
-// 566 / 496, 414 / 338; 8192, 960 -> 2560: 77 / 65, 71 / 55. The movers' four buffers cost a stage of operands; six
-// buffers and four stages measured 393 and 284 us in the first line, and with four epilogue warps the short ones 1 us
-// more.
+// What a pass of its own over gate | up took (402 MB forward, 671 MB backward for 8192 rows of 2 x 8192) then runs
+// under the main loop, 16 thousand cycles per tile at K = 2048. Values are rounded to bf16 before the activation, as
+// that pass reads them. Product and pass / fused, us: 8192 rows, 2048 -> 8192: forward 420 / 363, backward 306 / 226;
+// 16384, 2048 -> 5632: 566 / 496, 414 / 338; 8192, 960 -> 2560: 77 / 65, 71 / 55. The movers' four buffers cost a stage
+// of operands; six buffers and four stages measured 393 and 284 us in the first line, and with four epilogue warps the
+// short ones 1 us more.
 //
 // Work split: output tiles are dealt to the pairs in whole rounds; where D is accumulated (weight
 // gradients) the tiles of the last, partial round are cut along K into equal shares for all pairs, so that
@@ -42,12 +41,16 @@
 // sums depend on which pair is done first.) Measured, dW += dY^T X of 8192 tokens, uncut, cut, cut without an order:
 // 6144 x 2048 165, 158, 149 us; 960 x 960 (16 tiles) 52, 29, 24 us; 2048 x 2048 (64 tiles) 67, 77, 66 us.
 //
-// Row groups (the experts' products: rows of A and D in segments of whole 128-row tiles, one matrix B each): a pair takes
-// two neighbouring row tiles of one group, so each CTA's half of B serves both. The last tile of an odd segment goes
-// alone, its second CTA's rows are computed and dropped. Which tiles lead a pair is found at the start of the kernel
-// from the group of every row tile: no host read, no layout beside the one-CTA kernel's. One CTA / pairs, us: 49152 rows of
-// 64 experts, 2048 -> 2 x 1024 with the activation 427 / 373, its backward 286 / 231, 2048 x 1024 200 / 189; 8192 rows of
-// 8 experts 70 / 60, 48 / 39, 34 / 31.
+// Row groups (the experts' products: rows of A and D in segments of whole 128-row tiles, one matrix B each): a pair
+// takes two neighbouring row tiles of one group, so each CTA's half of B serves both. The last tile of an odd segment
+// goes alone, its second CTA's rows are computed and dropped. Which tiles lead a pair is found at the start of the
+// kernel from the group of every row tile: no host read, no layout beside the one-CTA kernel's. One CTA / pairs, us:
+// 49152 rows of 64 experts, 2048 -> 2 x 1024 with the activation 427 / 373, its backward 286 / 231, 2048 x 1024 200 /
+// 189; 8192 rows of 8 experts 70 / 60, 48 / 39, 34 / 31.
+//
+// Reduction groups (the experts' weight gradients: D a stack of [M, N] blocks, each summed over its own stretch of K):
+// the tiles of all groups in turn, none cut. With K short the fp32 reductions bind them more than the tensor cores (4.1
+// TB/s read and written). One CTA / pairs, us: 64 experts, 53248 rows, 2048 x 2048 539 / 515, 2048 x 1024 308 / 259.
 //
 // Operand layouts and raggedness as in gemm_bf16_sm100.cu.
 #include <cuda_bf16.h>
@@ -68,7 +71,9 @@ constexpr int kStagingBytes = 128 * 128;
 
 constexpr int kMaxRowTiles = 640;         // of a product with row groups; their list takes the rest of shared memory
 
-template <int BN, int OUT, bool kGroups = false>
+enum Groups : int { kNoGroups, kRowGroups, kSumGroups };
+
+template <int BN, int OUT, int kGroups = kNoGroups>
 struct Cfg {
   static constexpr bool kGate = OUT == GEMM_OUT_SWIGLU, kGateBwd = OUT == GEMM_OUT_SWIGLU_BWD;
   static constexpr bool kMovers = kGate || kGateBwd;
@@ -82,7 +87,7 @@ struct Cfg {
   static constexpr int kNumStaging = kMovers ? 4 : 2;
   static constexpr int kTiles = kStages * kStageBytes + kNumStaging * kStagingBytes;
   static constexpr int kSmemBytes = kTiles + (2 * kStages + 4 + 3 * kNumStaging) * 8 + 16 +
-                                    (kGroups ? kMaxRowTiles * 4 : 0);
+                                    (kGroups == kRowGroups ? kMaxRowTiles * 4 : 0);
   static_assert(kSmemBytes <= 227 * 1024, "shared memory of one CTA");
   static constexpr int kTmemCols = 2 * BN;
 };
@@ -91,7 +96,7 @@ struct Cfg {
 // With row groups: the rows begin at `row`, the second CTA has none where the tile is alone, B is that of group grp.
 struct Work {
   int m, n, kb0, kb1;
-  int row, grp;
+  int row, grp;                             // reduction groups: D's block is `grp`
   bool alone;
 };
 
@@ -116,27 +121,39 @@ struct Tiles {
 };
 
 // Walks a pair's work: whole tiles first, then its share of the tiles that are cut along K.
-template <bool kGroups>
+template <int kGroups>
 struct Schedule : Tiles {
+  const int* seg_start;                     // reduction groups: where each begins in K
   const uint32_t* lead;                     // row groups: the row tiles that lead a pair, see list_pairs
   int whole, pairs;                         // `whole` tiles are not cut
   int next;                                 // next whole tile of this pair
   int64_t unit, unit_end;                   // this pair's K blocks of the cut tiles
 
   __device__ __forceinline__ Schedule(int M, int N, int K, int BN, int whole_, int pair_id, int pairs_,
-                                      const uint32_t* lead_, int num_lead)
-      : Tiles(M, N, K, BN), lead(lead_), whole(whole_), pairs(pairs_), next(pair_id) {
-    if (kGroups) {
+                                      const uint32_t* lead_, int num_lead, const int* seg_start_)
+      : Tiles(M, N, K, BN), seg_start(seg_start_), lead(lead_), whole(whole_), pairs(pairs_), next(pair_id) {
+    if (kGroups == kRowGroups) {
       num_m = num_lead;
       whole = num_m * num_n;
     }
-    const int64_t units = (int64_t)(num_m * num_n - whole) * num_kb;
+    const int64_t units = kGroups == kSumGroups ? 0 : (int64_t)(num_m * num_n - whole) * num_kb;
     unit = units * pair_id / pairs;
     unit_end = units * (pair_id + 1) / pairs;
   }
   __device__ __forceinline__ bool get(Work& w) {
     int tile;
-    if (next < whole) {
+    if (kGroups == kSumGroups) {
+      const int per_group = num_m * num_n;
+      do {
+        if (next >= whole) return false;
+        tile = next;
+        next += pairs;
+        w.grp = tile / per_group;
+        tile -= w.grp * per_group;
+        w.kb0 = __ldg(seg_start + w.grp) / BK;
+        w.kb1 = __ldg(seg_start + w.grp + 1) / BK;
+      } while (w.kb1 <= w.kb0);
+    } else if (next < whole) {
       tile = next;
       next += pairs;
       w.kb0 = 0;
@@ -154,7 +171,7 @@ struct Schedule : Tiles {
     place(tile, w);
     w.row = w.m * 2 * BM;
     w.alone = false;
-    if (kGroups) {
+    if (kGroups == kRowGroups) {
       const uint32_t e = lead[w.m];
       w.row = (int)(e & 0x7fffu) * BM;
       w.alone = (e & 0x8000u) == 0;
@@ -219,11 +236,11 @@ __device__ __forceinline__ float swiglu_grad(float g, float u, float d, float& d
   return d * u * sg * (1.f + g * (1.f - sg));
 }
 
-template <int BN, int A_MN, int B_MN, int OUT, bool kGroups>
+template <int BN, int A_MN, int B_MN, int OUT, int kGroups>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Cfg<BN, OUT, kGroups>::kThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                  const __grid_constant__ OutMaps out, int M, int N, int K, int whole, int keep_gate,
-                 const int* tile_group, int* status) {
+                 const int* group_array, int* status) {
   using C = Cfg<BN, OUT, kGroups>;
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* staging = smem + C::kStages * C::kStageBytes;
@@ -279,15 +296,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   ahead_next();
   uint32_t* lead = reinterpret_cast<uint32_t*>(const_cast<int*>(abort_word) + 2);
   int num_lead = 0;
-  if (kGroups) {
+  if (kGroups == kRowGroups) {
     if (warp == 0) {
-      const int n = list_pairs(tile_group, (M + BM - 1) / BM, lead, lane);
+      const int n = list_pairs(group_array, (M + BM - 1) / BM, lead, lane);
       if (lane == 0) abort_word[1] = n;
     }
     __syncthreads();
     num_lead = abort_word[1];
   }
-  Schedule<kGroups> sched(M, N, K, BN, whole, pair_id, pairs, lead, num_lead);
+  Schedule<kGroups> sched(M, N, K, BN, whole, pair_id, pairs, lead, num_lead, group_array);
   Work w;
 
   if (warp == 0) {
@@ -298,7 +315,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       bool ok = true;
       while (ok && sched.get(w)) {
         const int m0 = w.row + (int)rank * BM;
-        const int b0 = !kGroups ? 0 : w.grp * (B_MN == 0 ? N : K);       // this group's B in the stack of all
+        const int b0 = kGroups != kRowGroups ? 0 : w.grp * (B_MN == 0 ? N : K);   // this group's B in the stack
         // SwiGLU forward: gate columns in the first CTA, the up columns of the same numbers in the second
         const int n0 = C::kGate ? w.n * (BN / 2) + (int)rank * (N / 2) : w.n * BN + (int)rank * (BN / 2);
         for (int kb = w.kb0; kb < w.kb1; ++kb) {
@@ -416,7 +433,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       };
       while (ok && sched.get(w)) {
         const int m0 = w.row + (int)rank * BM;
-        if (m0 >= M || (kGroups && rank != 0 && w.alone)) continue;
+        if (m0 >= M || (kGroups == kRowGroups && rank != 0 && w.alone)) continue;
         if (C::kGate) {
           const int n0 = w.n * (BN / 2);
           for (int c = 0; ok && c < BN / 128 && n0 + c * 64 < N / 2; ++c) {
@@ -455,7 +472,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       if (!mbar_wait_warp(&tmem_full[acc], acc_phase, abort_word, status, 400 + acc)) break;
       tc_fence_after();
       const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
-      if (m0 >= M || (kGroups && rank != 0 && w.alone)) {
+      if (m0 >= M || (kGroups == kRowGroups && rank != 0 && w.alone)) {
         // nothing of this CTA's half lies in D
       } else if (C::kGate) {
         const int n0 = w.n * (BN / 2);
@@ -580,7 +597,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll 1
       for (int c = 0; c < kChunks; ++c) {
         // skip what lies entirely outside D (uniform across threads)
-        if (n0 + c * kColsPerChunk >= N || m0 >= M || (kGroups && rank != 0 && w.alone)) break;
+        if (n0 + c * kColsPerChunk >= N || m0 >= M || (kGroups == kRowGroups && rank != 0 && w.alone)) break;
         uint8_t* sbuf = staging + buf * kStagingBytes;
         if (et == 0) tma_store_wait_read<kNumStaging - 1>();
         named_barrier_sync(1, kEpilogueThreads);
@@ -612,12 +629,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         fence_proxy_async_smem();
         named_barrier_sync(1, kEpilogueThreads);
         if (et == 0) {
-          if (OUT == GEMM_OUT_F32_ACC && w.kb0 != 0)       // not the first piece of its tile: this pair's slab
+          const int y = m0 + (kGroups == kSumGroups ? w.grp * M : 0);
+          if (OUT == GEMM_OUT_F32_ACC && kGroups == kNoGroups && w.kb0 != 0)   // not the first piece: this pair's slab
             tma_store_2d(&out.slabs, sbuf, c * kColsPerChunk, (2 * pair_id + (int)rank) * BM);
           else if (OUT == GEMM_OUT_F32_ACC)
-            tma_reduce_add_2d(&out.d, sbuf, n0 + c * kColsPerChunk, m0);
+            tma_reduce_add_2d(&out.d, sbuf, n0 + c * kColsPerChunk, y);
           else
-            tma_store_2d(&out.d, sbuf, n0 + c * kColsPerChunk, m0);
+            tma_store_2d(&out.d, sbuf, n0 + c * kColsPerChunk, y);
           tma_store_commit();
         }
         buf ^= 1;
@@ -711,14 +729,16 @@ add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_
 }
 
 // Maps of the operands, the kernel's attributes and its launch.
-// groups, tile_group: row groups, B has one matrix for each (1 and NULL: none).
-template <int BN, int A_MN, int B_MN, int OUT, bool kGroups = false>
+// groups, group_array: row groups and the group of every row tile (B has a matrix for each), or the beginnings of
+// reduction groups.
+template <int BN, int A_MN, int B_MN, int OUT, int kGroups = kNoGroups>
 static int start(const GemmPlan& plan, const void* A, const void* B, const OutMaps& out, int M, int N, int K, int lda,
-                 int ldb, int keep_gate, cudaStream_t stream, int groups = 1, const int* tile_group = nullptr) {
+                 int ldb, int keep_gate, cudaStream_t stream, int groups = 1, const int* group_array = nullptr) {
   using C = Cfg<BN, OUT, kGroups>;
   using pico_host::Swizzle;
   const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   CUtensorMap ta, tb;
+  if (kGroups != kRowGroups) groups = 1;           // in the maps of the operands
   int rc = A_MN == 0 ? pico_host::make_tmap_2d(&ta, A, bf, 2, K, M, (uint64_t)lda * 2, 64, BM, Swizzle::B128)
                      : pico_host::make_tmap_2d(&ta, A, bf, 2, M, K, (uint64_t)lda * 2, 64, 64, Swizzle::B128);
   if (rc) return rc;
@@ -741,7 +761,7 @@ static int start(const GemmPlan& plan, const void* A, const void* B, const OutMa
   }
   const int pairs = plan.whole == plan.tiles && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
   pico_host::launch_ahead(kern, 2 * pairs, C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K, plan.whole,
-                          keep_gate, tile_group, pico_status_buffer());
+                          keep_gate, group_array, pico_status_buffer());
   return 0;
 }
 
@@ -814,10 +834,11 @@ int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M
   return pair::dispatch<256>(plan, A, B, D, M, N, K, lda, ldb, ldd, a_mn, b_mn, out_mode, slabs, stream);
 }
 
-// `tiles` has room for one short tile per group, so from twice the groups on a group has about two. One CTA / pairs, us,
-// up, activation, down and their input gradients in all: 64 groups, 128 tiles (8192 rows) 389 / 391 to 160 tiles 478 /
-// 423, 208 tiles 668 / 672, 256 tiles 690 / 660 (rounds of whole tiles differ); 8 groups, 24 tiles 103 / 95. Below that
-// there are fewer pair tiles than pairs and their epilogues show: 8 groups, 16 tiles 64 / 68, 20 tiles 52 / 55.
+// `tiles` has room for one short tile per group, so from twice the groups on a group has about two. One CTA / pairs,
+// us, up, activation, down and their input gradients in all: 64 groups, 128 tiles (8192 rows) 389 / 391 to 160 tiles
+// 478 / 423, 208 tiles 668 / 672, 256 tiles 690 / 660 (rounds of whole tiles differ); 8 groups, 24 tiles 103 / 95.
+// Below that there are fewer pair tiles than pairs and their epilogues show: 8 groups, 16 tiles 64 / 68, 20 tiles 52 /
+// 55.
 bool gemm_pair_takes_rows(int M, int groups) {
   const int tiles = (M + pair::BM - 1) / pair::BM;
   return tiles <= pair::kMaxRowTiles && tiles >= 2 * (int64_t)groups && tiles >= 24 &&
@@ -831,11 +852,34 @@ int gemm_pair_rows(const void* A, const void* B, void* D, int M, int N, int K, i
   int rc = pico_host::make_tmap_2d(&out.d, D, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, N, M, (uint64_t)ldd * 2, 64,
                                    pair::BM, pico_host::Swizzle::B128);
   if (rc) return rc;
-  rc = b_mn ? pair::start<256, 0, 1, GEMM_OUT_BF16, true>(plan, A, B, out, M, N, K, lda, ldb, 0, stream, groups,
-                                                          tile_group)
-            : pair::start<256, 0, 0, GEMM_OUT_BF16, true>(plan, A, B, out, M, N, K, lda, ldb, 0, stream, groups,
-                                                          tile_group);
+  auto start = b_mn ? pair::start<256, 0, 1, GEMM_OUT_BF16, pair::kRowGroups>
+                    : pair::start<256, 0, 0, GEMM_OUT_BF16, pair::kRowGroups>;
+  rc = start(plan, A, B, out, M, N, K, lda, ldb, 0, stream, groups, tile_group);
   return rc ? rc : pair::launched();
+}
+
+// Four rounds and more; with fewer the last one costs more than wider tiles save (8 groups of 320 rows, 2048 x 1024,
+// 256 tiles: 21.8 us on one CTA, 23.6 on pairs; 16 groups of 584, 512 tiles: 63.9, 63.2).
+bool gemm_pair_takes_sums(int M, int N, int groups) {
+  return (int64_t)((M + 255) / 256) * ((N + 255) / 256) * groups >= 4 * (pico_host::num_sms() / 2) &&
+         pico_host::num_sms() >= 2;
+}
+
+int gemm_pair_sums(const void* A, const void* B, float* D, int M, int N, int K, int lda, int ldb, int ldd,
+                   const int* seg_start, int groups, cudaStream_t stream) {
+  const int64_t tiles = (int64_t)((M + 255) / 256) * ((N + 255) / 256) * groups;
+  if (tiles > INT32_MAX) {
+    pico_host::set_error("grouped gemm: too many tiles");
+    return -2;
+  }
+  const GemmPlan plan{true, 256, pico_host::num_sms() / 2, (int)tiles, (int)tiles};
+  pair::OutMaps out = {};
+  const int rc = pico_host::make_tmap_2d(&out.d, D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, N, (uint64_t)M * groups,
+                                         (uint64_t)ldd * 4, 32, pair::BM, pico_host::Swizzle::B128);
+  if (rc) return rc;
+  const int rc2 = pair::start<256, 1, 1, GEMM_OUT_F32_ACC, pair::kSumGroups>(plan, A, B, out, M, N, K, lda, ldb, 0,
+                                                                             stream, groups, seg_start);
+  return rc2 ? rc2 : pair::launched();
 }
 
 // All tiles of an [M, N] product whole.
@@ -861,9 +905,9 @@ static int half_maps(CUtensorMap* gate, CUtensorMap* up, const void* gu, int row
 
 }  // namespace pico
 
-// The fused form ends on an epilogue that nothing overlaps, 3 to 5 us longer than that of the plain product; the pass it
-// saves takes its launch and its bytes. So it pays from some number of activations on, where the plain product runs on
-// pairs too (elsewhere its narrower tiles waste less). Measured, product and pass / fused, us:
+// The fused form ends on an epilogue that nothing overlaps, 3 to 5 us longer than that of the plain product; the pass
+// it saves takes its launch and its bytes. So it pays from some number of activations on, where the plain product runs
+// on pairs too (elsewhere its narrower tiles waste less). Measured, product and pass / fused, us:
 //   forward           512 x 960 x 2560 12.3 / 13.1, 256 x 2048 x 8192 18.9 / 19.2, 4096 x 576 x 1536 21.4 / 21.1
 //   .. without gate|up 512 x 576 x 1536 8.3 / 8.6, 512 x 960 x 2560 12.3 / 10.9, 256 x 2048 x 8192 18.9 / 16.9
 //   backward          1024 x 960 x 2560 13.8 / 14.3, 4096 x 576 x 1536 20.0 / 18.7
@@ -899,12 +943,9 @@ extern "C" int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, voi
   rc = pico_host::make_tmap_2d(&out.d, act, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, I, M, (uint64_t)I * 2, 64,
                                pico::pair::BM, pico_host::Swizzle::B128);
   if (!rc && gate_up != nullptr) rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
-  if (!rc)
-    rc = tile_group != nullptr
-             ? pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU, true>(plan, x, w, out, M, 2 * I, K, ldx, ldw,
-                                                                         gate_up != nullptr, stream, groups, tile_group)
-             : pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU>(plan, x, w, out, M, 2 * I, K, ldx, ldw,
-                                                                   gate_up != nullptr, stream);
+  auto start = tile_group != nullptr ? pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU, pico::pair::kRowGroups>
+                                     : pico::pair::start<256, 0, 0, pico::GEMM_OUT_SWIGLU>;
+  if (!rc) rc = start(plan, x, w, out, M, 2 * I, K, ldx, ldw, gate_up != nullptr, stream, groups, tile_group);
   return rc ? rc : pico::pair::launched();
 }
 
@@ -919,10 +960,8 @@ extern "C" int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* g
   pico::pair::OutMaps out = {};
   rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
   if (!rc) rc = pico::half_maps(&out.d_gate, &out.d_up, d_gate_up, M, I);
-  if (!rc)
-    rc = tile_group != nullptr
-             ? pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD, true>(plan, dy, w, out, M, I, K, lddy, ldw, 1,
-                                                                             stream, groups, tile_group)
-             : pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD>(plan, dy, w, out, M, I, K, lddy, ldw, 1, stream);
+  auto start = tile_group != nullptr ? pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD, pico::pair::kRowGroups>
+                                     : pico::pair::start<256, 0, 1, pico::GEMM_OUT_SWIGLU_BWD>;
+  if (!rc) rc = start(plan, dy, w, out, M, I, K, lddy, ldw, 1, stream, groups, tile_group);
   return rc ? rc : pico::pair::launched();
 }

@@ -1,8 +1,9 @@
 // Host paths in native code: autograd nodes of the single operators that programs call by themselves, and the whole
-// forward pass of a dense model where no gradient is recorded. The kernels are those of the Python operators, in the same
-// order; with small tensors the Python between them takes longer than they do. Measured, us, through Python / here:
-// forward of 4 layers of width 576 on 33 tokens 749 / 170 (153 of kernels; 329 with a tensor and its views per operator); forward and backward of attention, 256 tokens
-// x 9 heads, 105 / 88; of a linear of 1999 x 960 x 2560, 96 / 74.
+// forward pass of a dense model where no gradient is recorded. The kernels are those of the Python operators, in the
+// same order; with small tensors the Python between them takes longer than they do. Measured, us, through Python /
+// here: forward of 4 layers of width 576 on 33 tokens 749 / 170 (153 of kernels; 329 with a tensor and its views per
+// operator); forward and backward of attention, 256 tokens x 9 heads, 105 / 88; of a linear of 1999 x 960 x 2560, 96 /
+// 74.
 #include <ATen/core/grad_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -92,10 +93,10 @@ static void ok(int rc, const char* what) {
   TORCH_CHECK(rc == 0, what, " failed (", rc, "): ", pico_last_error());
 }
 
-// Logits [b, s, V] of a dense decoder without gradients; a layer is (norm, q | k | v, output projection, norm, gate | up,
-// down projection, the two norms' eps). Each residual add rides in the norm that follows it (the sum is rounded to bf16
-// there as a separate add would round it). The activations live in one allocation, of a layer's size and not of the
-// model's: what one layer is done with the next writes over, in stream order.
+// Logits [b, s, V] of a dense decoder without gradients; a layer is (norm, q | k | v, output projection, norm, gate |
+// up, down projection, the two norms' eps). Each residual add rides in the norm that follows it (the sum is rounded to
+// bf16 there as a separate add would round it). The activations live in one allocation, of a layer's size and not of
+// the model's: what one layer is done with the next writes over, in stream order.
 using LayerWeights = std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, at::Tensor, double, double>;
 
 static at::Tensor dense_forward(const at::Tensor& ids_, const at::Tensor& embedding,

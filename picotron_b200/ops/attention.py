@@ -98,8 +98,9 @@ def flash_attention_forward(q, k, v, causal, sm_scale=None, q_pos0: int = 0, k_p
 def flash_attention_backward(dout, q, k, v, out, lse, causal, sm_scale=None, q_pos0: int = 0, k_pos0: int = 0,
                              rope=None):
     """tcgen05 kernel: returns (dq, dk, dv) as column slices of one ``[b, s, (H + 2*Hkv)*d]`` buffer when
-    the sequence lengths match (so a fused QKV projection can consume them without a copy). ``rope``: (cos, sin, position
-    of the first token) of the rotary embedding that q and k carry; dq and dk are then those of the unrotated ones."""
+    the sequence lengths match (so a fused QKV projection can consume them without a copy). ``rope``: (cos, sin,
+    position of the first token) of the rotary embedding that q and k carry; dq and dk are then those of the
+    unrotated ones."""
     from . import count_launch, ext
     scale = sm_scale if sm_scale is not None else 1.0 / math.sqrt(q.shape[-1])
     grads = ext().attention_bwd_new(dout, q, k, v, out, lse, scale, causal, q_pos0, k_pos0, *(rope or ()))

@@ -119,7 +119,8 @@ def wgrad_into(weight: torch.Tensor, dy2: torch.Tensor, x2: torch.Tensor):
 
 
 class _LinearFn(torch.autograd.Function):
-    """The Python form of ``LinearNode`` (``csrc/native_calls.cpp``), for calls that something besides autograd watches."""
+    """The Python form of ``LinearNode`` (``csrc/native_calls.cpp``), for calls that something besides autograd
+    watches."""
 
     @staticmethod
     def forward(ctx, x, w):

@@ -190,13 +190,14 @@ class _GroupedMLPFn(torch.autograd.Function):
 
 
 def grouped_mlp(x: torch.Tensor, gate_ups, downs, layout: GroupLayout):
-    """The gated MLPs of all experts over the padded expert-major ``x`` in one op, or None where its kernels do not apply:
-    ``gate_ups`` are gate and up of each expert in turn, ``downs`` the down projections. Rows past the last segment of the
-    layout are not written."""
+    """The gated MLPs of all experts over the padded expert-major ``x`` in one op, or None where its kernels do not
+    apply: ``gate_ups`` are gate and up of each expert in turn, ``downs`` the down projections. Rows past the last
+    segment of the layout are not written."""
     from .gemm import WeightSet
     gu, down = WeightSet.of(gate_ups), WeightSet.of(downs)
     if gu.fused_main_grad is None or down.fused_main_grad is None or x.shape[0] == 0 or x.stride(-1) != 1 \
-            or (x.stride(0) * 2) % 16 or gu.fused_weight.dtype != x.dtype or not kernel_ok(x, x.shape[1], gu.splits[0]) \
+            or (x.stride(0) * 2) % 16 or gu.fused_weight.dtype != x.dtype \
+            or not kernel_ok(x, x.shape[1], gu.splits[0]) \
             or not ext().gemm_rows_on_pairs(x.shape[0], layout.num_groups):
         return None
     return _GroupedMLPFn.apply(x, gu.fused_weight, down.fused_weight, layout, gu.fused_main_grad, down.fused_main_grad,

@@ -17,8 +17,8 @@ def _close(got, want, mag, k):
                                                (300, 264, 520), (4200, 1160, 200)])
 @pytest.mark.parametrize("pitch", [0, 16])
 def test_products_with_swiglu(rows, inter, hidden, pitch):
-    """Less than a tile, half a pair, ragged rows and columns, a gate tile that reaches into the up rows, more tiles than
-    pairs; operands with a row pitch."""
+    """Less than a tile, half a pair, ragged rows and columns, a gate tile that reaches into the up rows, more tiles
+    than pairs; operands with a row pitch."""
     from picotron_b200 import ops
     torch.manual_seed(1)
     dev = dict(device="cuda")
@@ -41,7 +41,8 @@ def test_products_with_swiglu(rows, inter, hidden, pitch):
     dg, du = dgu.chunk(2, -1)
     # 1 + g (1 - sigmoid) cancels for g near -1.28: its terms are at most 1 + |g|, a few 2^-24 of the factors around it
     slack = 16 * 2.0 ** -24 * d.abs() * u.abs() * sg * (1 + g.abs())
-    err, bound = (dg.double() - d * dg_of).abs(), (d * dg_of).abs() * 2 ** -8 + mag * dg_of.abs() * (hidden + 2) * 2 ** -24
+    err = (dg.double() - d * dg_of).abs()
+    bound = (d * dg_of).abs() * 2 ** -8 + mag * dg_of.abs() * (hidden + 2) * 2 ** -24
     assert (err <= bound + slack + 1e-30).all()
     _close(du, d * du_of, mag * du_of.abs(), hidden)
 
@@ -49,8 +50,8 @@ def test_products_with_swiglu(rows, inter, hidden, pitch):
 @pytest.mark.parametrize("rows", [75, 2560])
 @pytest.mark.parametrize("keep_grad_of_x", [True, False])
 def test_mlp_module_takes_the_one_op_and_matches_the_separate_ones(keep_grad_of_x, rows):
-    """Few rows (products and a pass) and enough for the fused epilogues: gradients accumulate in main_grad; a hook on the
-    down projection selects the separate ops."""
+    """Few rows (products and a pass) and enough for the fused epilogues: gradients accumulate in main_grad; a hook on
+    the down projection selects the separate ops."""
     from types import SimpleNamespace
     from picotron_b200 import ops
     from picotron_b200.models.llama import MLP
@@ -112,10 +113,10 @@ def test_row_groups_on_pairs(counts, spare, inter, hidden):
     dgu = ops.ext().grouped_swiglu_bwd(dy, wd.view(-1, inter), gu, tg, G)
     plain = torch.full((P, 2 * inter), 7.0, device="cuda", dtype=torch.bfloat16)
     back = torch.full((P, inter), 7.0, device="cuda", dtype=torch.bfloat16)
-    ops.ext().gemm_grouped(x, wg.view(-1, hidden), plain, P, 2 * inter, hidden, hidden, hidden, 2 * inter, False, False, 0,
-                           0, tg, G, 2 * inter)
-    ops.ext().gemm_grouped(dy, wd.view(-1, inter), back, P, inter, hidden, hidden, inter, inter, False, True, 0, 0, tg, G,
-                           hidden)
+    ops.ext().gemm_grouped(x, wg.view(-1, hidden), plain, P, 2 * inter, hidden, hidden, hidden, 2 * inter, False, False,
+                           0, 0, tg, G, 2 * inter)
+    ops.ext().gemm_grouped(dy, wd.view(-1, inter), back, P, inter, hidden, hidden, inter, inter, False, True, 0, 0, tg,
+                           G, hidden)
     ops.check_status()
     assert (plain[group < 0] == 7).all() and (back[group < 0] == 7).all()
     for g, c in enumerate(counts):
@@ -166,7 +167,7 @@ def test_expert_layer_with_the_activation_inside_matches_the_separate_ops(monkey
         got.append((y.detach().clone(), x.grad.clone(), store.flat_grads.clone(), ops.launches() - before))
     ops.check_status()
     assert torch.equal(got[0][0], got[1][0]) and got[0][3] == got[1][3] - 2
-    # the separate path rounds the activation's gradient; then the roundings of gate | up's gradient, of the routed rows'
-    # and of their sum fall differently on the two sides: 2^-9 of the value each, three of them on either side
+    # the separate path rounds the activation's gradient; then the roundings of gate | up's gradient, of the routed
+    # rows' and of their sum fall differently on the two sides: 2^-9 of the value each, three of them on either side
     for a, b in zip(got[0][1:3], got[1][1:3]):
         assert (a.float() - b.float()).norm() <= (1 + 2 * 3) * 2 ** -9 * b.float().norm()

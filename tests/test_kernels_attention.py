@@ -277,8 +277,8 @@ def test_rotary_attention_gradients_against_64_bits(b, s, H, Hkv, d, offset):
                                                 (2, 513, 3, 1, 128, False), (1, 129, 2, 2, 128, True)])
 def test_key_blocks_shared_by_several_ctas(b, s, H, Hkv, d, causal):
     """Few key blocks: the steps of each are split, unevenly and, where a block has fewer than shares, with empty ones.
-    dK and dV are sums of the shares in order, the same bits on each run; 2-norm of bf16 roundings of P and dS (2^-9 each)
-    and of the results against 64 bits."""
+    dK and dV are sums of the shares in order, the same bits on each run; 2-norm of bf16 roundings of P and dS (2^-9
+    each) and of the results against 64 bits."""
     from picotron_b200 import ops
     from picotron_b200.ops import attention as A
     torch.manual_seed(s)

@@ -363,3 +363,33 @@ def test_products_summed_in_parts_of_k(M, N, K):
         assert ((out.double() - ref).abs() / scale).max().item() < 2 ** -8 + K / 16 * 4 * 2 ** -23
     assert wide[:, :8].abs().max().item() == 0
     assert torch.equal(gemm.gemm_nt(a, b), gemm.gemm_nt(a, b))
+
+
+@pytest.mark.parametrize("counts,M,N", [([64, 0, 192, 0] * 40, 128, 520), ([0, 640, 64] * 13, 384, 1000),
+                                        ([0, 0], 256, 38000), ([128] * 150, 128, 264), ([320, 64], 256, 38003),
+                                        ([64, 0, 192, 0], 128, 136)])
+def test_grouped_weight_gradients_on_pairs(counts, M, N):
+    """Blocks of half a pair tile, ragged columns, empty first and last groups, nothing but empty groups, four and more
+    rounds of tiles, and one shape of the one-CTA kernel. fp32 sums of exact products: 2^-24 per addition of the sum
+    of the magnitudes."""
+    ops, _ = _ops()
+    torch.manual_seed(11)
+    G, K = len(counts), max(sum(counts), 64)
+    starts = [0]
+    for c in counts:
+        starts.append(starts[-1] + c)
+    seg = torch.tensor(starts, device="cuda", dtype=torch.int32)
+    a = torch.randn(K, M, device="cuda").to(torch.bfloat16)
+    b = torch.randn(K, (N + 7) // 8 * 8, device="cuda").to(torch.bfloat16)[:, :N]
+    wide = torch.randn(G * M, (N + 3) // 4 * 4 + 4, device="cuda")
+    before, acc = wide.clone(), wide[:, :N]
+    base = acc.double()
+    ops.ext().gemm_grouped(a, b, acc, M, N, K, M, b.stride(0), acc.stride(0), True, True, 2, 1, seg, G, 0)
+    ops.check_status()
+    assert torch.equal(wide[:, N:], before[:, N:])
+    for g, c in enumerate(counts):
+        rows = slice(starts[g], starts[g + 1])
+        x, y = a[rows].double(), b[rows].double()
+        want = base[g * M:(g + 1) * M] + x.t() @ y
+        mag = base[g * M:(g + 1) * M].abs() + x.abs().t() @ y.abs()
+        assert ((acc[g * M:(g + 1) * M].double() - want).abs() <= mag * (c + 2) * 2.0 ** -24).all()

@@ -17,7 +17,8 @@ def test_linear_node_matches_the_python_function(kind, needs):
     from picotron_b200.ops import gemm
     torch.manual_seed(0)
     x = {"2d": lambda: _bf16(70, 64), "3d": lambda: _bf16(3, 35, 64), "transposed": lambda: _bf16(64, 72).t(),
-         "sliced": lambda: _bf16(5, 40, 76)[:, 1:38, 4:68], "one row": lambda: _bf16(1, 64)}[kind]().requires_grad_(needs[0])
+         "sliced": lambda: _bf16(5, 40, 76)[:, 1:38, 4:68], "one row": lambda: _bf16(1, 64)}[kind]()
+    x.requires_grad_(needs[0])
     w = _bf16(136, 64).requires_grad_(needs[1])
     dy = _bf16(136, *x.shape[:-1]).movedim(0, -1) if kind != "one row" else _bf16(1, 136)     # not contiguous
     wanted = [t for t in (x, w) if t.requires_grad]
