@@ -491,6 +491,13 @@ static int route_check(const char* what, int T, int E, int k) {
   return 0;
 }
 
+// A warp per row, the rows in order of memory (8192 tokens x 6, width 2048: gather 57.3 -> 54.4 us, gradient of the
+// weighted sum 106 -> 98; the sums, which jump about, gained nothing).
+static int row_grid(int64_t rows) {
+  const int64_t blocks = (rows + 7) / 8;
+  return (int)(blocks < 1 ? 1 : blocks < INT32_MAX ? blocks : INT32_MAX);
+}
+
 static int warp_grid(int64_t items) {
   int64_t blocks = (items + 7) / 8;       // 8 warps per CTA
   const int cap = pico_host::num_sms() * 8;
@@ -574,7 +581,7 @@ extern "C" int pico_moe_gather(const void* x, const int32_t* row_of_slot, const 
     return -2;
   }
   if (slots <= 0) return 0;
-  moe_gather_kernel<<<warp_grid(slots), 256, 0, stream>>>((const __nv_bfloat16*)x, row_of_slot, used,
+  moe_gather_kernel<<<row_grid(slots), 256, 0, stream>>>((const __nv_bfloat16*)x, row_of_slot, used,
                                                          (__nv_bfloat16*)out, slots, k, d);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) pico_host::set_error("moe_gather: %s", cudaGetErrorString(e));
@@ -607,7 +614,7 @@ extern "C" int pico_moe_combine_bwd(const void* dy, const void* out, const int32
     return -2;
   }
   if (slots <= 0) return 0;
-  moe_combine_bwd_kernel<<<warp_grid(slots), 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)out,
+  moe_combine_bwd_kernel<<<row_grid(slots), 256, 0, stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)out,
                                                               row_of_slot, w, used, (__nv_bfloat16*)dout, dw, slots,
                                                               k, d);
   cudaError_t e = cudaGetLastError();

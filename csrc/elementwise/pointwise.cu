@@ -32,6 +32,15 @@ static inline int grid_for(int64_t work_items, int threads) {
   return (int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
+// One item per thread, for kernels that stream several large buffers: the blocks go over them in order, so what is in
+// flight at a time lies close together in memory. With 16 blocks per SM that stride over the whole buffers they drift
+// apart: AdamW over 600 M parameters 2404 us (5.8 TB/s), in order 2148 (6.4), over 71 M 289, 266; SwiGLU backward 8192
+// x 8192 116, 105. Rotary, embedding, norm and attention passes gained nothing or lost up to 5 us.
+static inline int grid_in_order(int64_t work_items, int threads) {
+  const int64_t blocks = (work_items + threads - 1) / threads;
+  return (int)(blocks < INT32_MAX ? (blocks > 0 ? blocks : 1) : INT32_MAX);
+}
+
 static inline int finish(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) pico_host::set_error("%s: %s", what, cudaGetErrorString(e));
@@ -384,7 +393,9 @@ extern "C" int pico_swiglu_bwd(const void* dy, const void* gu, int64_t ld_gu, vo
     pico_host::set_error("swiglu: width and strides must be multiples of 8");
     return -2;
   }
-  pico_host::launch_ahead(swiglu_bwd_kernel, grid_for((int64_t)rows * (I / 8), 256), 256, 0, stream,
+  // a device-side row count may leave most blocks nothing to do
+  const auto grid = rows_dev ? grid_for : grid_in_order;
+  pico_host::launch_ahead(swiglu_bwd_kernel, grid((int64_t)rows * (I / 8), 256), 256, 0, stream,
                           (const __nv_bfloat16*)dy, (const __nv_bfloat16*)gu, ld_gu, (__nv_bfloat16*)dgu, ld_dgu,
                           rows, I, rows_dev);
   return finish("swiglu_bwd");
@@ -399,8 +410,8 @@ extern "C" int pico_adamw(void* p_bf16, float* master, float* g, float* m, float
     pico_host::set_error("adamw: need bf16 params or fp32 master params");
     return -2;
   }
-  pico_host::launch_ahead(adamw_kernel, grid_for(n / 4 + 1, 256), 256, 0, stream, (__nv_bfloat16*)p_bf16, master, g, m,
-                          v, n, lr, beta1, beta2, eps, weight_decay, bias_corr1, bias_corr2, grad_scale, zero_grad);
+  pico_host::launch_ahead(adamw_kernel, grid_in_order(n / 4 + 1, 256), 256, 0, stream, (__nv_bfloat16*)p_bf16, master,
+                          g, m, v, n, lr, beta1, beta2, eps, weight_decay, bias_corr1, bias_corr2, grad_scale, zero_grad);
   return finish("adamw");
 }
 
