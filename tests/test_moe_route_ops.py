@@ -408,3 +408,23 @@ def test_local_experts_layer_balances_like_the_tensor_path(renorm, aux, bias_rat
     for a, b in zip(got[0][0], got[1][0]):
         assert ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-6)).item() < 2 ** -6
     assert all(torch.equal(a, b) for a, b in zip(got[0][1], got[1][1])) and (got[0][1][-1].any().item() == (bias_rate > 0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("T,E,k", [(1, 8, 8), (700, 32, 8), (5000, 64, 8), (300, 65, 3), (300, 128, 8), (300, 129, 8)])
+def test_route_kernel_at_the_edges_of_its_lanes(T, E, k):
+    """One, two, four and eight experts per lane at their limits, more tokens than warps: the choice and the counts are
+    exact (distinct logits), probabilities and weights fp32 (1e-6)."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import moe_route as mr
+    g = torch.Generator().manual_seed(E)
+    logits = torch.stack([torch.randperm(E, generator=g) for _ in range(T)]).float().div(16).to(torch.bfloat16).cuda()
+    probs, idx, w, counts = mr.route(logits, None, k, True)
+    ops.check_status()
+    want = torch.softmax(logits.double(), -1)
+    chosen = torch.sort(logits.float(), dim=-1, descending=True, stable=True).indices[:, :k]
+    ww = want.gather(1, chosen)
+    if k > 1:
+        ww = ww / ww.sum(-1, keepdim=True)
+    assert torch.equal(idx.long(), chosen) and torch.equal(counts.long(), torch.bincount(chosen.flatten(), minlength=E))
+    assert torch.allclose(probs.double(), want, atol=1e-6) and torch.allclose(w.double(), ww, atol=1e-6)
