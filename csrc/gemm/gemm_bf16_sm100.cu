@@ -614,13 +614,6 @@ GemmPlan plan_gemm(int sms, int M, int N, int K, int a_mn, int b_mn, int out_mod
     best_cost = wide;
     best.bn = 256;
   }
-  // One round of 128 x 64 tiles: a K block costs no more than one of 128 x 128 (latency and the way from L2 set it, not
-  // the tensor cores) and the epilogue is half. 128 / 64 wide, us: 33 x 576 x 1536 7.6 / 7.3, its input gradient 8.4 /
-  // 7.2, 960 x 960 += of 512 rows 6.3 / 5.3, of 4096 21.7 / 18.9.
-  if (tiles(128, 64) <= sms && (double)kb * 256 * 1.3 + 1000 < best_cost) {
-    best_cost = (double)kb * 256 * 1.3 + 1000;
-    best.bn = 64;
-  }
   const int64_t t = tiles(2 * BM, 256);
   if (sms >= 2 && M > BM && N > 128 && gemm_pair_has(a_mn, b_mn, out_mode) && t < INT32_MAX) {
     const int64_t pairs = sms / 2, rest = t % pairs;

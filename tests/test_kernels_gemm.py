@@ -393,24 +393,3 @@ def test_grouped_weight_gradients_on_pairs(counts, M, N):
         want = base[g * M:(g + 1) * M] + x.t() @ y
         mag = base[g * M:(g + 1) * M].abs() + x.abs().t() @ y.abs()
         assert ((acc[g * M:(g + 1) * M].double() - want).abs() <= mag * (c + 2) * 2.0 ** -24).all()
-
-
-@pytest.mark.parametrize("M,N,K", [(33, 576, 576), (1, 72, 8), (129, 136, 200), (500, 1000, 1536), (1016, 1152, 72)])
-def test_one_round_of_narrow_tiles(M, N, K):
-    """Products of few tiles run 64 columns wide: last tiles of 8 columns, single rows, all layouts, against 64 bits.
-    fp32 sums: 2^-24 of the magnitudes per addition; bf16 results are rounded once."""
-    ops, gemm = _ops()
-    for mode, a_mn, b_mn in ((0, False, False), (0, False, True), (0, True, True), (2, True, True)):
-        assert ops.ext().gemm_plan(148, M, N, K, a_mn, b_mn, mode, 0)[:2] == [0, 64]
-    torch.manual_seed(M + N + K)
-    a, b = torch.randn(M, K, device="cuda").to(torch.bfloat16), torch.randn(N, K, device="cuda").to(torch.bfloat16)
-    want, mag = a.double() @ b.double().t(), a.double().abs() @ b.double().abs().t()
-    at, bt = torch.zeros(K, (M + 7) // 8 * 8, device="cuda", dtype=torch.bfloat16)[:, :M], b.t().contiguous()
-    at.copy_(a.t())
-    acc = torch.randn(M, N, device="cuda")
-    base = acc.double()
-    for out in (gemm.gemm_nt(a, b), gemm.gemm_nn(a, bt), gemm.gemm_tn(at, bt)):
-        assert ((out.double() - want).abs() <= want.abs() * 2 ** -8 + mag * (K + 2) * 2.0 ** -24).all()
-    gemm.gemm_tn(at, bt, out=acc, accumulate=True)
-    ops.check_status()
-    assert ((acc.double() - base - want).abs() <= (mag + base.abs()) * (K + 3) * 2.0 ** -24).all()
