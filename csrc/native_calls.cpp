@@ -47,6 +47,7 @@ struct LinearNode : torch::autograd::Function<LinearNode> {
     g_launches += launches;
     ctx->save_for_backward({x2, w});
     ctx->saved_data["shape"] = x.sizes().vec();
+    ctx->saved_data["w_learns"] = w.requires_grad();
     return y;
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
@@ -59,7 +60,9 @@ struct LinearNode : torch::autograd::Function<LinearNode> {
       g_launches += launches;
       dx = d.view(ctx->saved_data["shape"].toIntVector());
     }
-    if (ctx->needs_input_grad(1) && !python_wgrad(w, dy2, x2, dw)) {
+    // needs_input_grad is about this backward, w_learns about the weight: a backward for x alone still accumulates into
+    // main_grad or postpones, as the Python function (and those of the other projections) does
+    if (ctx->saved_data["w_learns"].toBool() && !python_wgrad(w, dy2, x2, dw) && ctx->needs_input_grad(1)) {
       const int64_t K = dy2.size(0), M = dy2.size(1), N = x2.size(1);
       dw = at::empty({M, N}, dy2.options());
       g_launches += gemm(dy2, x2, dw, M, N, K, dy2.stride(0), x2.stride(0), N, true, true, 0, 0);

@@ -1,5 +1,7 @@
 """Native autograd nodes and the native forward pass give what the Python operators and modules give, bit for bit, and
 leave to those what something else watches."""
+import contextlib
+
 import pytest
 import torch
 
@@ -53,6 +55,38 @@ def test_linear_node_leaves_main_grad_and_postponed_gradients_to_python():
     want = dy.double().t() @ x.detach().double()
     assert (w.main_grad.double() - want).norm() <= 1e-5 * want.norm()
     assert (late.double() - want).norm() <= 2 ** -8 * want.norm()
+
+
+def _main_grad(w):
+    w.main_grad = torch.zeros(w.shape, device="cuda")
+    w.calls = []
+    w.grad_ready_hook = lambda: w.calls.append(1)
+    return w.main_grad
+
+
+@pytest.mark.parametrize("how", ["grad", "backward"])
+@pytest.mark.parametrize("where", ["main_grad", "queue"])
+@pytest.mark.parametrize("learns", [True, False])
+def test_a_backward_for_the_input_alone_keeps_the_weight_gradient(how, where, learns):
+    """The weight's gradient goes into main_grad, or into the queue, whether or not this backward asks for it, as long as
+    the weight learns: as with the Python function."""
+    from picotron_b200.ops import gemm
+    torch.manual_seed(4)
+    x, dy = _bf16(40, 64).requires_grad_(), _bf16(40, 72)
+    w = torch.nn.Parameter(_bf16(72, 64), requires_grad=learns)
+    results = []
+    for call in (gemm.linear, gemm._LinearFn.apply):
+        buf = _main_grad(w)
+        x.grad = None
+        with contextlib.ExitStack() as stack:
+            queue = stack.enter_context(gemm.defer_wgrad()) if where == "queue" else []
+            y = call(x, w)
+            dx = torch.autograd.grad(y, x, dy)[0] if how == "grad" else y.backward(dy, inputs=[x]) or x.grad
+        assert len(queue) == int(learns and where == "queue")
+        gemm.run_deferred(queue)
+        assert len(w.calls) == int(learns) and bool(buf.any()) == learns and w.grad is None
+        results.append((dx, buf))
+    assert all(torch.equal(a, b) for a, b in zip(*results))
 
 
 @pytest.mark.parametrize("b,s,H,Hkv,d,causal", [(1, 33, 3, 1, 64, False), (2, 130, 4, 4, 128, True)])
