@@ -322,8 +322,8 @@ class DecoderLayer(nn.Module):
         self.ptb_overlap = fused_ptb and overlap
 
     def native_weights(self, hidden: int):
-        """((weights and eps of this layer), (heads, kv heads, head_dim)) for ``dense_forward``, or None (see
-        ``Llama._native_layers``)."""
+        """((weights and eps of this layer), (heads, kv heads, head_dim, width of the MLP)) for ``dense_forward``, which
+        takes one such shape for all layers, or None (see ``Llama._native_layers``)."""
         if self.parallel_block:
             return None
         # straight from the dicts: attribute access by name costs the host more than the rest of this
@@ -353,7 +353,8 @@ class DecoderLayer(nn.Module):
                 or w_down.shape != (hidden, inter) or not w_out.is_contiguous() or not w_down.is_contiguous() \
                 or not gemm_ops._gemm_ok(hidden, width, inter):
             return None
-        return ((w1, qkv.weight, w_out, w2, gate_up.weight, w_down, n1.eps, n2.eps), (heads, kv_heads, attn.head_dim))
+        return ((w1, qkv.weight, w_out, w2, gate_up.weight, w_down, n1.eps, n2.eps),
+                (heads, kv_heads, attn.head_dim, inter))
 
     def forward(self, x, rope):
         if self.parallel_block:
@@ -450,8 +451,8 @@ class Llama(nn.Module):
 
     def _native_layers(self, input_ids):
         """What ``dense_forward`` (``csrc/native_calls.cpp``) needs of the layers, or None where the pass has to go
-        through the modules: sharded, expert or parallel-block layers, weights that are not stored side by side, types
-        and sizes off the kernels, or anyone watching a module's call."""
+        through the modules: sharded, expert or parallel-block layers, layers of different shapes, weights that are not
+        stored side by side, types and sizes off the kernels, or anyone watching a module's call."""
         emb, head = self.embedding, self.final_proj
         if not (type(emb) is Embedding and type(head) is FinalProjection and type(self.final_norm) is RMSNorm
                 and input_ids.is_cuda and input_ids.dim() == 2 and input_ids.dtype == torch.int64
@@ -475,7 +476,7 @@ class Llama(nn.Module):
     def forward(self, input_ids, position_ids=None, hidden_states=None):
         native = self._native_layers(input_ids) if untracked() else None
         if native is not None:
-            layers, (heads, kv_heads, head_dim) = native
+            layers, (heads, kv_heads, head_dim, _) = native
             w = self.embedding.weight
             _, _, (cos, sin) = self.rope.tables(w.device, w.dtype)
             return ext().dense_forward(input_ids, w, layers, self.final_norm.weight, self.final_norm.eps,

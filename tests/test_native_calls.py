@@ -138,16 +138,20 @@ def test_watched_calls_take_the_python_functions():
         assert "_LinearFn" in y.grad_fn.name()
 
 
-def _model(name, layers, seq):
+def _model(name, layers, seq, widths=None):
+    """``widths``: those of the layers' MLPs, where they differ."""
     from picotron_b200.config import MODEL_SHAPES
-    from picotron_b200.models.llama import Llama
+    from picotron_b200.models.llama import MLP, Llama
     from picotron_b200.param_store import ParamStore
     from types import SimpleNamespace
     shape = dict(MODEL_SHAPES["HuggingFaceTB/SmolLM-135M"], num_hidden_layers=layers, max_position_embeddings=seq,
                  init_std=0.05, **name)
     torch.manual_seed(3)
+    config = SimpleNamespace(**shape)
     with torch.device("cuda"):
-        model = Llama(SimpleNamespace(**shape))
+        model = Llama(config)
+        for layer, width in zip(model.decoder_layers, widths or ()):
+            layer.mlp = MLP(config, width)
     model.reset_parameters()
     model = model.to(torch.bfloat16)
     return model, ParamStore(model)
@@ -190,6 +194,7 @@ def test_native_forward_is_left_where_it_does_not_apply():
     loose, _ = _model({}, 1, 32)
     for m in loose.modules():                                    # weights that are not stored side by side
         m.__dict__.pop("_fused_group", None)
+    uneven, _ = _model({}, 2, 32, widths=(1536, 768))
     with torch.no_grad():
-        assert parallel._native_layers(ids) is None and loose._native_layers(ids) is None
-        assert parallel(ids).shape == loose(ids).shape == (1, 20, 49152)
+        for other in (parallel, loose, uneven):
+            assert other._native_layers(ids) is None and other(ids).shape == (1, 20, 49152)
