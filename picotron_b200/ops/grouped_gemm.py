@@ -111,6 +111,14 @@ def grouped_gemm_tn(dy, x, layout: GroupLayout, out: torch.Tensor, accumulate: b
     return out
 
 
+def _grads_ready(params) -> None:
+    """``params`` have their whole gradient of this backward pass in ``main_grad``."""
+    for p in params:
+        hook = getattr(p, "grad_ready_hook", None)
+        if hook is not None:
+            hook()
+
+
 class _GroupedLinearFn(torch.autograd.Function):
     """``w`` is the stacked ``[G * out_rows, in]`` weight block. When it is the fused view of
     parameters that carry ``main_grad`` buffers, the weight gradient accumulates there and autograd
@@ -132,10 +140,7 @@ class _GroupedLinearFn(torch.autograd.Function):
             dx = grouped_gemm_nn(dy, w, layout, out_rows)
         if ctx.main_grad is not None:
             grouped_gemm_tn(dy, x, layout, ctx.main_grad, accumulate=True)
-            for p in ctx.params:
-                hook = getattr(p, "grad_ready_hook", None)
-                if hook is not None:
-                    hook()
+            _grads_ready(ctx.params)
             return (dx, None, None, None, None) + (None,) * len(ctx.params)
         pgrads = (None,) * len(ctx.params)
         if ctx.needs_input_grad[1] or any(ctx.needs_input_grad[5:]):
@@ -162,14 +167,15 @@ def grouped_linear(x: torch.Tensor, mods, layout: GroupLayout, out_rows: int) ->
 
 class _GroupedMLPFn(torch.autograd.Function):
     """``down(silu(gate(x)) * up(x))`` of every expert with the activation inside the grouped products (see
-    ``gated_mlp``). ``w_gu`` and ``w_down`` are fused views of parameters that carry ``main_grad`` buffers."""
+    ``gated_mlp``). ``w_gu`` and ``w_down`` are fused views of parameters that carry ``main_grad`` buffers; ``params``
+    are those of the gate and up projections, then those of the down projections."""
 
     @staticmethod
-    def forward(ctx, x, w_gu, w_down, layout, grad_gu, grad_down, *params):
+    def forward(ctx, x, w_gu, w_down, layout, grad_gu, grad_down, num_gu, *params):
         gate_up, act = ext().grouped_swiglu(x, w_gu, layout.tile_group, layout.num_groups)
         count_launch()
         ctx.save_for_backward(x, w_gu, w_down, gate_up, act)
-        ctx.layout, ctx.grads, ctx.params = layout, (grad_gu, grad_down), params
+        ctx.layout, ctx.grads, ctx.params = layout, (grad_gu, grad_down), (params[:num_gu], params[num_gu:])
         return grouped_gemm_nt(act, w_down, layout, w_down.shape[0] // layout.num_groups)
 
     @staticmethod
@@ -180,13 +186,11 @@ class _GroupedMLPFn(torch.autograd.Function):
         d_gate_up = ext().grouped_swiglu_bwd(dy, w_down, gate_up, layout.tile_group, layout.num_groups)
         count_launch()
         grouped_gemm_tn(dy, act, layout, grad_down, accumulate=True)
+        _grads_ready(ctx.params[1])      # a reduction that this starts has the products below to hide behind
         dx = grouped_gemm_nn(d_gate_up, w_gu, layout, gate_up.shape[1]) if ctx.needs_input_grad[0] else None
         grouped_gemm_tn(d_gate_up, x, layout, grad_gu, accumulate=True)
-        for p in ctx.params:
-            hook = getattr(p, "grad_ready_hook", None)
-            if hook is not None:
-                hook()
-        return (dx, None, None, None, None, None) + (None,) * len(ctx.params)
+        _grads_ready(ctx.params[0])
+        return (dx,) + (None,) * (len(ctx.needs_input_grad) - 1)
 
 
 def grouped_mlp(x: torch.Tensor, gate_ups, downs, layout: GroupLayout):
@@ -201,7 +205,7 @@ def grouped_mlp(x: torch.Tensor, gate_ups, downs, layout: GroupLayout):
             or not ext().gemm_rows_on_pairs(x.shape[0], layout.num_groups):
         return None
     return _GroupedMLPFn.apply(x, gu.fused_weight, down.fused_weight, layout, gu.fused_main_grad, down.fused_main_grad,
-                               *gu.params, *down.params)
+                               len(gu.params), *gu.params, *down.params)
 
 
 def grouped_linear_ref(x, weights: List[torch.Tensor], layout: GroupLayout):

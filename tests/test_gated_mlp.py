@@ -171,3 +171,50 @@ def test_expert_layer_with_the_activation_inside_matches_the_separate_ops(monkey
     # rows' and of their sum fall differently on the two sides: 2^-9 of the value each, three of them on either side
     for a, b in zip(got[0][1:3], got[1][1:3]):
         assert (a.float() - b.float()).norm() <= (1 + 2 * 3) * 2 ** -9 * b.float().norm()
+
+
+def _expert_layer():
+    from types import SimpleNamespace
+    from picotron_b200 import process_group_manager as pgm
+    from picotron_b200.param_store import ParamStore
+    from picotron_b200.parallel.expert_parallel import MoELayer
+    if pgm.process_group_manager is None:
+        pgm.setup_process_group_manager(1, 1, 1, 1, 1)
+    cfg = SimpleNamespace(hidden_size=256, intermediate_size=192, num_experts=4, num_experts_per_tok=2, init_std=0.05)
+    with torch.device("cuda"):
+        layer = MoELayer(cfg).to(torch.bfloat16)
+    layer.train()
+    return layer, ParamStore(layer)
+
+
+def _nodes(fn, seen=None):
+    """Names of all nodes of a graph."""
+    seen = {} if seen is None else seen
+    if fn is not None and fn not in seen:
+        seen[fn] = fn.name()
+        for nxt, _ in fn.next_functions:
+            _nodes(nxt, seen)
+    return " ".join(seen.values())
+
+
+def test_down_projections_of_experts_are_ready_before_the_products_of_gate_and_up(monkeypatch):
+    """A data-parallel reduction that a down projection's hook starts runs beside the rest of the backward pass: its
+    hooks come before the input gradient and the weight gradient of gate and up, as with the separate operators."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import grouped_gemm
+    torch.manual_seed(6)
+    layer, store = _expert_layer()
+    x = torch.randn(1, 1500, 256, device="cuda").to(torch.bfloat16).requires_grad_()
+    events = []
+    for name, p in layer.named_parameters():
+        p.grad_ready_hook = lambda kind=name.split(".")[-2]: events.append(kind)
+    for name in ("grouped_gemm_nn", "grouped_gemm_tn"):
+        plain = getattr(grouped_gemm, name)
+        monkeypatch.setattr(grouped_gemm, name, lambda *a, _f=plain, _n=name, **k: (events.append(_n), _f(*a, **k))[1])
+    y = layer(x)
+    assert "GroupedMLP" in _nodes(y.grad_fn)
+    y.backward(torch.randn_like(y))
+    ops.check_status()
+    events = [e for e in events if e != "gate"]                   # the router's
+    assert events[:1] + events[5:7] == ["grouped_gemm_tn", "grouped_gemm_nn", "grouped_gemm_tn"]
+    assert events[1:5] == ["down_proj"] * 4 and sorted(events[7:]) == ["gate_proj"] * 4 + ["up_proj"] * 4
