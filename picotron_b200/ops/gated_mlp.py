@@ -50,9 +50,14 @@ class _GatedMLPFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, gate_up, act, w_down = ctx.saved_tensors
         dy2 = gemm._as_2d(dy)
-        d_gate_up, n = ext().gemm_swiglu_bwd(dy2, w_down, gate_up)
-        count_launch(n)
+        # frozen gate and up of an input without gradient are not part of the graph of the separate operators
+        gate_up_learns = ctx.needs_input_grad[0] or any(ctx.needs_input_grad[3:])
+        if gate_up_learns:
+            d_gate_up, n = ext().gemm_swiglu_bwd(dy2, w_down, gate_up)
+            count_launch(n)
         dw = gemm.wgrad_into(w_down, dy2, act) if ctx.needs_input_grad[2] else None
+        if not gate_up_learns:
+            return (None, None, dw) + (None,) * (len(ctx.needs_input_grad) - 3)
         dx, grads = gemm.backward_all(d_gate_up, x2, ctx.ws, need_dx=ctx.needs_input_grad[0])
         return (dx.view(ctx.x_shape) if dx is not None else None, None, dw, *grads)
 

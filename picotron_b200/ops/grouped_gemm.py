@@ -183,10 +183,15 @@ class _GroupedMLPFn(torch.autograd.Function):
         x, w_gu, w_down, gate_up, act = ctx.saved_tensors
         layout, (grad_gu, grad_down) = ctx.layout, ctx.grads
         dy = dy.contiguous()
-        d_gate_up = ext().grouped_swiglu_bwd(dy, w_down, gate_up, layout.tile_group, layout.num_groups)
-        count_launch()
+        # frozen gate and up of an input without gradient are not part of the graph of the separate operators
+        gate_up_learns = ctx.needs_input_grad[0] or any(ctx.needs_input_grad[7:7 + len(ctx.params[0])])
+        if gate_up_learns:
+            d_gate_up = ext().grouped_swiglu_bwd(dy, w_down, gate_up, layout.tile_group, layout.num_groups)
+            count_launch()
         grouped_gemm_tn(dy, act, layout, grad_down, accumulate=True)
         _grads_ready(ctx.params[1])      # a reduction that this starts has the products below to hide behind
+        if not gate_up_learns:
+            return (None,) * len(ctx.needs_input_grad)
         dx = grouped_gemm_nn(d_gate_up, w_gu, layout, gate_up.shape[1]) if ctx.needs_input_grad[0] else None
         grouped_gemm_tn(d_gate_up, x, layout, grad_gu, accumulate=True)
         _grads_ready(ctx.params[0])

@@ -218,3 +218,41 @@ def test_down_projections_of_experts_are_ready_before_the_products_of_gate_and_u
     events = [e for e in events if e != "gate"]                   # the router's
     assert events[:1] + events[5:7] == ["grouped_gemm_tn", "grouped_gemm_nn", "grouped_gemm_tn"]
     assert events[1:5] == ["down_proj"] * 4 and sorted(events[7:]) == ["gate_proj"] * 4 + ["up_proj"] * 4
+
+
+@pytest.mark.parametrize("grouped", [False, True])
+@pytest.mark.parametrize("learns", ["down", "up and down", "input"])
+def test_gate_and_up_that_no_gradient_reaches_get_none(grouped, learns):
+    """Frozen gate and up projections of an input that needs no gradient stay out of the backward pass, as with the
+    separate operators: nothing is added to their main_grad and their hooks stay silent."""
+    from types import SimpleNamespace
+    from picotron_b200 import ops
+    from picotron_b200.models.llama import MLP
+    from picotron_b200.ops import grouped_gemm
+    from picotron_b200.param_store import ParamStore
+    torch.manual_seed(7)
+    if grouped:
+        layer, store = _expert_layer()
+        experts = list(layer.local_experts)
+        layout = grouped_gemm.GroupLayout.uniform(4, 1024, "cuda")
+        x = torch.randn(4096, 256, device="cuda").to(torch.bfloat16)
+    else:
+        with torch.device("cuda"):
+            layer = MLP(SimpleNamespace(hidden_size=256, intermediate_size=192, init_std=0.05)).to(torch.bfloat16)
+        store, experts = ParamStore(layer), [layer]
+        x = torch.randn(300, 256, device="cuda").to(torch.bfloat16)
+    gate_up = [m for e in experts for m in (e.gate_proj, e.up_proj)]
+    downs = [e.down_proj for e in experts]
+    called = set()
+    for m in gate_up + downs:
+        m.weight.grad_ready_hook = lambda m=m: called.add(m)
+    for m in gate_up:
+        m.weight.requires_grad_(learns == "up and down" and any(m is e.up_proj for e in experts))
+    x.requires_grad_(learns == "input")
+    y = grouped_gemm.grouped_mlp(x, gate_up, downs, layout) if grouped else layer(x)
+    assert "MLPFn" in y.grad_fn.name()
+    y.backward(torch.randn_like(y))
+    ops.check_status()
+    assert all(m.weight.main_grad.any() for m in downs) and called >= set(downs)
+    reached = learns != "down"            # one product accumulates for both of the pair
+    assert all(bool(m.weight.main_grad.any()) == reached and (m in called) == reached for m in gate_up)
