@@ -374,13 +374,13 @@ __global__ void __launch_bounds__(256)
 moe_gather_kernel(const __nv_bfloat16* __restrict__ x, const int32_t* __restrict__ row_of_slot,
                   const int32_t* __restrict__ used, __nv_bfloat16* __restrict__ out, int slots, int k, int d) {
   const int lane = threadIdx.x & 31;
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;   // row_grid: up to 2^28 blocks
+  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int nvec = d / 8;
   const int n = min(slots, *used);
-  for (int s = warp; s < n; s += nwarps) {
+  for (int64_t s = warp; s < n; s += nwarps) {
     const int row = row_of_slot[s];
-    uint4* dst = reinterpret_cast<uint4*>(out + (int64_t)s * d);
+    uint4* dst = reinterpret_cast<uint4*>(out + s * d);
     if (row < 0) {
       for (int v = lane; v < nvec; v += 32) dst[v] = make_uint4(0, 0, 0, 0);
       continue;

@@ -294,6 +294,23 @@ def test_layout_reports_rows_that_it_cannot_place():
 
 
 @pytest.mark.gpu
+def test_gather_of_more_rows_than_32_bits_count_threads_for():
+    """A warp per row from 2^27 rows on: 2^32 threads and more."""
+    from picotron_b200 import ops
+    n, d, k = 2 ** 27 + 5, 8, 2
+    x = torch.randn(1024, d, device="cuda").to(torch.bfloat16)
+    row = torch.arange(n, device="cuda", dtype=torch.int32) % (1024 * k)
+    row[::1000] = -1
+    out = torch.empty(n, d, device="cuda", dtype=torch.bfloat16)
+    ops.ext().moe_gather(x, row, torch.tensor([n], device="cuda", dtype=torch.int32), out, k)
+    ops.check_status()
+    for lo in range(0, n, 2 ** 24):
+        r = row[lo:lo + 2 ** 24]
+        want = x[r.clamp(min=0).long() // k].masked_fill((r < 0)[:, None], 0)
+        assert torch.equal(out[lo:lo + 2 ** 24], want)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("E,k", [(8, 2), (64, 6)])
 def test_tokens_that_are_not_finite_stay_among_themselves(E, k):
     """A diverging token through the whole layer: NaN in its own outputs and input gradient, the others as without it."""
