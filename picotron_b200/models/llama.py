@@ -190,10 +190,20 @@ class Attention(nn.Module):
         return self.out_proj(out)
 
 
+#: (class, method) -> the function that this file defines there, for the methods whose work ``MLP._one_op`` and
+#: ``Llama._native_layers`` take over (filled below the classes); one that a program replaces has to be called
+_WRITTEN: dict = {}
+_METHODS = {"forward", "hidden", "_fused_local"}
+
+
+def as_written(cls, base, method: str) -> bool:
+    return getattr(cls, method) is _WRITTEN[base, method]
+
+
 def own_hooks(mod: nn.Module) -> bool:
-    """Whether a call of ``mod`` does more than its class's forward pass: hooks on it, a patched forward."""
+    """Whether a call of ``mod`` does more than its class's forward pass: hooks on it, methods replaced on it."""
     return bool(mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks
-                or "forward" in mod.__dict__)
+                or not _METHODS.isdisjoint(mod.__dict__))
 
 
 def hooked(mod: nn.Module) -> bool:
@@ -223,9 +233,12 @@ class MLP(nn.Module):
 
     def _one_op(self, x):
         """The weights of ``ops.gated_mlp`` when the whole MLP can run as that op: unsharded linears (no collective
-        between them) and nobody watching the calls of the down projection, which it does not make."""
+        between them), and nobody watching or replacing the calls of the down projection and of ``hidden``, which it
+        does not make."""
         down = self.down_proj
-        if not (type(self.gate_proj) is type(self.up_proj) is type(down) is Linear) or hooked(down):
+        if not (type(self.gate_proj) is type(self.up_proj) is type(down) is Linear) or hooked(down) \
+                or "hidden" in self.__dict__ or not as_written(type(self), MLP, "hidden") \
+                or not as_written(Linear, Linear, "forward"):
             return None
         ws = gemm_ops.WeightSet.of([self.gate_proj, self.up_proj])
         return ws if gated_mlp_ops.fits(x, ws, down.weight) else None
@@ -452,12 +465,13 @@ class Llama(nn.Module):
     def _native_layers(self, input_ids):
         """What ``dense_forward`` (``csrc/native_calls.cpp``) needs of the layers, or None where the pass has to go
         through the modules: sharded, expert or parallel-block layers, layers of different shapes, weights that are not
-        stored side by side, types and sizes off the kernels, or anyone watching a module's call."""
+        stored side by side, types and sizes off the kernels, or anyone watching or replacing a module's call."""
         emb, head = self.embedding, self.final_proj
         if not (type(emb) is Embedding and type(head) is FinalProjection and type(self.final_norm) is RMSNorm
                 and input_ids.is_cuda and input_ids.dim() == 2 and input_ids.dtype == torch.int64
                 and input_ids.numel() > 0 and use_kernels(emb.weight, head.weight)
                 and not torch.nn.modules.module._has_any_global_hook()
+                and all(getattr(cls, method) is fn for (cls, method), fn in _WRITTEN.items())
                 and not any(own_hooks(m) for m in (emb, self.final_norm, head))):
             return None
         hidden = emb.weight.shape[1]
@@ -486,3 +500,8 @@ class Llama(nn.Module):
         for layer in self.decoder_layers_iter():
             x = layer(x, self.rope)
         return lm_head(self, x)
+
+
+_WRITTEN.update({(cls, method): getattr(cls, method)
+                 for cls in (Embedding, RMSNorm, Linear, FinalProjection, Attention, MLP, DecoderLayer)
+                 for method in sorted(_METHODS) if hasattr(cls, method)})

@@ -198,3 +198,48 @@ def test_native_forward_is_left_where_it_does_not_apply():
     with torch.no_grad():
         for other in (parallel, loose, uneven):
             assert other._native_layers(ids) is None and other(ids).shape == (1, 20, 49152)
+
+
+@pytest.mark.parametrize("where", ["instance", "class"])
+@pytest.mark.parametrize("owner,method", [("MLP", "hidden"), ("MLP", "forward"), ("Linear", "forward"),
+                                          ("Attention", "_fused_local"), ("RMSNorm", "forward"),
+                                          ("DecoderLayer", "forward")])
+def test_replaced_methods_are_called(monkeypatch, where, owner, method):
+    """A program that replaces a method of a module or of its class sees it called, with gradients and without."""
+    from picotron_b200.models import llama
+    model, _ = _model({}, 2, 32)
+    ids = torch.randint(0, 49152, (1, 20), device="cuda")
+    cls, layer = getattr(llama, owner), model.decoder_layers[1]
+    mod = {"MLP": layer.mlp, "Linear": layer.mlp.down_proj, "Attention": layer.attention,
+           "RMSNorm": layer.post_attention_layernorm, "DecoderLayer": layer}[owner]
+    plain, seen = getattr(cls, method), []
+
+    def instead(self, *a, **k):
+        seen.append(self)
+        return plain(self, *a, **k)
+    if where == "class":
+        monkeypatch.setattr(cls, method, instead)
+    else:
+        setattr(mod, method, lambda *a, **k: instead(mod, *a, **k))
+    for grad in (True, False):
+        seen.clear()
+        with torch.set_grad_enabled(grad):
+            model(ids)
+        assert any(m is mod for m in seen)
+
+
+def test_subclass_of_the_mlp_keeps_its_own_hidden():
+    from types import SimpleNamespace
+    from picotron_b200.models.llama import MLP
+    from picotron_b200.param_store import ParamStore
+
+    class Doubled(MLP):
+        def hidden(self, x):
+            return 2 * super().hidden(x)
+    torch.manual_seed(5)
+    with torch.device("cuda"):
+        mlp = Doubled(SimpleNamespace(hidden_size=64, intermediate_size=128, init_std=0.05)).to(torch.bfloat16)
+    ParamStore(mlp)
+    x = _bf16(20, 64)
+    y, want = mlp(x), torch.nn.functional.linear(mlp.hidden(x), mlp.down_proj.weight)
+    assert (y.float() - want.float()).norm() <= 2 ** -7 * want.float().norm()
