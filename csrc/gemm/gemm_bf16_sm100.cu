@@ -654,7 +654,20 @@ sum_parts_kernel(const float* __restrict__ slabs, __nv_bfloat16* __restrict__ D,
   }
 }
 
+// Tile width of the one-CTA kernel's grouped and collective forms.
+static int one_cta_bn(int sms, int M, int N) {
+  if (N <= 64) return 64;
+  // no more 128 x 128 tiles than SMs: one wave either way
+  return N <= 128 || ((N + 127) / 128) * ((M + 127) / 128) <= sms ? 128 : 256;
+}
+
 }  // namespace pico
+
+extern "C" int pico_gemm_rows_plan(int sms, int M, int N, int K, int groups) {
+  if (M <= 0 || N <= 128 || K <= 0 || !pico::gemm_pair_takes_rows(M, groups)) return 0;
+  if (sms <= 0) sms = pico_host::num_sms();
+  return pico::gemm_pair_rows_pay(sms, M, N, K, pico::one_cta_bn(sms, M, N));
+}
 
 // Few 128 x 128 tiles and a long reduction, as in the input gradient of the vocabulary projection for a short
 // micro-batch (128 tokens, hidden 576, vocabulary 49152: 5 tiles; ~250 us whole, 13 us in parts). The whole form takes
@@ -703,14 +716,12 @@ static int run_gemm(const void* A, const void* B, void* D, int M, int N, int K, 
   if (comm == nullptr)
     plan = pico::plan_gemm(pico_host::num_sms(), M, N, K, a_mn_major, b_mn_major, out_mode, max_ctas,
                            scratch != nullptr);
-  else if (N <= 64)
-    plan.bn = 64;
-  else if (N <= 128 || ((N + 127) / 128) * ((M + 127) / 128) <= pico_host::num_sms())
-    plan.bn = 128;   // no more 128 x 128 tiles than SMs: one wave either way
+  else
+    plan.bn = pico::one_cta_bn(pico_host::num_sms(), M, N);
   if (comm != nullptr && comm->tile_group != nullptr && comm->seg_start == nullptr && comm->d_num_dest == 0 &&
       comm->a_flags == nullptr && comm->num_groups > 0 && out_mode == pico::OUT_BF16 && max_ctas <= 0 &&
-      a_mn_major == 0 && N > 128 && comm->b_group_rows == (b_mn_major ? K : N) &&
-      (b_mn_major == 0 || K % pico::BK == 0) && pico::gemm_pair_takes_rows(M, comm->num_groups))
+      a_mn_major == 0 && comm->b_group_rows == (b_mn_major ? K : N) && (b_mn_major == 0 || K % pico::BK == 0) &&
+      pico_gemm_rows_plan(0, M, N, K, comm->num_groups))
     return pico::gemm_pair_rows(A, B, D, M, N, K, lda, ldb, ldd, b_mn_major, comm->tile_group, comm->num_groups,
                                 stream);
   if (comm != nullptr && comm->seg_start != nullptr && comm->tile_group == nullptr && comm->d_num_dest == 0 &&

@@ -33,9 +33,10 @@ bool gemm_pair_has(int a_mn_major, int b_mn_major, int out_mode);
 int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb,
               int ldd, int a_mn_major, int b_mn_major, int out_mode, float* slabs, cudaStream_t stream);
 
-// bf16 D with row groups (PicoGemmComm::tile_group, K-major A, B stacked) on the same kernel, and whether their number
-// and size suit it.
+// bf16 D with row groups (PicoGemmComm::tile_group, K-major A, B stacked) on the same kernel, whether their number and
+// size suit it, and whether the plain product is then faster than on the one-CTA kernel's tiles of width bn.
 bool gemm_pair_takes_rows(int M, int groups);
+bool gemm_pair_rows_pay(int sms, int M, int N, int K, int bn);
 int gemm_pair_rows(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd,
                    int b_mn_major, const int* tile_group, int groups, cudaStream_t stream);
 

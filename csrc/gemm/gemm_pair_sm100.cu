@@ -835,14 +835,32 @@ int gemm_pair(const GemmPlan& plan, const void* A, const void* B, void* D, int M
 }
 
 // `tiles` has room for one short tile per group, so from twice the groups on a group has about two. One CTA / pairs,
-// us, up, activation, down and their input gradients in all: 64 groups, 128 tiles (8192 rows) 389 / 391 to 160 tiles
-// 478 / 423, 208 tiles 668 / 672, 256 tiles 690 / 660 (rounds of whole tiles differ); 8 groups, 24 tiles 103 / 95.
-// Below that there are fewer pair tiles than pairs and their epilogues show: 8 groups, 16 tiles 64 / 68, 20 tiles 52 /
-// 55.
+// us, up, activation, down and their input gradients in all, width 2048 and 1024: 64 groups, 128 tiles (8192 rows) 389 /
+// 391 to 160 tiles 478 / 423, 208 tiles 668 / 672, 256 tiles 690 / 660 (rounds of whole tiles differ); 8 groups, 24 tiles
+// 103 / 95. Below that there are fewer pair tiles than pairs and their epilogues show: 8 groups, 16 tiles 64 / 68, 20
+// tiles 52 / 55. Plain products are held against the one-CTA kernel by gemm_pair_rows_pay too. With the activation
+// inside, the narrow ones lose on the GPU as well (8 groups, 24 tiles, 256 x 256: forward 8.1 / 9.8, backward 7.8 / 10.6;
+// 128 tiles 13.7 / 14.7, 13.1 / 11.7), but there the host sets the time, and one operator takes it less than three: forward
+// and backward of an expert layer of width 256 to 1024, 24 to 272 tiles, 700 / 630 with 8 experts, 830 / 755 with 16.
 bool gemm_pair_takes_rows(int M, int groups) {
   const int tiles = (M + pair::BM - 1) / pair::BM;
   return tiles <= pair::kMaxRowTiles && tiles >= 2 * (int64_t)groups && tiles >= 24 &&
          groups < 32768 && pico_host::num_sms() >= 2;
+}
+
+// Cycles of both kernels, as in plan_gemm: 512 for a K block of a round of pairs, though a round takes no less than its
+// epilogue's ~5000, and ~1000 to list the pairs; on the one-CTA kernel 333 for a K block of 128-wide tiles in one wave,
+// 573 for one of a round of 256-wide tiles. So narrow products with few row tiles, and short ones, stay there. One CTA /
+// pairs, us, 8 groups: 24 row tiles, N = K = 256 4.9 / 6.8, 512 5.9 / 8.2, 1024 10.4 / 11.1; 64, N = K = 512 7.8 / 8.8;
+// 128, N = 2048, K = 1024 56 / 49; 384, N = 1024, K = 256 32.9 / 41.1, K = 1024 84 / 74. Over 1100 products (N 256 ..
+// 4096, K 128 .. 4096, 24 .. 384 row tiles, 8 .. 64 groups) the choice is 0.3 % slower than the better one on average;
+// pairs for all of them 7.4 %, for none 4.0 %.
+bool gemm_pair_rows_pay(int sms, int M, int N, int K, int bn) {
+  const auto parts = [](int64_t n, int64_t of) { return (n + of - 1) / of; };
+  if (sms < 2) return false;
+  const int64_t kb = parts(K, pair::BK), rows = parts(M, pair::BM), round = kb * 512 > 5000 ? kb * 512 : 5000;
+  const int64_t one = parts(rows * parts(N, bn), sms) * kb * (bn < 256 ? 333 : 573);
+  return parts(parts(rows, 2) * parts(N, 256), sms / 2) * round + 1000 < one;
 }
 
 int gemm_pair_rows(const void* A, const void* B, void* D, int M, int N, int K, int lda, int ldb, int ldd, int b_mn,

@@ -138,6 +138,35 @@ def test_row_groups_on_pairs(counts, spare, inter, hidden):
         assert ((dga.double() - d * of).abs() <= bound).all()
 
 
+@pytest.mark.parametrize("counts,spare,N,K,on_pairs", [([5, 0, 9, 1, 13, 3], 1, 2048, 1024, True),
+                                                       ([11, 12, 1], 0, 2184, 2048, True),
+                                                       ([2] * 40 + [9] * 40, 3, 1032, 704, True),
+                                                       ([11, 12, 1], 0, 512, 512, False),
+                                                       ([33, 0, 91], 2, 1024, 192, False)])
+@pytest.mark.parametrize("b_mn_major", [False, True])
+def test_plain_products_with_row_groups(counts, spare, N, K, on_pairs, b_mn_major):
+    """Either side of the rule between the one-CTA kernel and pairs: odd and empty segments, ragged columns, tiles of no
+    group, several rounds."""
+    from picotron_b200 import ops
+    torch.manual_seed(N + K)
+    G, tg = len(counts), _tiles(counts, spare)
+    P = tg.numel() * 128
+    assert ops.ext().gemm_rows_plan(0, P, N, K, G) == on_pairs
+    group = tg.long().repeat_interleave(128)
+    x = torch.randn(P, K, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(G, *((K, N) if b_mn_major else (N, K)), device="cuda") / K ** 0.5).to(torch.bfloat16)
+    out = torch.full((P, N), 7.0, device="cuda", dtype=torch.bfloat16)
+    w2 = w.view(-1, w.shape[-1])
+    ops.ext().gemm_grouped(x, w2, out, P, N, K, K, w2.shape[1], N, False, b_mn_major, 0, 0, tg, G,
+                           K if b_mn_major else N)
+    ops.check_status()
+    assert (out[group < 0] == 7).all()
+    for g, c in enumerate(counts):
+        if c:
+            a, b = x[group == g].double(), w[g].double() if b_mn_major else w[g].double().t()
+            _close(out[group == g], a @ b, a.abs() @ b.abs(), K)
+
+
 def test_expert_layer_with_the_activation_inside_matches_the_separate_ops(monkeypatch):
     from types import SimpleNamespace
     from picotron_b200 import ops

@@ -191,6 +191,27 @@ def test_untracked_only_where_nothing_watches_the_call():
     assert seen == [False, True, False, False, False, True]
 
 
+def test_products_with_row_groups_run_on_pairs_where_that_is_faster():
+    """The rule looks at the width and the reduction too. Sizes whose sides were measured: narrow products of few row
+    tiles (one wave of 128-wide tiles) and short ones of many stay on the one-CTA kernel, the others do not."""
+    from picotron_b200 import ops
+    if not ops.ext_available():
+        pytest.skip("extension not built")
+    plan = ops.ext().gemm_rows_plan
+    for T in (24, 32, 48, 64):
+        for N in (256, 384, 512):
+            for K in (128, 256, 512, 1024):
+                assert not plan(148, T * 128, N, K, 8)
+    assert not plan(148, 24 * 128, 768, 768, 8) and not plan(148, 384 * 128, 1024, 256, 64)
+    for T in (128, 256, 448):
+        for N in (1024, 2048, 4096):
+            for K in (1024, 2048):
+                assert plan(148, T * 128, N, K, 8) and plan(148, T * 128 - 127, N, K, 64)
+    # as before: fewer than 24 tiles, less than two per group, more than the kernel's list holds, one half of a pair's tile
+    assert not any(plan(148, T * 128, N, 2048, G) for T, N, G in ((23, 4096, 8), (127, 4096, 64), (641, 4096, 64),
+                                                                  (128, 128, 8), (0, 4096, 0)))
+
+
 def test_gemm_plan_cuts_what_it_prices_as_cut():
     """The model that chooses a product's tiles and the launch share one decision about cutting the last round along K:
     no tile, or every tile of the partial round, each pair's share at least 3 blocks, accumulating products that have
