@@ -900,15 +900,18 @@ int gemm_pair_sums(const void* A, const void* B, float* D, int M, int N, int K, 
   return rc2 ? rc2 : pair::launched();
 }
 
-// All tiles of an [M, N] product whole.
-static int whole_plan(int M, int N, GemmPlan& plan) {
+// All tiles of an [M, N] product whole. With row groups odd segments take a pair tile more each, so their number is found
+// in the kernel and the grid has all pairs (32 row tiles in 8 odd segments on a grid for 16 pair tiles of each column:
+// two rounds, 13.9 us instead of 9.8 forward, 15.8 instead of 10.6 backward, 256 x 256).
+static int whole_plan(int M, int N, bool row_groups, GemmPlan& plan) {
   const int64_t tiles = (int64_t)((M + 255) / 256) * ((N + 255) / 256);
   const int sms = pico_host::num_sms();
   if (tiles > INT32_MAX || sms < 2) {
     pico_host::set_error("swiglu gemm: too many tiles, or fewer than two SMs");
     return -2;
   }
-  plan = GemmPlan{true, 256, sms / 2, (int)tiles, (int)tiles};
+  const int count = row_groups ? INT32_MAX : (int)tiles;
+  plan = GemmPlan{true, 256, sms / 2, count, count};
   return 0;
 }
 
@@ -955,7 +958,7 @@ extern "C" int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, voi
     return -2;
   }
   pico::GemmPlan plan;
-  int rc = pico::whole_plan(M, 2 * I, plan);
+  int rc = pico::whole_plan(M, 2 * I, tile_group != nullptr, plan);
   if (rc) return rc;
   pico::pair::OutMaps out = {};
   rc = pico_host::make_tmap_2d(&out.d, act, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, I, M, (uint64_t)I * 2, 64,
@@ -973,7 +976,7 @@ extern "C" int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* g
   if (M <= 0 || I <= 0 || K <= 0) return 0;
   if (tile_group != nullptr && !row_groups_ok(M, K, groups, true)) return -2;
   pico::GemmPlan plan;
-  int rc = pico::whole_plan(M, I, plan);
+  int rc = pico::whole_plan(M, I, tile_group != nullptr, plan);
   if (rc) return rc;
   pico::pair::OutMaps out = {};
   rc = pico::half_maps(&out.gate, &out.up, gate_up, M, I);
