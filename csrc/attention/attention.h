@@ -48,8 +48,8 @@ int pico_attention_bwd(const void* q, const void* k, const void* v, const void* 
                        int64_t dq_batch_stride, int64_t dq_row_stride, int64_t dk_batch_stride,
                        int64_t dk_row_stride, int64_t dv_batch_stride, int64_t dv_row_stride,
                        float* slabs, int splits, cudaStream_t stream);
-// slabs: NULL and splits 1, or pico_attention_bwd_splits(p) and 2 * splits * [b, sk, kv_heads, d] fp32 scratch: dK and
-// dV are then summed from that many partial results, in order.
+// splits: 1 with slabs NULL, or more (what pico_attention_bwd_splits says) with 2 * splits * [b, sk, kv_heads, d] fp32
+// scratch: dK and dV are then summed from that many partial results, in order.
 int pico_attention_bwd_splits(const PicoAttnParams* p);
 
 #ifdef __cplusplus

@@ -794,7 +794,8 @@ extern "C" int pico_attention_bwd_splits(const PicoAttnParams* p) {
   // slab bytes per split at 5 TB/s, in steps
   const double slab = 16.0 * p->batch * p->seq_k * p->kv_heads * p->head_dim / 5e6 / (p->head_dim == 64 ? 1.7 : 2.9);
   int best = 1;
-  double best_time = 0;      // a split that gains less than a tenth (as 3 x 1333 x 15/5 x 64, 69.0 / 69.9) is left
+  // a split that is modelled to gain less than 15 % (as 3 x 1333 x 15/5 x 64, 69.0 / 69.9 in two) is left
+  double best_time = 0;
   for (int n = 1; n <= 16 && n <= longest && key_blocks * n <= 65535; ++n) {
     const double own = (double)((longest + n - 1) / n) + 3, mean = (work + 3 * ctas * n) / sms;
     const double time = (own > mean ? own : mean) + (n > 1 ? 2 + n * slab : 0);

@@ -883,55 +883,6 @@ void attention_fwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v
         "attention_fwd");
 }
 
-// The scratch is fp32: delta of lse's size, dq_accum of q's, slabs for `splits` partial dk and dv (NULL where that is
-// 1).
-static void run_attention_bwd(PicoAttnParams& p, const at::Tensor& q, const at::Tensor& k, const at::Tensor& v,
-                              const at::Tensor& out, const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq,
-                              at::Tensor& dk, at::Tensor& dv, float* delta, float* dq_accum, float* slabs, int splits,
-                              const c10::optional<at::Tensor>& cos, const c10::optional<at::Tensor>& sin,
-                              int64_t rope_pos0) {
-  if (cos.has_value() && cos->defined()) {
-    TORCH_CHECK(sin.has_value() && sin->defined() && cos->is_cuda() && sin->is_cuda() &&
-                    cos->scalar_type() == at::kFloat && sin->scalar_type() == at::kFloat && cos->is_contiguous() &&
-                    sin->is_contiguous() && cos->dim() == 2 && cos->sizes() == sin->sizes() &&
-                    cos->size(1) == q.size(3) / 2,
-                "attention_bwd: rotary tables are fp32 [positions, head_dim / 2]");
-    TORCH_CHECK(rope_pos0 >= 0 && rope_pos0 + std::max(q.size(1), k.size(1)) <= cos->size(0),
-                "attention_bwd: rotary tables too short");
-    TORCH_CHECK(((reinterpret_cast<uintptr_t>(cos->data_ptr()) | reinterpret_cast<uintptr_t>(sin->data_ptr())) & 15) ==
-                    0, "attention_bwd: 16-byte aligned rotary tables");
-    p.rope_cos = cos->data_ptr<float>();
-    p.rope_sin = sin->data_ptr<float>();
-    p.rope_pos0 = (int)rope_pos0;
-  }
-  for (const at::Tensor* t : std::initializer_list<const at::Tensor*>{&dout, &dq, &dk, &dv}) {
-    TORCH_CHECK(t->scalar_type() == at::kBFloat16 && t->dim() == 4 && t->stride(3) == 1 &&
-                    t->stride(2) == t->size(3), "attention_bwd: [b, s, h, d] bf16 tensors with packed heads");
-  }
-  check(pico_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
-                           (const float*)lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), delta, dq_accum,
-                           &p, dout.stride(0), dout.stride(1), dq.stride(0), dq.stride(1), dk.stride(0), dk.stride(1),
-                           dv.stride(0), dv.stride(1), slabs, splits, stream_of(q)),
-        "attention_bwd");
-}
-
-void attention_bwd(const at::Tensor& q, const at::Tensor& k, const at::Tensor& v, const at::Tensor& out,
-                   const at::Tensor& dout, const at::Tensor& lse, at::Tensor& dq, at::Tensor& dk, at::Tensor& dv,
-                   at::Tensor& delta, at::Tensor& dq_accum, double sm_scale, bool causal, int64_t q_pos0,
-                   int64_t k_pos0, const c10::optional<at::Tensor>& cos, const c10::optional<at::Tensor>& sin,
-                   int64_t rope_pos0) {
-  c10::cuda::CUDAGuard guard(q.device());
-  PicoAttnParams p = attn_params(q, k, v, out, sm_scale, causal, q_pos0, k_pos0);
-  TORCH_CHECK(delta.scalar_type() == at::kFloat && dq_accum.scalar_type() == at::kFloat &&
-                  dq_accum.is_contiguous() && delta.numel() >= lse.numel() && dq_accum.numel() >= q.numel(),
-              "attention_bwd: fp32 scratch too small");
-  const int splits = pico_attention_bwd_splits(&p);
-  at::Tensor slabs;
-  if (splits > 1) slabs = at::empty({2 * splits * k.numel()}, lse.options());
-  run_attention_bwd(p, q, k, v, out, dout, lse, dq, dk, dv, (float*)delta.data_ptr(), (float*)dq_accum.data_ptr(),
-                    splits > 1 ? slabs.data_ptr<float>() : nullptr, splits, cos, sin, rope_pos0);
-}
-
 bool packed_heads(const at::Tensor& t) {
   return t.stride(3) == 1 && t.stride(2) == t.size(3) && (t.stride(1) * 2) % 16 == 0 && (t.stride(0) * 2) % 16 == 0 &&
          reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
@@ -952,7 +903,9 @@ std::tuple<at::Tensor, at::Tensor> attention_fwd_new(const at::Tensor& q_, const
   return {out, lse};
 }
 
-// (dq, dk, dv): column slices of one [b, s, (H + 2 Hkv) d] buffer when the sequence lengths match
+// (dq, dk, dv): column slices of one [b, s, (H + 2 Hkv) d] buffer when the sequence lengths match. cos, sin: of the rotary
+// embedding that q and k carry; splits: into how many shares the steps of a key block go, 0 for what
+// pico_attention_bwd_splits says.
 std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tensor& dout_, const at::Tensor& q_,
                                                                  const at::Tensor& k_, const at::Tensor& v_,
                                                                  const at::Tensor& out_, const at::Tensor& lse,
@@ -960,7 +913,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
                                                                  int64_t k_pos0,
                                                                  const c10::optional<at::Tensor>& cos,
                                                                  const c10::optional<at::Tensor>& sin,
-                                                                 int64_t rope_pos0) {
+                                                                 int64_t rope_pos0, int64_t splits) {
   at::Tensor q = pack_heads(q_), k = pack_heads(k_), v = pack_heads(v_);
   at::Tensor out = pack_heads(out_), dout = pack_heads(dout_);
   TORCH_CHECK(lse.scalar_type() == at::kFloat && lse.is_contiguous() && dout.sizes() == q.sizes() &&
@@ -979,14 +932,36 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
     dk = at::empty({b, sk, kvh, d}, q.options());
     dv = at::empty({b, sk, kvh, d}, q.options());
   }
-  // one allocation for the scratch, its parts on 256-byte boundaries
+  for (const at::Tensor* t : std::initializer_list<const at::Tensor*>{&dout, &dq, &dk, &dv}) {
+    TORCH_CHECK(t->scalar_type() == at::kBFloat16 && t->dim() == 4 && t->stride(3) == 1 &&
+                    t->stride(2) == t->size(3), "attention_bwd: [b, s, h, d] bf16 tensors with packed heads");
+  }
   PicoAttnParams p = attn_params(q, k, v, out, sm_scale, causal, q_pos0, k_pos0);
-  const int splits = pico_attention_bwd_splits(&p);
+  if (cos.has_value() && cos->defined()) {
+    TORCH_CHECK(sin.has_value() && sin->defined() && cos->is_cuda() && sin->is_cuda() &&
+                    cos->scalar_type() == at::kFloat && sin->scalar_type() == at::kFloat && cos->is_contiguous() &&
+                    sin->is_contiguous() && cos->dim() == 2 && cos->sizes() == sin->sizes() && cos->size(1) == d / 2,
+                "attention_bwd: rotary tables are fp32 [positions, head_dim / 2]");
+    TORCH_CHECK(rope_pos0 >= 0 && rope_pos0 + std::max(sq, sk) <= cos->size(0),
+                "attention_bwd: rotary tables too short");
+    TORCH_CHECK(((reinterpret_cast<uintptr_t>(cos->data_ptr()) | reinterpret_cast<uintptr_t>(sin->data_ptr())) & 15) ==
+                    0, "attention_bwd: 16-byte aligned rotary tables");
+    p.rope_cos = cos->data_ptr<float>();
+    p.rope_sin = sin->data_ptr<float>();
+    p.rope_pos0 = (int)rope_pos0;
+  }
+  TORCH_CHECK(splits >= 0 && splits <= 16 && splits * ((sk + 127) / 128) <= 65535, "attention_bwd: 0 to 16 splits");
+  if (splits == 0) splits = pico_attention_bwd_splits(&p);
+  // one allocation for the scratch, its parts on 256-byte boundaries
   const int64_t accum = b * sq * H * d, slabs = splits > 1 ? 2 * splits * b * sk * kvh * d : 0;
   at::Tensor scratch = at::empty({accum + slabs + b * H * sq}, q.options().dtype(at::kFloat));
   float* f = scratch.data_ptr<float>();
-  run_attention_bwd(p, q, k, v, out, dout, lse, dq, dk, dv, f + accum + slabs, f, splits > 1 ? f + accum : nullptr,
-                    splits, cos, sin, rope_pos0);
+  check(pico_attention_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+                           (const float*)lse.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
+                           f + accum + slabs, f, &p, dout.stride(0), dout.stride(1), dq.stride(0), dq.stride(1),
+                           dk.stride(0), dk.stride(1), dv.stride(0), dv.stride(1), splits > 1 ? f + accum : nullptr,
+                           (int)splits, stream_of(q)),
+        "attention_bwd");
   return {dq, dk, dv};
 }
 
@@ -1026,7 +1001,21 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("attention_bwd_new", &attention_bwd_new, py::arg("dout"), py::arg("q"), py::arg("k"), py::arg("v"),
         py::arg("out"), py::arg("lse"), py::arg("sm_scale"), py::arg("causal"), py::arg("q_pos0"), py::arg("k_pos0"),
         py::arg("cos") = c10::optional<at::Tensor>(), py::arg("sin") = c10::optional<at::Tensor>(),
-        py::arg("rope_pos0") = 0);
+        py::arg("rope_pos0") = 0, py::arg("splits") = 0);
+  m.def("attention_bwd_splits", [](int64_t b, int64_t sq, int64_t sk, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                                   bool causal, int64_t q_pos0, int64_t k_pos0) {
+    PicoAttnParams p = {};
+    p.batch = (int)b;
+    p.seq_q = (int)sq;
+    p.seq_k = (int)sk;
+    p.heads = (int)heads;
+    p.kv_heads = (int)kv_heads;
+    p.head_dim = (int)head_dim;
+    p.causal = causal;
+    p.q_pos0 = (int)q_pos0;
+    p.k_pos0 = (int)k_pos0;
+    return pico_attention_bwd_splits(&p);
+  });
   m.def("rmsnorm_fwd", &rmsnorm_fwd);
   m.def("rmsnorm_bwd", &rmsnorm_bwd);
   m.def("rmsnorm_bwd_num_partials", &rmsnorm_bwd_num_partials);
@@ -1055,11 +1044,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("moe_scatter_sum", &moe_scatter_sum);
   m.def("status_fetch", &status_fetch);
   m.def("attention_fwd", &attention_fwd);
-  m.def("attention_bwd", &attention_bwd, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("out"), py::arg("dout"),
-        py::arg("lse"), py::arg("dq"), py::arg("dk"), py::arg("dv"), py::arg("delta"), py::arg("dq_accum"),
-        py::arg("sm_scale"), py::arg("causal"), py::arg("q_pos0"), py::arg("k_pos0"),
-        py::arg("cos") = c10::optional<at::Tensor>(), py::arg("sin") = c10::optional<at::Tensor>(),
-        py::arg("rope_pos0") = 0);
   m.def("symm_alloc", &symm_alloc);
   m.def("symm_open", &symm_open);
   m.def("symm_close", &symm_close);

@@ -86,7 +86,7 @@ struct AttentionNode : torch::autograd::Function<AttentionNode> {
     const auto saved = ctx->get_saved_variables();
     auto [dq, dk, dv] = attention_bwd_new(grads[0], saved[0], saved[1], saved[2], saved[3], saved[4],
                                           ctx->saved_data["sm_scale"].toDouble(), ctx->saved_data["causal"].toBool(),
-                                          0, 0, c10::nullopt, c10::nullopt, 0);
+                                          0, 0, c10::nullopt, c10::nullopt, 0, 0);
     g_launches += 3;
     return {dq, dk, dv, at::Tensor(), at::Tensor()};
   }

@@ -19,7 +19,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> attention_bwd_new(const at::Tenso
                                                                  double sm_scale, bool causal, int64_t q_pos0,
                                                                  int64_t k_pos0, const c10::optional<at::Tensor>& cos,
                                                                  const c10::optional<at::Tensor>& sin,
-                                                                 int64_t rope_pos0);
+                                                                 int64_t rope_pos0, int64_t splits);
 
 void def_native_calls(pybind11::module_& m);
 

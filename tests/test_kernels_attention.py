@@ -273,14 +273,15 @@ def test_rotary_attention_gradients_against_64_bits(b, s, H, Hkv, d, offset):
             assert (a - w).norm() <= 0.015 * w.norm()
 
 
-@pytest.mark.parametrize("b,s,H,Hkv,d,causal", [(1, 300, 1, 1, 64, True), (1, 1100, 8, 1, 64, True),
-                                                (2, 513, 3, 1, 128, False), (1, 129, 2, 2, 128, True)])
-def test_key_blocks_shared_by_several_ctas(b, s, H, Hkv, d, causal):
-    """Few key blocks: the steps of each are split, unevenly and, where a block has fewer than shares, with empty ones.
-    dK and dV are sums of the shares in order, the same bits on each run; 2-norm of bf16 roundings of P and dS (2^-9
-    each) and of the results against 64 bits."""
+@pytest.mark.parametrize("b,s,H,Hkv,d,causal,shared", [(1, 300, 1, 1, 64, True, False), (1, 1100, 8, 1, 64, True, True),
+                                                       (2, 513, 3, 1, 128, False, True), (1, 129, 2, 2, 128, True, False)])
+def test_key_blocks_shared_by_several_ctas(b, s, H, Hkv, d, causal, shared):
+    """Few key blocks: where they have enough steps the steps of each are split. dK and dV are sums of the shares in
+    order, the same bits on each run; 2-norm of bf16 roundings of P and dS (2^-9 each) and of the results against 64
+    bits."""
     from picotron_b200 import ops
     from picotron_b200.ops import attention as A
+    assert (ops.ext().attention_bwd_splits(b, s, s, H, Hkv, d, causal, 0, 0) > 1) == shared
     torch.manual_seed(s)
     q, go = (torch.randn(b, s, H, d, device="cuda").to(torch.bfloat16) for _ in range(2))
     k, v = (torch.randn(b, s, Hkv, d, device="cuda").to(torch.bfloat16) for _ in range(2))
@@ -297,3 +298,60 @@ def test_key_blocks_shared_by_several_ctas(b, s, H, Hkv, d, causal):
     ref = torch.einsum("bhqk,bkhd->bqhd", score.softmax(-1), vr.repeat_interleave(H // Hkv, 2))
     for got, want in zip(first, torch.autograd.grad(ref, (qr, kr, vr), go.double())):
         assert (got.double() - want).norm() <= 3 * 2 ** -9 * want.norm()
+
+
+@pytest.mark.parametrize("splits", [0, 1, 2, 3, 16])
+@pytest.mark.parametrize("b,sq,sk,H,Hkv,d,causal,q0,k0,rope", [
+    (1, 300, 300, 1, 1, 64, True, 0, 0, False), (2, 129, 129, 4, 2, 128, True, 0, 0, True),
+    (3, 257, 257, 3, 1, 64, True, 0, 0, True), (1, 640, 640, 3, 3, 64, False, 0, 0, True),
+    (2, 200, 330, 4, 2, 64, True, 130, 0, False), (1, 1024, 1024, 8, 2, 64, True, 1024, 0, False),
+    (1, 300, 300, 2, 1, 128, True, 0, 200, False)])
+def test_any_number_of_shares(b, sq, sk, H, Hkv, d, causal, q0, k0, rope, splits):
+    """One to 16 shares of a key block's steps, uneven ones and more than there are steps, several batches; steps of a
+    ring, where the keys lie behind the queries or ahead of some (rows without a key); rotated q and k, whose gradients
+    are rotated back from the slabs. Against 64 bits: roundings of P and dS to bf16 and of the results (2^-9 each), one
+    more where dK is rounded before it is rotated."""
+    from picotron_b200 import ops
+    from picotron_b200.ops import attention as A
+    from picotron_b200.ops import rope as R
+    torch.manual_seed(sq + sk)
+    q, go = (torch.randn(b, sq, H, d, device="cuda").to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(b, sk, Hkv, d, device="cuda").to(torch.bfloat16) for _ in range(2))
+    tables = ()
+    if rope:
+        tables = (*R.rope_tables_for_kernel(*R.get_cos_sin(sk + 9, d, 10000.0, device="cuda")), 4)
+    out, lse = A.flash_attention_forward(q, k, v, causal, None, q0, k0)
+
+    def run():
+        return ops.ext().attention_bwd_new(go, q, k, v, out, lse, d ** -0.5, causal, q0, k0, *(tables or (None, None, 0)),
+                                           splits)
+    grads = [t.clone() for t in run()]
+    again = run()
+    assert torch.equal(again[1], grads[1]) and torch.equal(again[2], grads[2])
+    ops.check_status()
+    q6, k6, v6, g6 = (t.double().transpose(1, 2) for t in (q, k.repeat_interleave(H // Hkv, 2),
+                                                           v.repeat_interleave(H // Hkv, 2), go))
+    score = q6 @ k6.transpose(-1, -2) * d ** -0.5
+    if causal:
+        hidden = torch.arange(sk, device="cuda")[None] + k0 > torch.arange(sq, device="cuda")[:, None] + q0
+        score = score.masked_fill(hidden, float("-inf"))
+    p = score.softmax(-1).nan_to_num(0.0)
+    ds = p * (g6 @ v6.transpose(-1, -2) - (g6 * (p @ v6)).sum(-1, keepdim=True)) * d ** -0.5
+    want = [ds @ k6, ds.transpose(-1, -2) @ q6, p.transpose(-1, -2) @ g6]
+    want = [t.transpose(1, 2) if i == 0 else t.transpose(1, 2).unflatten(2, (Hkv, -1)).sum(3) for i, t in enumerate(want)]
+    if rope:
+        for i in (0, 1):
+            lo, hi = want[i].chunk(2, -1)
+            c, n = (t[4:4 + want[i].shape[1]].double()[None, :, None] for t in tables[:2])
+            want[i] = torch.cat([lo * c + hi * n, hi * c - lo * n], -1)
+    for got, w in zip(grads, want):
+        assert (got.double() - w).norm() <= (4 if rope else 3) * 2 ** -9 * w.norm()
+
+
+def test_wrong_numbers_of_shares_are_refused():
+    from picotron_b200 import ops
+    q = torch.zeros(1, 64, 1, 64, device="cuda", dtype=torch.bfloat16)
+    lse = torch.zeros(1, 1, 64, device="cuda")
+    for splits in (-1, 17):
+        with pytest.raises(RuntimeError, match="splits"):
+            ops.ext().attention_bwd_new(q, q, q, q, q, lse, 1.0, True, 0, 0, None, None, 0, splits)

@@ -191,6 +191,22 @@ def test_untracked_only_where_nothing_watches_the_call():
     assert seen == [False, True, False, False, False, True]
 
 
+def test_attention_backward_shares_the_steps_of_few_key_blocks():
+    """Sizes whose sides were measured (148 SMs, which the rule takes where there is no GPU): many key blocks, or few
+    steps, stay whole; nothing is cut into more shares than the longest block has steps."""
+    from picotron_b200 import ops
+    if not ops.ext_available():
+        pytest.skip("extension not built")
+    rule = ops.ext().attention_bwd_splits
+    for b, s, H, Hkv, d in ((1, 8192, 4, 1, 128), (4, 2048, 4, 1, 64), (1, 4096, 1, 1, 64), (1, 256, 9, 3, 64)):
+        assert 1 < rule(b, s, s, H, Hkv, d, s > 256, 0, 0) <= min(16, -(-s // 128) * H // Hkv)
+    for b, s, H, Hkv, d in ((2, 2048, 8, 8, 128), (3, 1333, 15, 5, 64), (8, 1024, 15, 5, 64), (1, 300, 1, 1, 64),
+                            (1, 16384, 32, 8, 128), (1, 1, 1, 1, 64)):
+        assert rule(b, s, s, H, Hkv, d, True, 0, 0) == 1
+    assert rule(1, 1024, 1024, 8, 2, 64, True, 1024, 0) > 1           # a ring step: keys behind all queries
+    assert rule(1, 1024, 1024, 8, 2, 64, True, 0, 1024) == 1          # ahead of all: no steps at all
+
+
 def test_products_with_row_groups_run_on_pairs_where_that_is_faster():
     """The rule looks at the width and the reduction too. Sizes whose sides were measured: narrow products of few row
     tiles (one wave of 128-wide tiles) and short ones of many stay on the one-CTA kernel, the others do not."""
