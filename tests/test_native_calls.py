@@ -177,6 +177,31 @@ def test_native_forward_matches_the_modules(b, s):
     assert model(ids).grad_fn is not None                       # with gradients the modules run
 
 
+@pytest.mark.parametrize("b,s,shape,in_epilogue,parts", [
+    (2, 500, dict(intermediate_size=2048, num_attention_heads=8, num_key_value_heads=4), True, False),
+    (1, 33, dict(intermediate_size=8192, num_attention_heads=8, num_key_value_heads=2), False, True),
+    (2, 200, dict(intermediate_size=8192, num_attention_heads=16, num_key_value_heads=16), True, True),
+    (1, 7, dict(intermediate_size=6144, num_attention_heads=8, num_key_value_heads=8), False, True)])
+def test_native_forward_with_every_layout_of_its_memory(b, s, shape, in_epilogue, parts):
+    """The activation in the gate-up product (no room for gate | up) and by itself, the down projection whole and in
+    parts of K (slabs in the same allocation), head_dim 64 and 128; three layers, so every buffer is used again."""
+    from picotron_b200 import ops
+    model, _ = _model(dict(hidden_size=1024, vocab_size=4096, **shape), 3, 600)
+    inter = shape["intermediate_size"]
+    assert ops.ext().gemm_swiglu_pays(b * s, inter, 1024, False, False) == in_epilogue
+    assert (ops.ext().gemm_parts_of_k(b * s, 1024, inter) > 0) == parts
+    ids = torch.randint(0, 4096, (b, s), device="cuda")
+    with torch.no_grad():
+        assert model._native_layers(ids) is not None
+        native = [model(ids) for _ in range(2)]
+        handle = model.final_norm.register_forward_hook(lambda *a: None)
+        assert model._native_layers(ids) is None
+        modules = model(ids)
+        handle.remove()
+    ops.check_status()
+    assert all(torch.equal(n, modules) for n in native) and modules.float().std() > 0.01
+
+
 def test_native_forward_is_left_where_it_does_not_apply():
     ids = torch.randint(0, 49152, (1, 20), device="cuda")
     model, _ = _model({}, 2, 32)
