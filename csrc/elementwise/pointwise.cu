@@ -218,7 +218,7 @@ __global__ void embedding_fwd_kernel(const __nv_bfloat16* __restrict__ W,
 }
 
 // Bound by the reductions' way through L2: four fp32 columns per request (8192 x 2048: 25 us, with one
-// column per request 88).
+// column per request 88, called repeatedly; 41 and 105 with the L2 flushed before each call).
 template <bool kAligned>
 __global__ void embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dout,
                                      const int64_t* __restrict__ ids, float* __restrict__ dW,

@@ -28,9 +28,10 @@
 // What a pass of its own over gate | up took (402 MB forward, 671 MB backward for 8192 rows of 2 x 8192) then runs
 // under the main loop, 16 thousand cycles per tile at K = 2048. Values are rounded to bf16 before the activation, as
 // that pass reads them. Product and pass / fused, us: 8192 rows, 2048 -> 8192: forward 420 / 363, backward 306 / 226;
-// 16384, 2048 -> 5632: 566 / 496, 414 / 338; 8192, 960 -> 2560: 77 / 65, 71 / 55. The movers' four buffers cost a stage
-// of operands; six buffers and four stages measured 393 and 284 us in the first line, and with four epilogue warps the
-// short ones 1 us more.
+// 16384, 2048 -> 5632: 566 / 496, 414 / 338; 8192, 960 -> 2560: 77 / 65, 71 / 55 (eight in a row on another machine:
+// 412 / 356, 326 / 246; 573 / 503, 440 / 321; 98 / 77, 80 / 61). The movers' four buffers cost a stage of operands; six
+// buffers and four stages measured 393 and 284 us in the first line, and with four epilogue warps the short ones 1 us
+// more.
 //
 // Work split: output tiles are dealt to the pairs in whole rounds; where D is accumulated (weight
 // gradients) the tiles of the last, partial round are cut along K into equal shares for all pairs, so that
