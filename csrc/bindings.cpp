@@ -993,6 +993,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_rows_plan", [](int64_t sms, int64_t M, int64_t N, int64_t K, int64_t groups) {
     return pico_gemm_rows_plan((int)sms, (int)M, (int)N, (int)K, (int)groups) != 0;
   });
+  m.def("gemm_swiglu_pairs", [](int64_t M, int64_t I, bool row_groups, bool backward) {
+    return pico_gemm_swiglu_pairs((int)M, (int)I, row_groups, backward);
+  });
   m.def("gemm_swiglu_pays", [](int64_t M, int64_t I, int64_t K, bool keep, bool backward) {
     return pico_gemm_swiglu_pays((int)M, (int)I, (int)K, keep, backward) != 0;
   });

@@ -48,6 +48,8 @@ int pico_gemm_swiglu(const void* x, const void* w, void* gate_up, void* act, int
 int pico_gemm_swiglu_pays(int M, int I, int K, int keep_gate, int backward);
 int pico_gemm_swiglu_bwd(const void* dy, const void* w, const void* gate_up, void* d_gate_up, int M, int I, int K,
                          int lddy, int ldw, const int* tile_group, int groups, cudaStream_t stream);
+// How many CTA pairs the two launch.
+int pico_gemm_swiglu_pairs(int M, int I, int row_groups, int backward);
 // Whether M rows in `groups` row groups run on CTA pairs with the activation in the epilogues, and whether a plain
 // product with N columns does (sms: 0 for this GPU's).
 int pico_gemm_rows_on_pairs(int M, int groups);

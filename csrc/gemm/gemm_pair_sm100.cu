@@ -729,6 +729,10 @@ add_pieces_kernel(const float* __restrict__ slabs, float* __restrict__ D, int64_
   }
 }
 
+static int pairs_launched(const GemmPlan& plan) {
+  return plan.whole == plan.tiles && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
+}
+
 // Maps of the operands, the kernel's attributes and its launch.
 // groups, group_array: row groups and the group of every row tile (B has a matrix for each), or the beginnings of
 // reduction groups.
@@ -760,8 +764,7 @@ static int start(const GemmPlan& plan, const void* A, const void* B, const OutMa
     }
     attr_dev = dev;
   }
-  const int pairs = plan.whole == plan.tiles && plan.tiles < plan.pairs ? plan.tiles : plan.pairs;
-  pico_host::launch_ahead(kern, 2 * pairs, C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K, plan.whole,
+  pico_host::launch_ahead(kern, 2 * pairs_launched(plan), C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K, plan.whole,
                           keep_gate, group_array, pico_status_buffer());
   return 0;
 }
@@ -939,6 +942,12 @@ extern "C" int pico_gemm_swiglu_pays(int M, int I, int K, int keep_gate, int bac
   const pico::GemmPlan plan = pico::plan_gemm(pico_host::num_sms(), M, backward ? I : 2 * I, K, 0, backward,
                                               pico::GEMM_OUT_BF16, 0, false);
   return plan.pair && (int64_t)M * I >= (backward ? 4000000 : keep_gate ? 2500000 : 1250000);
+}
+
+extern "C" int pico_gemm_swiglu_pairs(int M, int I, int row_groups, int backward) {
+  pico::GemmPlan plan;
+  return M <= 0 || I <= 0 || pico::whole_plan(M, backward ? I : 2 * I, row_groups != 0, plan)
+             ? 0 : pico::pair::pairs_launched(plan);
 }
 
 static bool row_groups_ok(int M, int K, int groups, bool whole_k) {

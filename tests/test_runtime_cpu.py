@@ -191,6 +191,21 @@ def test_untracked_only_where_nothing_watches_the_call():
     assert seen == [False, True, False, False, False, True]
 
 
+def test_products_with_swiglu_have_a_pair_for_every_tile_of_odd_segments():
+    """Segments of an odd number of row tiles need more pair tiles than the rows have in all: the grid has all pairs
+    then. Without row groups it has no more than tiles."""
+    from picotron_b200 import ops
+    if not ops.ext_available():
+        pytest.skip("extension not built")
+    pairs = ops.ext().gemm_swiglu_pairs
+    for tiles, inter in ((24, 64), (32, 256), (32, 1024), (640, 2048)):
+        for backward in (False, True):
+            width = inter if backward else 2 * inter
+            columns = -(-width // 256)
+            assert pairs(tiles * 128, inter, True, backward) == 74
+            assert pairs(tiles * 128, inter, False, backward) == min(74, -(-tiles // 2) * columns)
+
+
 def test_attention_backward_shares_the_steps_of_few_key_blocks():
     """Sizes whose sides were measured (148 SMs, which the rule takes where there is no GPU): many key blocks, or few
     steps, stay whole; nothing is cut into more shares than the longest block has steps."""
