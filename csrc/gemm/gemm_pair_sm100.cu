@@ -764,8 +764,8 @@ static int start(const GemmPlan& plan, const void* A, const void* B, const OutMa
     }
     attr_dev = dev;
   }
-  pico_host::launch_ahead(kern, 2 * pairs_launched(plan), C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K, plan.whole,
-                          keep_gate, group_array, pico_status_buffer());
+  pico_host::launch_ahead(kern, 2 * pairs_launched(plan), C::kThreads, C::kSmemBytes, stream, ta, tb, out, M, N, K,
+                          plan.whole, keep_gate, group_array, pico_status_buffer());
   return 0;
 }
 
